@@ -242,7 +242,7 @@ struct SceneHost {
 
 // ---------------------------------------------------------------------------
 // Page-locked host words for asynchronous read-backs of single device words
-// (the P2G staging decision).  One page-locked block for the process, handed
+// (the count of small P2G items).  One page-locked block for the process, handed
 // out word by word: cudaHostAlloc per engine costs milliseconds (it pins
 // pages), which a solver's construction and first step would pay.
 // ---------------------------------------------------------------------------
@@ -377,7 +377,7 @@ public:
             for (auto e : e4)
                 if (e) cudaEventDestroy(e);
         if (host_word_) g_pinned_words.give(host_word_);
-        if (stage_event_) cudaEventDestroy(stage_event_);
+        if (warp_event_) cudaEventDestroy(warp_event_);
         giveStream(device_, stream_);
     }
 
@@ -1017,8 +1017,8 @@ public:
         keys_valid_ = false;
         sorted_valid_ = false;
         incremental_ok_ = false;
-        stage_check_ = true;
-        stage_pending_ = false;  // a read-back issued before the sync above is stale
+        warp_check_ = true;
+        warp_pending_ = false;  // a read-back issued before the sync above is stale
         for (bool& f : warp_few_) f = false;  // the new set's small items: decided on the device until read back
         any_implicit_ = false;
         for (auto& s : scenes_) any_implicit_ |= s->beta > 0.f;
@@ -1134,7 +1134,7 @@ public:
         c.nscenes = (int)scenes_.size();
         c.stream = stream_;
         c.num_sms = num_sms_;
-        c.p2g_stage = p2g_stage_;
+        c.p2g_stage = kDefaultP2GStage;
         c.particle_blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((max_n_ + kThreads - 1) / kThreads,
                                                                            (size_t)num_sms_ * 16));
         c.node_blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((max_nodes_ + kThreads - 1) / kThreads,
@@ -1386,7 +1386,7 @@ public:
     bool steadyNow() const {
         bool stale = false;
         for (auto& s : scenes_) stale |= s->stress_stale;
-        return use_graphs_ && keys_valid_ && incremental_ok_ && !stale && !profiling_ && !dirty_ && !stage_check_ &&
+        return use_graphs_ && keys_valid_ && incremental_ok_ && !stale && !profiling_ && !dirty_ && !warp_check_ &&
                !tune_run_;
     }
 
@@ -1434,11 +1434,11 @@ public:
     // Captures, ahead of time, the graphs of the states the next steps visit
     // (they alternate between particle buffers and key buffers), so that a
     // timed run replays graphs from its first step instead of capturing inside
-    // its timed region.  Resolves a pending staging decision first.
+    // its timed region.  Resolves a pending item-count read-back first.
     mpm_status prepareGraphs() {
-        if (stage_pending_) {
-            CUDA_TRY(cudaEventSynchronize(stage_event_));
-            MPM_TRY(checkP2GStage());
+        if (warp_pending_) {
+            CUDA_TRY(cudaEventSynchronize(warp_event_));
+            MPM_TRY(checkWarpItems());
         }
         const int p0 = parity_, k0 = kcur_, s0 = sorted_;
         const bool kv = keys_valid_, sv = sorted_valid_, io = incremental_ok_;
@@ -1628,7 +1628,7 @@ public:
     }
     int p2gStageOf(const Combo& c) const {
         const int st = tuningOf(c.S, c.transfer).p2g_stage;
-        return st ? st : p2g_stage_;
+        return st ? st : kDefaultP2GStage;
     }
     ComboSplit comboSplit() const {
         ComboSplit g;
@@ -1733,7 +1733,7 @@ public:
         advanceClock();
         ++run;
         CUDA_TRY(cudaStreamSynchronize(stream_));
-        if (stage_pending_) MPM_TRY(checkP2GStage());
+        if (warp_pending_) MPM_TRY(checkWarpItems());
         uint32_t cnt[kMaxCombos] = {};
         CUDA_TRY(cudaMemcpy(cnt, counters_.as<uint32_t>() + kG2PCountWord, sizeof(cnt), cudaMemcpyDeviceToHost));
         std::vector<std::string> keys(nc);
@@ -1805,44 +1805,38 @@ public:
         return MPM_OK;
     }
 
-    // P2G stages 32 particles per warp pass in dense scenes and 16 in sparse
-    // ones (fewer than 8 particles per cell on average: the smaller staging
-    // buffer fits 3 CTAs per SM and the passes are rarely full).  Decided
-    // once after the first step that follows a change of the scene set,
-    // from the number of work items of that step.  The count is read back
-    // asynchronously (a copy into pinned host memory and an event), so the
-    // host does not wait for the GPU: the steps that follow run with direct
-    // launches until the event has completed, and only then is the step
-    // captured as a CUDA graph (a change of staging size would drop it).
-    mpm_status checkP2GStage() {
-        if (!stage_check_) return MPM_OK;
-        if (!stage_pending_) {
+    // Whether any combination has too few small P2G items for the warp kernel,
+    // so that its launch can be skipped: decided once after the first step
+    // that follows a change of the scene set, from that step's counts.  They
+    // are read back asynchronously (a copy into pinned host memory and an
+    // event), so the host does not wait for the GPU: the steps that follow
+    // run with direct launches until the event has completed, and only then
+    // is the step captured as a CUDA graph (a change would drop it).
+    mpm_status checkWarpItems() {
+        if (!warp_check_) return MPM_OK;
+        if (!warp_pending_) {
             if (!host_word_) {
                 host_word_ = g_pinned_words.take();
-                if (!host_word_) return fail(MPM_ERR_OOM, "no page-locked host word for the staging read-back");
-                CUDA_TRY(cudaEventCreateWithFlags(&stage_event_, cudaEventDisableTiming));
+                if (!host_word_) return fail(MPM_ERR_OOM, "no page-locked host word for the item-count read-back");
+                CUDA_TRY(cudaEventCreateWithFlags(&warp_event_, cudaEventDisableTiming));
             }
-            CUDA_TRY(cudaMemcpyAsync(host_word_, counters_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_));
-            static_assert(1 + kMaxCombos <= PinnedWords::kLine, "read-back line too short");
-            CUDA_TRY(cudaMemcpyAsync(host_word_ + 1, counters_.as<uint32_t>() + kP2GSmallWord,
+            static_assert(kMaxCombos <= PinnedWords::kLine, "read-back line too short");
+            CUDA_TRY(cudaMemcpyAsync(host_word_, counters_.as<uint32_t>() + kP2GSmallWord,
                                      sizeof(uint32_t) * kMaxCombos, cudaMemcpyDeviceToHost, stream_));
-            CUDA_TRY(cudaEventRecord(stage_event_, stream_));
-            stage_pending_ = true;
+            CUDA_TRY(cudaEventRecord(warp_event_, stream_));
+            warp_pending_ = true;
             return MPM_OK;
         }
-        const cudaError_t q = cudaEventQuery(stage_event_);
+        const cudaError_t q = cudaEventQuery(warp_event_);
         if (q == cudaErrorNotReady) return MPM_OK;
         CUDA_TRY(q);
-        stage_pending_ = false;
-        stage_check_ = false;
-        const uint32_t items = host_word_[0];
-        const int stage = (items > 0 && ntot_ / items < 512) ? 16 : 32;
-        bool changed = stage != p2g_stage_;
-        p2g_stage_ = stage;
+        warp_pending_ = false;
+        warp_check_ = false;
+        bool changed = false;
         // a combination with too few small P2G items for warps skips the
         // warp kernel's launch (the device would leave them to p2gKernel)
         for (int k = 0; k < kMaxCombos; ++k) {
-            const bool few = host_word_[1 + k] < kWarpAutoMinItems;
+            const bool few = host_word_[k] < kWarpAutoMinItems;
             changed |= few != warp_few_[k];
             warp_few_[k] = few;
         }
@@ -1865,7 +1859,7 @@ public:
                 CUDA_TRY(cudaEventRecord(e1, stream_));
                 step_events_.push_back({e0, e1});
             }
-            MPM_TRY(checkP2GStage());
+            MPM_TRY(checkWarpItems());
             advanceClock();
         }
         return MPM_OK;
@@ -1974,7 +1968,7 @@ public:
         CUDA_TRY(cudaEventRecord(ev_[0][0], stream_));
         for (int i = 0; i < n; ++i) {
             MPM_TRY(stepOnce());
-            MPM_TRY(checkP2GStage());
+            MPM_TRY(checkWarpItems());
             advanceClock();
         }
         CUDA_TRY(cudaEventRecord(ev_[0][1], stream_));
@@ -2013,7 +2007,7 @@ public:
 
     mpm_status synchronize() {
         CUDA_TRY(cudaStreamSynchronize(stream_));
-        if (stage_pending_) MPM_TRY(checkP2GStage());  // its read-back has landed
+        if (warp_pending_) MPM_TRY(checkWarpItems());  // its read-back has landed
         MPM_TRY(downloadWait());
         uint32_t e = 0;
         CUDA_TRY(cudaMemcpy(&e, err_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -2381,9 +2375,9 @@ private:
     int device_ = 0, num_sms_ = 148;
     cudaMemPool_t pool_ = nullptr;         // the device's scene pool (init)
     size_t staging_reserved_ = 0;          // particles whose download staging the pool was grown for
-    uint32_t* host_word_ = nullptr;        // pinned: work-item count read back by checkP2GStage
-    cudaEvent_t stage_event_ = nullptr;    // completion of that read-back
-    bool stage_pending_ = false;
+    uint32_t* host_word_ = nullptr;        // pinned: work-item count read back by checkWarpItems
+    cudaEvent_t warp_event_ = nullptr;    // completion of that read-back
+    bool warp_pending_ = false;
     cudaStream_t stream_ = nullptr;
     cudaStream_t compact_stream_ = nullptr;  // block compaction beside the sort
     cudaEvent_t compact_fork_ = nullptr, compact_join_ = nullptr;
@@ -2394,13 +2388,12 @@ private:
     bool any_cfl_ = false;     // some scene steps with a CFL dt (two more launches per step)
     bool any_implicit_ = false;  // some scene solves the semi-implicit update
     DevMem cell_range_, block_range_, solve_pofs_, solve_prep_, solve_T_, solve_iter_;
-    int p2g_stage_ = 32;       // see checkP2GStage()
     uint32_t g2p_cap_ = 1;   // G2P items per combination (rebuild)
     // launch settings per (stencil, transfer) combination (mpm_tuning)
     std::map<std::pair<int, int>, mpm_tuning> tuning_;
     bool tune_run_ = false;                          // autotune: sequential launches with events
     std::vector<std::array<cudaEvent_t, 4>> tune_ev_;  // per combination: P2G start/end, G2P start/end
-    bool stage_check_ = true;
+    bool warp_check_ = true;
     // the previous step's sorted keys are aligned with the live particle order
     // (sortLive may sort incrementally); MPM_FULL_SORT=1 always sorts all keys,
     // MPM_INCREMENTAL_SORT=1 sorts incrementally whatever the size (both for
@@ -2420,7 +2413,7 @@ private:
         outside_, counters_, block_slot_, tiles_, scenes_dev_, err_, tmp_, g2p_items_, tmaps_, spans_, p2g_lists_;
     // Per combination: the first step after a change of the scene set found
     // fewer than kWarpAutoMinItems small P2G items, so the step does not
-    // launch the warp kernel (see checkP2GStage, warpModeOf).
+    // launch the warp kernel (see checkWarpItems, warpModeOf).
     bool warp_few_[kMaxCombos] = {};
     bool profiling_ = false;
     bool step_timing_ = false;

@@ -30,6 +30,10 @@ constexpr int kSortTileKeys = kThreads * 8;  // keys per radix-sort tile (8 per 
 // scene -- P2G 0.150 and 0.144 ms against 0.145 ms -- and slowed the grid
 // pass, which sums more tiles per node.)
 constexpr uint32_t kBlockChunk = 4096;
+// Particles that a P2G warp stages at a time unless the caller sets it
+// (mpm_tuning.p2g_stage): a full warp.  16 and 24 were slower for every density
+// measured (two-ball P2G 0.128, 0.111 and 0.099 ms at 16, 24 and 32).
+constexpr int kDefaultP2GStage = 32;
 // G2P has no sums across particles, so its work items can be smaller without
 // changing any result: a block is split into ceil(count / chunk) G2P items,
 // which balances the persistent CTAs better than P2G's items.  The chunk is an

@@ -24,6 +24,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 namespace mpm {
 
@@ -436,286 +437,498 @@ __global__ void __launch_bounds__(kThreads) stressKernel(const SceneDev* __restr
 }
 
 // ---------------------------------------------------------------------------
-// P2G: one CTA per active 4^3-cell block (persistent loop).  Each warp takes
-// whole cells (dynamically, cell by cell); its lanes own the S^3 stencil
-// nodes of the cell and accumulate the cell's particles, in sorted order, in
-// registers.  Cell partial sums are merged into the (S+3)^3 block tile by a
-// fixed-order gather, and the tile is written to scratch.  Which warp takes a
-// cell does not matter: every sum has a fixed order, no floating-point
-// atomics, bitwise deterministic.
+// P2G.  The unit of summation is a row: the (up to) four cells of a block that
+// follow one another along x, so their particles follow one another in sorted
+// order.  A warp takes whole rows and keeps a window of S nodes along x, for
+// all S^2 columns (offsets b, c along y, z), in its lanes' registers: when the
+// row's particles have passed a node, its sums leave the window.  So a row
+// leaves one partial of (S+3) x S^2 nodes where one partial per cell would be
+// four of S^3.  The lanes form G groups that take a cell's particles in turn;
+// a lane holds kCols columns.  Every sum has a fixed order (a group's
+// particles in sorted order, the groups in a fixed tree, rows in order), there
+// are no floating-point atomics, and which warp takes a row does not matter:
+// bitwise deterministic.
 //
-// Staged payload of a particle (floats, 16-byte aligned rows):
-//   shared part (one broadcast float4 per 4 values)
-//     APIC / SPLIT : m, q[3] | hC[0..3] | hC[4..7] | hC[8], T[0..2] | T[3..5], -
-//                    q = m v - m C delta, hC = h m C (C = B D^-1), T = stress term
-//     PIC-FLIP     : m, m v[3] | T[0..3] | T[4..5], -, -
-//     MASS         : m, -, -, -
-//   weights: (N(d), N'(d)/h) pairs per axis and stencil offset (float2)
+// What bounds it: instruction issue and, in the inner loop, what a lane reads
+// per particle -- a 16-byte shared-memory load keeps the SM's load path busy
+// for four cycles, broadcast or not.  Hence the staging forms everything that
+// depends on the particle and one axis only.  With X, Y, Z the spline factors
+// of node (a, b, c) and X', Y', Z' their derivatives, a node's share of
+// (momentum + dt force)_i is
+//   w XX_a^i + X_a R^i,   w = Y_b Z_c,   R^i = Z_c Y_b^i + Y_b Z_c^i
+//   XX_a^i = X_a (q_i + a hC_i0) + X'_a T_i0
+//   Y_b^i  = b Y_b hC_i1 + Y'_b T_i1,   Z_c^i = c Z_c hC_i2 + Z'_c T_i2
+// (q = m v - m C delta, hC = h m C with C = B D^-1, T = stress term): 28 floats
+// read and 16 __ffma2_rn per particle and column for cubic splines.  Against
+// one partial per cell with the column factors formed in the inner loop (42
+// floats): two-ball scene (1M particles, 35 a cell) 0.134 -> 0.099 ms and 77M ->
+// 50M warp instructions, 8.4M-particle slab (3 a cell) 1.18 -> 0.95 ms, 2M
+// particles quadratic (36 a cell) 0.198 -> 0.139 ms, 65k-particle cube 0.035 ->
+// 0.021 ms.
+//
+// Staged payload of a particle, in 16-byte words (an odd number, so that the
+// same word of eight particles lies in different banks):
+//   APIC fused : (XX_a^x XX_a^y XX_a^z m X_a) [S] | X_0.. | (Y_b^x Y_b^y Y_b^z Y_b) [S] | (Z_c^i, Z_c) [S]
+//   PIC-FLIP   : (m v, m) | X_0.. | X'_0.. | (T_i0, -) | (Y'_b T_i1, Y_b) [S] | (Z'_c T_i2, Z_c) [S]
+//                momentum w X_a m v, force X'_a w T_i0 + X_a R^i
+//   SPLIT      : the first with T = 0, then X' | T_i0 | (Y'_b T_i1, -) [S] | (Z'_c T_i2, -) [S]
+//   MASS       : m X_0.. | Y_0.. | Z_0..
 // ---------------------------------------------------------------------------
-// Staging-record stride (floats): a multiple of 4 (float4 loads) whose
-// multiples q * P, q < groups, start at least 4 banks apart, so that the
-// broadcast loads of a warp's particle groups never share a bank.
-__host__ __device__ constexpr bool stageStrideOk(int P, int groups) {
-    for (int a = 0; a < groups; ++a)
-        for (int b = a + 1; b < groups; ++b) {
-            const int d = ((b - a) * P) % 32;
-            if (d < 4 || d > 28) return false;
-        }
-    return true;
-}
-__host__ __device__ constexpr int stageStride(int base, int groups) {
-    int P = (base + 3) / 4 * 4;
-    while (!stageStrideOk(P, groups)) P += 4;
-    return P;
-}
-
-// One lane's sums for one stencil node, in packed FP32 pairs so that the
-// x and y components go through one __ffma2_rn (two exactly rounded FMAs: the
-// same results as fmaf), and the mass with the z momentum:
-//   mz = (m, p_z), pxy = (p_x, p_y), fxy = (f_x, f_y), fz = f_z.
+// One lane's sums for one stencil node, in packed FP32 pairs so that two
+// components go through one __ffma2_rn (two exactly rounded FMAs):
+//   pxy = (p_x, p_y), pzm = (p_z, m), fxy = (f_x, f_y), fz = f_z.
 // Field f of the tile layout (m, p[3], f[3]) is get(f).
 struct NodeAcc {
-    float2 mz, pxy, fxy;
+    float2 pxy, pzm, fxy;
     float fz;
     __device__ __forceinline__ void zero() {
-        mz = pxy = fxy = make_float2(0.f, 0.f);
+        pxy = pzm = fxy = make_float2(0.f, 0.f);
         fz = 0.f;
     }
     __device__ __forceinline__ float get(int f) const {
-        return f == 0 ? mz.x : f == 1 ? pxy.x : f == 2 ? pxy.y : f == 3 ? mz.y : f == 4 ? fxy.x : f == 5 ? fxy.y : fz;
+        return f == 0 ? pzm.y : f == 1 ? pxy.x : f == 2 ? pxy.y : f == 3 ? pzm.x : f == 4 ? fxy.x : f == 5 ? fxy.y : fz;
     }
 };
 
-template <int S, int MODE, int STAGE = 16>
-struct P2GLayout {
+// A staged particle's layout (offsets in 16-byte words).
+template <int S, int MODE>
+struct P2GStage {
     static constexpr int F = modeFields(MODE);
-    static constexpr int NS = S * S * S;              // stencil nodes
-    static constexpr int PAIRS = S * S;               // (a, b) columns; a lane owns one column of S nodes
-    static constexpr int G = 32 / PAIRS;              // particle groups per warp (one particle each per pass)
+    static constexpr int T = S + 3;                   // nodes of a row along x
     static constexpr int TN = tileNodes(S);
-    static constexpr int SH = (MODE == MODE_MASS) ? 4 : (MODE == MODE_FLIP ? 12 : 20);  // shared floats
-    static constexpr int WB = SH;                     // weight pairs start
-    static constexpr int P = stageStride(SH + 6 * S, G);
-    static constexpr int kStage = STAGE;              // particles staged per warp round
-    static constexpr int kSlots = 32;                 // segment partials per round (<= 32: one per lane)
-    static constexpr int kSeg = 96;                   // particles per segment (at most)
-    static constexpr int kMaxSeg = 128;               // >= 64 + kBlockChunk / kSeg + 1
-    static constexpr int kCtlInts = 2 * 64 + 3 * kMaxSeg + 4;
-    // dynamic shared memory of nw warps: stage [nw][kStage][P] floats,
-    // partials [kSlots][F][NS] floats, then the control ints (cellBeg[64],
-    // cellEnd[64], segCell/segBeg/segEnd[kMaxSeg], ctl[4]); the kernel takes
-    // its pointers from these offsets
-    static constexpr size_t smemFor(int nw) {
-        return ((size_t)nw * kStage * P + (size_t)kSlots * F * NS) * 4 + (size_t)kCtlInts * 4;
-    }
-    // Threads per CTA.  Dense cubic scenes (staging 24 or 32 particles per
-    // pass) get two CTAs of 12 warps per SM where they fit its shared memory
-    // (at most ~113 KB each): 24 warps, the register file's limit at 80
-    // registers, working on two blocks.  Otherwise CTAs of 8 warps, three per
-    // SM where they fit: sparse scenes (staging 16, chosen below 8 particles
-    // per cell) have too few staging windows per block to keep 12 warps busy
-    // (8.4M-particle slab P2G 2.8 ms with 8 warps against 3.4 ms with 12).
-    static constexpr int NT = (S == 4 && STAGE >= 24 && smemFor(12) <= 113 * 1024) ? 384 : 256;
-    static constexpr int NW = NT / 32;
-    // CTAs per SM the launch bound asks for: as many as the shared memory
-    // holds (228 KB per SM, 1 KB of it reserved per CTA), at most 3 (80
-    // registers); the register budget follows from it.
-    static constexpr int MIN_CTAS = NT == 384 ? 2 : ((smemFor(8) + 1024) * 3 <= 228 * 1024 ? 3 : 2);
-    static constexpr int TJ = (TN + NT - 1) / NT;
-    static constexpr size_t kPartialOff = (size_t)NW * kStage * P;
-    static constexpr size_t kCtlOff = kPartialOff + (size_t)kSlots * F * NS;
-    static constexpr size_t smemBytes = smemFor(NW);
-    static_assert(smemBytes == kCtlOff * 4 + (size_t)kCtlInts * 4, "layout");
-    static_assert(kMaxSeg >= 64 + (int)(kBlockChunk / kSeg) + 1, "segment list too small");
+    static constexpr bool kC = MODE == MODE_APIC_FUSED || MODE == MODE_SPLIT;  // XX words
+    static constexpr bool kSepF = MODE == MODE_FLIP || MODE == MODE_SPLIT;     // force apart from momentum
+    static constexpr int WXX = 0;                     // XX (or m v, m)
+    static constexpr int WX = MODE == MODE_MASS ? 0 : (kC ? S : 1);
+    static constexpr int WXD = WX + 1;                // X' (kSepF), then T_i0
+    static constexpr int WT = WXD + 1;
+    static constexpr int WY = MODE == MODE_MASS ? 1 : (kSepF ? WT + 1 : WX + 1);
+    static constexpr int WZ = WY + (MODE == MODE_MASS ? 1 : S);
+    static constexpr int WYF = MODE == MODE_SPLIT ? WZ + S : WY;  // the force's Y and Z words
+    static constexpr int WZF = MODE == MODE_SPLIT ? WYF + S : WZ;
+    static constexpr int kWords = WZF + (MODE == MODE_MASS ? 1 : S);
+    static constexpr int P4 = kWords | 1;             // 16-byte words per staged particle
+    static constexpr int kSeg = 192;                  // particles per row segment (at most)
 };
 
-// P2G staging of one particle (sorted position gs) at `my`: mass, momentum
-// terms, stress factors and stencil weights in the layout of P2GStage.  The
-// CTA and warp P2G kernels share it (and p2gAccumulate), so their sums are
-// bitwise the same.
-template <int S, int MODE, int P, int WB>
-__device__ __forceinline__ void p2gStageParticle(const StepArgs& args, const SceneDev& sc, const float* pf, size_t cap,
-                                                 float dt, float h, float inv_h, uint32_t gs, float* my) {
-    uint32_t old = args.perm[gs] - sc.key_offset;
-    const bool bad = old >= sc.n;  // range check: flag and contribute nothing
-    if (bad) {
-        atomicOr(args.err, ERR_INDEX);
-        old = 0;
+// How a warp's lanes share a row: G particle groups, each lane one column:
+// lane = group + G (b + S c).  (Two columns a lane and 4 groups for cubic, the
+// three of a b and 8 groups for quadratic read half as much shared memory per
+// particle, but double or treble the accumulators and the sums over the groups
+// at every flushed node: two-ball P2G 0.102 against 0.104 ms, 2M-particle
+// quadratic scene 0.143 against 0.139 ms, 8.4M-particle slab 1.12 against
+// 0.95 ms.)
+template <int S, int MODE>
+struct P2GLanes {
+    static constexpr int F = modeFields(MODE);
+    static constexpr int G = S == 4 ? 2 : (S == 3 ? 3 : 8);
+    // A flushed node's F values are summed over the groups; a lane then owns
+    // kOut of them (see groupReduce).
+    static constexpr int half(int n) { return (n + 1) / 2; }
+    static constexpr int kOut = G == 3 ? F : G == 2 ? half(F) : half(half(half(F)));
+    int grp, b, c;
+    bool on;
+    __device__ __forceinline__ explicit P2GLanes(int lane) {
+        grp = lane % G;
+        b = (lane / G) % S;
+        c = (lane / G) / S;
+        on = c < S;
     }
-    float x[3] = {ldg(pf + (F_X + 0) * cap + old), ldg(pf + (F_X + 1) * cap + old),
-                  ldg(pf + (F_X + 2) * cap + old)};
-    int base[3];
-    stencilBase(sc, x, base);
-    float delta[3];
+    // The first particle >= lo (index in its segment) that this lane's group
+    // takes: a segment's particles go to the groups in turn, however it is
+    // cut into passes and cells.
+    __device__ __forceinline__ int first(int lo) const {
+        const int r = lo % G;
+        return grp >= r ? grp - r : grp - r + G;
+    }
+};
+
+// Sums over the groups of the warp of the values v[0..N-1].  A power of two of
+// groups: halving exchanges (each step a lane passes on half of its values and
+// adds the other half), the lane's share ends up in v[0..kOut-1].  Three
+// groups: added in turn, valid in group 0.
+template <int N, int BIT, int G>
+__device__ __forceinline__ void groupReduce(float* v, int lane) {
+    if constexpr (G == 3) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float s1 = __shfl_down_sync(0xffffffffu, v[i], 1), s2 = __shfl_down_sync(0xffffffffu, v[i], 2);
+            v[i] = (v[i] + s1) + s2;
+        }
+    } else if constexpr (BIT < G) {
+        constexpr int H = (N + 1) / 2;
+        const bool up = (lane & BIT) != 0;
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const float hi = i + H < N ? v[i + H] : 0.f;
+            const float mine = up ? hi : v[i], other = up ? v[i] : hi;
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, other, BIT);
+        }
+        groupReduce<H, 2 * BIT, G>(v, lane);
+    }
+}
+// The index of the value that ends up in v[i] of a lane of
+// group `grp`, or -1 where the lane has none.
+template <int N, int BIT, int G>
+__device__ __forceinline__ int valueOf(int i, int grp) {
+    if constexpr (G == 3) {
+        return grp == 0 ? i : -1;
+    } else if constexpr (BIT < G) {
+        constexpr int H = (N + 1) / 2;
+        const int k = valueOf<H, 2 * BIT, G>(i, grp);
+        if (k < 0) return -1;
+        const int j = (grp & BIT) ? k + H : k;
+        return j < N ? j : -1;
+    } else {
+        return i < N ? i : -1;
+    }
+}
+
+// Origin (node index) of the (S+3)^3 tile of an active block: 4 B - 4 per axis.
+__device__ __forceinline__ void tileOrigin(const SceneDev& sc, uint32_t block, int* t0) {
+    const uint32_t lb = block - sc.block_base;
+    t0[0] = 4 * (int)(lb % (uint32_t)sc.nb[0]) - 4;
+    t0[1] = 4 * (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]) - 4;
+    t0[2] = 4 * (int)(lb / ((uint32_t)sc.nb[0] * (uint32_t)sc.nb[1])) - 4;
+}
+
+// num / h with one correction by the remainder (Markstein's method): as exact
+// as a division of these operands, in three instructions.
+__device__ __forceinline__ float quotient(float num, float h, float inv_h) {
+    const float q = num * inv_h;
+    return fmaf(fmaf(-q, h, num), inv_h, q);
+}
+
+// What P2G reads of a particle, in registers: loaded one staging pass ahead, so
+// that the loads are in flight while the warp accumulates the pass before.
+template <int S, int MODE>
+struct P2GRaw {
+    using R = P2GStage<S, MODE>;
+    float x[3], m, v[3], t[6], B[9];
+    bool bad;  // range check failed: the particle contributes nothing
+    __device__ __forceinline__ void load(const StepArgs& args, const SceneDev& sc, const float* pf, size_t cap,
+                                         uint32_t perm) {
+        uint32_t old = perm - sc.key_offset;
+        bad = old >= sc.n;
+        if (bad) {
+            atomicOr(args.err, ERR_INDEX);
+            old = 0;
+        }
+        const float* pp = pf + old;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) x[a] = ldg(pp + (F_X + a) * cap);
+        m = ldg(pp + F_MASS * cap);
+        if constexpr (MODE == MODE_MASS) return;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[a] = ldg(pp + (F_V + a) * cap);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t[k] = ldg(pp + (F_TAU + k) * cap);
+        if (MODE == MODE_APIC_FUSED || (MODE == MODE_SPLIT && sc.transfer == MPM_TRANSFER_APIC)) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) B[k] = ldg(pp + (F_B + k) * cap);
+        } else if (MODE == MODE_SPLIT) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) B[k] = 0.f;
+        }
+    }
+};
+
+// Staging of one particle (of `cell` in the block whose tile starts at t0) at
+// `my`, in the layout above.  The stencil base comes from the cell, which the
+// key was formed from.
+template <int S, int MODE>
+__device__ __forceinline__ void p2gStageParticle(const SceneDev& sc, const P2GRaw<S, MODE>& raw, float dt, float h,
+                                                 float inv_h, const int* t0, uint32_t cell, float4* my) {
+    using R = P2GStage<S, MODE>;
+    const float (&x)[3] = raw.x;
+    const float (&v)[3] = raw.v;
+    const float m = raw.bad ? 0.f : raw.m;
+    float t[6], mC[9];
+    if (MODE != MODE_MASS) {
+        const float ts = raw.bad ? 0.f : (MODE == MODE_APIC_FUSED ? -dt : -1.0f);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t[k] = ts * raw.t[k];
+        if (R::kC) {
+            const float md = m * sc.dinv;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) mC[k] = md * raw.B[k];
+        }
+    }
+    const int base[3] = {t0[0] + (int)(cell & 3u), t0[1] + (int)((cell >> 2) & 3u), t0[2] + (int)(cell >> 4)};
+    float delta[3], wk[3][S], dwk[3][S];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float gp0 = __fadd_rn(sc.origin[a], __fmul_rn(h, (float)base[a]));
         delta[a] = x[a] - gp0;
-        // Node distances.  The linear kernel's weights
-        // have relative error ~ulp(d)/w near |d| = 1, so it
-        // forms each one as the reference does,
-        // (x_p - (o + h i)) / h; the B-splines are smooth
-        // there and use d0 - k (exact subtraction).
-        float dk[S], wk[S], dwk[S];
+        // Node distances.  The linear kernel's weights have relative error
+        // ~ulp(d)/w near |d| = 1, so it forms each one as the reference does,
+        // (x_p - (o + h i)) / h; the B-splines are smooth there and use
+        // d0 - k (exact subtraction).
+        float dk[S];
         if (S == 2) {
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 const float gp = __fadd_rn(sc.origin[a], __fmul_rn(h, (float)(base[a] + k)));
-                dk[k] = __fdiv_rn(__fsub_rn(x[a], gp), h);
+                dk[k] = quotient(__fsub_rn(x[a], gp), h, inv_h);
             }
         } else {
-            dk[0] = __fdiv_rn(delta[a], h);
+            dk[0] = quotient(delta[a], h, inv_h);
 #pragma unroll
             for (int k = 1; k < S; ++k) dk[k] = dk[0] - (float)k;
         }
-        splineWeights<S>(dk, wk, dwk);
+        splineWeights<S>(dk, wk[a], dwk[a]);
+#pragma unroll
+        for (int k = 0; k < S; ++k) dwk[a][k] *= inv_h;
+    }
+    auto row4 = [](const float* w) {
+        return make_float4(w[0], w[1], S > 2 ? w[S > 2 ? 2 : 0] : 0.f, S > 3 ? w[S > 3 ? 3 : 0] : 0.f);
+    };
+    if (MODE == MODE_MASS) {
+        float mx[S];
+#pragma unroll
+        for (int k = 0; k < S; ++k) mx[k] = m * wk[0][k];
+        my[R::WXX] = row4(mx);
+        my[R::WY] = row4(wk[1]);
+        my[R::WZ] = row4(wk[2]);
+        return;
+    }
+    my[R::WX] = row4(wk[0]);
+    if (R::kC) {
+        float q[3], hC[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            q[i] = m * v[i] - (mC[3 * i] * delta[0] + mC[3 * i + 1] * delta[1] + mC[3 * i + 2] * delta[2]);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) hC[k] = h * mC[k];
+        const float tx[3] = {t[0], t[3], t[4]}, ty[3] = {t[3], t[1], t[5]}, tz[3] = {t[4], t[5], t[2]};
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-            if (MODE == MODE_MASS) {
-                my[WB + a * S + k] = wk[k];
-            } else {  // (w, w'/h) pairs: 8-byte stores (WB is even, rows 16-byte aligned)
-                *reinterpret_cast<float2*>(my + WB + 2 * (a * S + k)) = make_float2(wk[k], dwk[k] * inv_h);
+            const float wy = (float)k * wk[1][k], wz = (float)k * wk[2][k];
+            float xx[3], yy[3], zz[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                xx[i] = wk[0][k] * fmaf((float)k, hC[3 * i], q[i]);
+                yy[i] = wy * hC[3 * i + 1];
+                zz[i] = wz * hC[3 * i + 2];
+                if (MODE == MODE_APIC_FUSED) {
+                    xx[i] = fmaf(dwk[0][k], tx[i], xx[i]);
+                    yy[i] = fmaf(dwk[1][k], ty[i], yy[i]);
+                    zz[i] = fmaf(dwk[2][k], tz[i], zz[i]);
+                }
             }
+            my[R::WXX + k] = make_float4(xx[0], xx[1], xx[2], m * wk[0][k]);
+            my[R::WY + k] = make_float4(yy[0], yy[1], yy[2], wk[1][k]);
+            my[R::WZ + k] = make_float4(zz[0], zz[1], zz[2], wk[2][k]);
         }
+    } else {
+        my[R::WXX] = make_float4(m * v[0], m * v[1], m * v[2], m);
     }
-    const float m = bad ? 0.f : ldg(pf + F_MASS * cap + old);
-    if (MODE == MODE_MASS) my[0] = m;
-    if (MODE != MODE_MASS) {
-        float v[3] = {ldg(pf + (F_V + 0) * cap + old), ldg(pf + (F_V + 1) * cap + old),
-                      ldg(pf + (F_V + 2) * cap + old)};
-        const float ts = bad ? 0.f : ((MODE == MODE_APIC_FUSED) ? -dt : -1.0f);
-        float T[6];
+    if (R::kSepF) {
+        my[R::WXD] = row4(dwk[0]);
+        my[R::WT] = make_float4(t[0], t[3], t[4], 0.f);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) T[k] = ts * ldg(pf + (F_TAU + k) * cap + old);
-        // the row's header in 16-byte stores: (m, p), then the stress
-        // factors (and APIC's h m C): the layout the accumulation reads
-        float4* my4 = reinterpret_cast<float4*>(my);
-        if (MODE == MODE_FLIP) {
-            my4[0] = make_float4(m, m * v[0], m * v[1], m * v[2]);
-            my4[1] = make_float4(T[0], T[1], T[2], T[3]);
-            *reinterpret_cast<float2*>(my + 8) = make_float2(T[4], T[5]);
-        } else {
-            float mC[9];
-            if (sc.transfer == MPM_TRANSFER_APIC) {
-                const float md = m * sc.dinv;
-#pragma unroll
-                for (int k = 0; k < 9; ++k) mC[k] = md * ldg(pf + (F_B + k) * cap + old);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 9; ++k) mC[k] = 0.f;
-            }
-            float q[3], hC[9];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-                q[a] = m * v[a] - (mC[3 * a] * delta[0] + mC[3 * a + 1] * delta[1] + mC[3 * a + 2] * delta[2]);
-#pragma unroll
-            for (int k = 0; k < 9; ++k) hC[k] = h * mC[k];
-            my4[0] = make_float4(m, q[0], q[1], q[2]);
-            my4[1] = make_float4(hC[0], hC[1], hC[2], hC[3]);
-            my4[2] = make_float4(hC[4], hC[5], hC[6], hC[7]);
-            my4[3] = make_float4(hC[8], T[0], T[1], T[2]);
-            my4[4] = make_float4(T[3], T[4], T[5], 0.f);  // [19] is padding of the header
+        for (int k = 0; k < S; ++k) {
+            const float dy = dwk[1][k], dz = dwk[2][k];
+            my[R::WYF + k] = make_float4(dy * t[3], dy * t[1], dy * t[5], wk[1][k]);
+            my[R::WZF + k] = make_float4(dz * t[4], dz * t[5], dz * t[2], wk[2][k]);
         }
     }
 }
 
+__device__ __forceinline__ float pick(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
+
 // One lane's sums over the staged particles q0, q0 + G, ... below qhi (its
-// group's share of a segment, in order) for the stencil column (na, nb).
-template <int S, int MODE, int P, int WB, int G>
-__device__ __forceinline__ void p2gAccumulate(const float* st, int q0, int qhi, int na, int nb, NodeAcc* acc) {
-    const float fa = (float)na, fb = (float)nb;
-    for (int q = q0; q < qhi; q += G) {
-        const float* pq = st + q * P;
-        const float4 s0 = *reinterpret_cast<const float4*>(pq);
-        const float m = s0.x;
+// group's share of a cell at x offset X in its row, in order) for the column
+// (b, c).  The window's register of tile node n is n % S, so the cell's nodes a
+// sit in acc[(X + a) % S].
+template <int S, int MODE, int X>
+__device__ __forceinline__ void p2gAccumulate(const float4* st, int q0, int qhi, int b, int c, NodeAcc (&acc)[S]) {
+    using R = P2GStage<S, MODE>;
+#pragma unroll 1
+    for (int q = q0; q < qhi; q += P2GLanes<S, MODE>::G) {
+        const float4* pq = st + q * R::P4;
         if (MODE == MODE_MASS) {
-            const float mw = m * (pq[WB + na] * pq[WB + S + nb]);
+            const float4 xm = pq[R::WXX];
+            const float w = reinterpret_cast<const float*>(pq + R::WY)[b] * reinterpret_cast<const float*>(pq + R::WZ)[c];
 #pragma unroll
-            for (int c = 0; c < S; ++c) acc[c].mz.x = fmaf(mw, pq[WB + 2 * S + c], acc[c].mz.x);
+            for (int a = 0; a < S; ++a) acc[(X + a) % S].pzm.y = fmaf(w, pick(xm, a), acc[(X + a) % S].pzm.y);
             continue;
         }
-        // column factors: w = wab Z_c and
-        // T grad w = Z_c A + Z'_c Bz with A = T (X'Y, XY', 0), Bz = T (0, 0, XY)
-        const float2 xa = *reinterpret_cast<const float2*>(pq + WB + 2 * na);
-        const float2 yb = *reinterpret_cast<const float2*>(pq + WB + 2 * (S + nb));
-        const float wab = xa.x * yb.x, dab = xa.y * yb.x, adb = xa.x * yb.y;
-        float T[6];
-        float2 uxy, mu;  // (u_x, u_y) and (m, u_z)
-        float2 hxy = make_float2(0.f, 0.f);
-        float hz = 0.f;
-        if (MODE == MODE_FLIP) {
-            const float4 s1 = *reinterpret_cast<const float4*>(pq + 4);
-            const float4 s2 = *reinterpret_cast<const float4*>(pq + 8);
-            T[0] = s1.x; T[1] = s1.y; T[2] = s1.z; T[3] = s1.w; T[4] = s2.x; T[5] = s2.y;
-            uxy = make_float2(s0.y, s0.z);
-            mu = make_float2(m, s0.w);
-        } else {
-            const float4 s1 = *reinterpret_cast<const float4*>(pq + 4);
-            const float4 s2 = *reinterpret_cast<const float4*>(pq + 8);
-            const float4 s3 = *reinterpret_cast<const float4*>(pq + 12);
-            const float4 s4 = *reinterpret_cast<const float4*>(pq + 16);
-            const float hC[9] = {s1.x, s1.y, s1.z, s1.w, s2.x, s2.y, s2.z, s2.w, s3.x};
-            T[0] = s3.y; T[1] = s3.z; T[2] = s3.w; T[3] = s4.x; T[4] = s4.y; T[5] = s4.z;
-            const float qv[3] = {s0.y, s0.z, s0.w};
-            float u[3];
+        const float4 xw = pq[R::WX], y = pq[R::WY + b], z = pq[R::WZ + c];
+        const float w = y.w * z.w;
+        const float2 w2 = dup2(w);
+        if (R::kC) {
+            const float2 Rxy = __ffma2_rn(dup2(z.w), make_float2(y.x, y.y), __fmul2_rn(dup2(y.w), make_float2(z.x, z.y)));
+            const float2 Rz0 = make_float2(fmaf(z.w, y.z, y.w * z.z), 0.f);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) u[i] = fmaf(hC[3 * i], fa, fmaf(hC[3 * i + 1], fb, qv[i]));
-            uxy = make_float2(u[0], u[1]);
-            mu = make_float2(m, u[2]);
-            hxy = make_float2(hC[2], hC[5]);
-            hz = hC[8];
-        }
-        const float2 Axy = make_float2(fmaf(T[0], dab, T[3] * adb), fmaf(T[3], dab, T[1] * adb));
-        const float Az = fmaf(T[4], dab, T[5] * adb);
-        const float2 Bxy = make_float2(T[4] * wab, T[5] * wab);
-        const float Bz = T[2] * wab;
-#pragma unroll
-        for (int c = 0; c < S; ++c) {
-            const float2 zc = *reinterpret_cast<const float2*>(pq + WB + 2 * (2 * S + c));
-            const float wgt = wab * zc.x;
-            const float2 w2 = make_float2(wgt, wgt), zx2 = make_float2(zc.x, zc.x),
-                         zy2 = make_float2(zc.y, zc.y);
-            if (c > 0 && MODE != MODE_FLIP) {  // u at node c: u += h C e_z, component-wise
-                uxy = __fadd2_rn(uxy, hxy);
-                mu.y += hz;
+            for (int a = 0; a < S; ++a) {
+                NodeAcc& n = acc[(X + a) % S];
+                const float4 xx = pq[R::WXX + a];
+                const float2 xa = dup2(pick(xw, a));
+                n.pxy = __ffma2_rn(w2, make_float2(xx.x, xx.y), __ffma2_rn(xa, Rxy, n.pxy));
+                n.pzm = __ffma2_rn(w2, make_float2(xx.z, xx.w), __ffma2_rn(xa, Rz0, n.pzm));
             }
-            // m += m w and p_z += w u_z in one pair
-            acc[c].mz = __ffma2_rn(mu, w2, acc[c].mz);
-            if (MODE == MODE_APIC_FUSED) {
-                // p += w u + Z_c A + Z'_c Bz (the order of the nested fmaf)
-                acc[c].pxy = __ffma2_rn(zy2, Bxy, __ffma2_rn(zx2, Axy, __ffma2_rn(w2, uxy, acc[c].pxy)));
-                acc[c].mz.y = fmaf(zc.y, Bz, fmaf(zc.x, Az, acc[c].mz.y));
-            } else {  // PIC-FLIP and SPLIT keep p and f apart
-                acc[c].pxy = __ffma2_rn(w2, uxy, acc[c].pxy);
-                acc[c].fxy = __ffma2_rn(zy2, Bxy, __ffma2_rn(zx2, Axy, acc[c].fxy));
-                acc[c].fz = fmaf(zc.y, Bz, fmaf(zc.x, Az, acc[c].fz));
+        } else {
+            const float4 mv = pq[R::WXX];
+            const float2 Pxy = __fmul2_rn(w2, make_float2(mv.x, mv.y)), Pzm = __fmul2_rn(w2, make_float2(mv.z, mv.w));
+#pragma unroll
+            for (int a = 0; a < S; ++a) {
+                NodeAcc& n = acc[(X + a) % S];
+                const float2 xa = dup2(pick(xw, a));
+                n.pxy = __ffma2_rn(xa, Pxy, n.pxy);
+                n.pzm = __ffma2_rn(xa, Pzm, n.pzm);
+            }
+        }
+        if (R::kSepF) {
+            const float4 xd = pq[R::WXD], t0 = pq[R::WT];
+            const float4 yf = MODE == MODE_SPLIT ? pq[R::WYF + b] : y, zf = MODE == MODE_SPLIT ? pq[R::WZF + c] : z;
+            const float2 Rxy =
+                __ffma2_rn(dup2(z.w), make_float2(yf.x, yf.y), __fmul2_rn(dup2(y.w), make_float2(zf.x, zf.y)));
+            const float Rz = fmaf(z.w, yf.z, y.w * zf.z);
+            const float2 Bxy = __fmul2_rn(w2, make_float2(t0.x, t0.y));
+            const float Bz = w * t0.z;
+#pragma unroll
+            for (int a = 0; a < S; ++a) {
+                NodeAcc& n = acc[(X + a) % S];
+                const float xa = pick(xw, a), da = pick(xd, a);
+                n.fxy = __ffma2_rn(dup2(da), Bxy, __ffma2_rn(dup2(xa), Rxy, n.fxy));
+                n.fz = fmaf(da, Bz, fmaf(xa, Rz, n.fz));
             }
         }
     }
 }
+
+// A warp's state within a row segment, and one staging pass of it.
+template <int S, int MODE>
+struct RowWindow {
+    using L = P2GLanes<S, MODE>;
+    NodeAcc acc[S];
+    int col;         // tile x of the first node still in the window
+    unsigned cells;  // cells of the segment that had particles
+    __device__ __forceinline__ void reset() {
+        col = 0;
+        cells = 0u;
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int a = 0; a < S; ++a) acc[a].zero();
+        reset();
+    }
+    // Tile node n along x is final: its sums over the groups go to out(n, v),
+    // v the lane's share; where no cell touched it, out(n, null).
+    template <int N, class Out>
+    __device__ __forceinline__ void flush(int lane, Out&& out) {
+        constexpr unsigned touch = ((((1u << S) - 1u) << N) >> (S - 1)) & 15u;  // cells N - S + 1 .. N
+        if (cells & touch) {
+            float v[L::F];
+#pragma unroll
+            for (int f = 0; f < L::F; ++f) v[f] = acc[N % S].get(f);
+            acc[N % S].zero();
+            groupReduce<L::F, 1, L::G>(v, lane);
+            out(N, v);
+        } else {
+            out(N, (const float*)nullptr);
+        }
+    }
+    // The staged particles [qlo, qhi) of a pass, which belong to one segment of
+    // row `row`; cl is the lane's staged particle's cell, j0 the index in the
+    // segment of particle qlo.  Nodes x < lim are final after it (lim = 4:
+    // the segment ends, and all are).
+    template <class Out>
+    __device__ __forceinline__ void pass(const float4* st, uint32_t cl, int qlo, int qhi, int row, int j0, int lim,
+                                         int lane, const L& ln, Out&& out) {
+        const bool mine = lane >= qlo && lane < qhi;
+        step<0>(st, cl, mine, qlo, row, j0, lim, lane, ln, out);
+        step<1>(st, cl, mine, qlo, row, j0, lim, lane, ln, out);
+        step<2>(st, cl, mine, qlo, row, j0, lim, lane, ln, out);
+        step<3>(st, cl, mine, qlo, row, j0, lim, lane, ln, out);
+        if (lim == 4) {
+            flush<4>(lane, out);
+            if constexpr (S > 2) flush<5>(lane, out);
+            if constexpr (S > 3) flush<6>(lane, out);
+            reset();
+        }
+    }
+    template <int X, class Out>
+    __device__ __forceinline__ void step(const float4* st, uint32_t cl, bool mine, int qlo, int row, int j0, int lim,
+                                         int lane, const L& ln, Out&& out) {
+        const unsigned m = __ballot_sync(0xffffffffu, mine && cl == (uint32_t)(4 * row + X));
+        if (m) {
+            const int a = __ffs(m) - 1, e = a + __popc(m);
+            if (ln.on) p2gAccumulate<S, MODE, X>(st, a + ln.first(j0 + a - qlo), e, ln.b, ln.c, acc);
+            cells |= 1u << X;
+        }
+        if (X < lim && col == X) {
+            flush<X>(lane, out);
+            col = X + 1;
+        }
+    }
+};
+
+// Row starts of an item's `count` particles (keys sorted by cell): row r's
+// particles are [beg[r], beg[r + 1]), r < 16.  Thread t of nt writes those of
+// the rows that begin at its particles.
+__device__ __forceinline__ void findRows(const uint32_t* keys, int count, int* beg, int t, int nt) {
+#pragma unroll 4
+    for (int i = t; i < count; i += nt) {
+        const int r = (int)((keys[i] & 63u) >> 2), before = i ? (int)((keys[i - 1] & 63u) >> 2) : -1;
+        for (int q = before + 1; q <= r; ++q) beg[q] = i;
+        if (i == count - 1)
+            for (int q = r + 1; q <= 16; ++q) beg[q] = count;
+    }
+}
+
+template <int S, int MODE, int STAGE = 16>
+struct P2GLayout : P2GStage<S, MODE> {
+    using R = P2GStage<S, MODE>;
+    static constexpr int F = R::F, T = R::T;
+    static constexpr int kStage = STAGE;              // particles staged per warp pass
+    static constexpr int kSlots = 16;                 // segment partials per round: a block's rows, one segment each
+    // Floats between a partial's x nodes: with 18 (cubic), 9 (quadratic) and
+    // 4 (linear) the gather's (x, y) neighbours fall in different banks.
+    static constexpr int CS = S == 4 ? 18 : S * S;
+    static constexpr int kSlotFloats = F * T * CS;
+    static constexpr int kMaxSeg = 48;                // >= 16 + kBlockChunk / kSeg + 1
+    static constexpr int kCtlInts = 17 + 3 * kMaxSeg + 4 + 3;
+    // dynamic shared memory of nw warps: stage [nw][kStage][P4] 16-byte words,
+    // partials [kSlots][F][T][CS] floats, then the control ints (rowBeg[17],
+    // segRow/segBeg/segEnd[kMaxSeg], ctl[4]); the kernel takes its pointers
+    // from these offsets
+    static constexpr size_t smemFor(int nw) {
+        return (size_t)nw * kStage * R::P4 * 16 + (size_t)kSlots * kSlotFloats * 4 + (size_t)kCtlInts * 4;
+    }
+    static constexpr bool kThreeOf8 = (smemFor(8) + 1024) * 3 <= 228 * 1024;
+    // Threads per CTA: three CTAs of 8 warps per SM where the shared memory
+    // holds them (228 KB per SM, 1 KB of it reserved per CTA), else two.
+    static constexpr int NT = 256;
+    static constexpr int NW = NT / 32;
+    static constexpr int MIN_CTAS = kThreeOf8 && S * F <= 16 ? 3 : 2;
+    static constexpr int TJ = (R::TN + NT - 1) / NT;
+    static constexpr size_t kPartialOff = (size_t)NW * kStage * R::P4 * 4;  // floats
+    static constexpr size_t kCtlOff = kPartialOff + (size_t)kSlots * kSlotFloats;
+    static constexpr size_t smemBytes = smemFor(NW);
+    static_assert(smemBytes == kCtlOff * 4 + (size_t)kCtlInts * 4, "layout");
+    static_assert(kMaxSeg >= 16 + (int)(kBlockChunk / R::kSeg) + 1, "segment list too small");
+    static_assert(kSlots <= 32 && kStage <= 32, "a round's segments and a pass's particles: one per lane");
+};
 
 template <int S, int MODE, int STAGE>
 __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MODE, STAGE>::MIN_CTAS)
     p2gKernel(StepArgs args, int want_transfer) {
     using L = P2GLayout<S, MODE, STAGE>;
-    constexpr int F = L::F;
+    constexpr int F = L::F, T = L::T, TN = L::TN, CS = L::CS;
     extern __shared__ float4 smem4[];
     float* smem = reinterpret_cast<float*>(smem4);
-    float* stage = smem;                     // [warp][kStage][P]
-    float* partial = smem + L::kPartialOff;  // [slot][F][NS]
-    int* cellBeg = (int*)(smem + L::kCtlOff);
-    int* cellEnd = cellBeg + 64;
-    int* segCell = cellEnd + 64;                                // segment list, in cell order
-    int* segBeg = segCell + L::kMaxSeg;
+    float* partial = smem + L::kPartialOff;  // [slot][F][T][CS]
+    int* rowBeg = (int*)(smem + L::kCtlOff); // item index of each row's first particle, then the item's count
+    int* segRow = rowBeg + 17;                                  // segment list, in row order
+    int* segBeg = segRow + L::kMaxSeg;
     int* segEnd = segBeg + L::kMaxSeg;
-    int* ctl = segEnd + L::kMaxSeg;                             // [0] segments, [1] next segment
+    int* ctl = segEnd + L::kMaxSeg;                             // [0] segments, [1] next window
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // lane -> particle group grp and stencil column (na, nb): the lane
-    // accumulates nodes (na, nb, 0..S-1) for the group's particles
-    // grp, grp + G, grp + 2G, ... of each staged batch.
-    const int grp = lane / L::PAIRS, na = (lane % L::PAIRS) % S, nb = (lane % L::PAIRS) / S;
-    const bool lane_on = grp < L::G;
+    float4* st = smem4 + (size_t)warp * L::kStage * L::P4;
     // the combination's list of items for whole CTAs, or every active item
     const uint32_t* list = args.p2g_lists ? args.p2g_lists + (size_t)(2 * args.combo + 1) * args.p2g_list_cap : nullptr;
     // the long items from the list's front first, then the others from its
@@ -742,51 +955,35 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
             if (scg.S != S || (want_transfer >= 0 && scg.transfer != want_transfer)) continue;
             if (MODE == MODE_MASS && !scg.init_pass) continue;
         }
-        // the scene's entry into shared memory: the staging reads its fields
-        // per particle
+        const uint32_t i0 = it.start;
+        const int icount = (int)it.count;
+        const uint32_t* keys = args.sorted_keys + i0;
+        const uint32_t* perm = args.perm + i0;
+        // the scene's entry into shared memory (the staging reads its fields
+        // per particle)
         if (warp == 0) {
             const int4* src = reinterpret_cast<const int4*>(args.scenes + it.scene);
             int4* dst = reinterpret_cast<int4*>(&sc_s);
             for (int q = lane; q < (int)(sizeof(SceneDev) / 16); q += 32) dst[q] = src[q];
         }
-        for (int c = threadIdx.x; c < 64; c += L::NT) cellBeg[c] = cellEnd[c] = 0;
+        findRows(keys, icount, rowBeg, (int)threadIdx.x, L::NT);
         __syncthreads();
-        const SceneDev& sc = sc_s;
-        const float* pf = sc.buf[args.parity].f;
-        const size_t cap = sc.cap;
-        const uint32_t i0 = it.start, icount = it.count;
-
-        // Cell ranges inside the work item (keys are sorted by cell).
-        for (uint32_t i = threadIdx.x; i < icount; i += L::NT) {
-            uint32_t g = i0 + i;
-            uint32_t c = args.sorted_keys[g] & 63u;
-            if (i == 0 || (args.sorted_keys[g - 1] & 63u) != c) cellBeg[c] = (int)i;
-            if (i == icount - 1 || (args.sorted_keys[g + 1] & 63u) != c) cellEnd[c] = (int)i + 1;
-        }
-        __syncthreads();
-        // Segment list: every non-empty cell cut into runs of at most kSeg
-        // particles, in cell order (warp 0; lane l owns cells 2l and 2l+1).
         if (warp == 0) {
-            const int c0 = 2 * lane, c1 = 2 * lane + 1;
-            const int b0 = cellBeg[c0], e0 = cellEnd[c0], b1 = cellBeg[c1], e1 = cellEnd[c1];
-            const int n0 = e0 > b0 ? (e0 - b0 + L::kSeg - 1) / L::kSeg : 0;
-            const int n1 = e1 > b1 ? (e1 - b1 + L::kSeg - 1) / L::kSeg : 0;
-            int x = n0 + n1;
+            // Segment list: every non-empty row cut into equal runs of at most
+            // kSeg particles, in row order (lane r < 16 owns row r).
+            const int lo = lane < 16 ? rowBeg[lane] : 0, end = lane < 16 ? rowBeg[lane + 1] : 0;
+            const int len = end - lo, n = (len + L::kSeg - 1) / L::kSeg;
+            int x = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o) x += y;
             }
-            int off = x - (n0 + n1);
-            for (int j = 0; j < n0; ++j, ++off) {
-                segCell[off] = c0;
-                segBeg[off] = b0 + j * L::kSeg;
-                segEnd[off] = min(e0, b0 + (j + 1) * L::kSeg);
-            }
-            for (int j = 0; j < n1; ++j, ++off) {
-                segCell[off] = c1;
-                segBeg[off] = b1 + j * L::kSeg;
-                segEnd[off] = min(e1, b1 + (j + 1) * L::kSeg);
+            int o = x - n;
+            for (int j = 0; j < n; ++j, ++o) {
+                segRow[o] = lane;
+                segBeg[o] = lo + len * j / n;
+                segEnd[o] = lo + len * (j + 1) / n;
             }
             if (lane == 31) {
                 ctl[0] = x;
@@ -794,109 +991,120 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
             }
         }
         __syncthreads();
+        const SceneDev& sc = sc_s;
+        const float* pf = sc.buf[args.parity].f;
+        const size_t cap = sc.cap;
         const int nseg = ctl[0];
-
-        float tacc[L::TJ][F];
-#pragma unroll
-        for (int j = 0; j < L::TJ; ++j)
-#pragma unroll
-            for (int f = 0; f < F; ++f) tacc[j][f] = 0.f;
+        float* tile = args.tiles + (size_t)w * args.tile_stride;
 
         const float dt = sc.dt, h = sc.h, inv_h = sc.inv_h;
-        for (int r0 = 0; r0 < nseg; r0 += L::kSlots) {
-            const int rend = min(nseg, r0 + L::kSlots);
-            // ---- particle phase: warps take segments of this round dynamically ----
-            float* st = stage + (size_t)warp * L::kStage * L::P;
-            // The round's particles [rb, re) are cut into windows of kStage; a
-            // warp takes a window and handles the segments that start in it:
-            // several sparse cells share one staging pass, a long segment
-            // takes several.  Each segment is summed by one warp, in order.
+        int t0[3];
+        tileOrigin(sc, it.block, t0);
+        // ---- particle phase of a round: warps take its segments dynamically ----
+        // The round's particles [rb, re) are cut into windows (of kStage,
+        // fewer where that leaves warps without one); a warp takes a window
+        // and handles the segments that start in it: several sparse rows
+        // share one staging pass, a long segment takes several.  Each segment
+        // is summed by one warp, in order.
+        auto particles = [&](int r0, int rend) {
+            using LN = P2GLanes<S, MODE>;
+            const LN ln(lane);
+            // where the lane's share of a flushed node goes in a partial (-1: nowhere)
+            int off[LN::kOut];
+#pragma unroll
+            for (int i = 0; i < LN::kOut; ++i) {
+                const int k = valueOf<F, 1, LN::G>(i, ln.grp);
+                off[i] = k < 0 || !ln.on ? -1 : k * T * CS + ln.b + S * ln.c;
+            }
             const int rb = segBeg[r0], re = segEnd[rend - 1];
-            const int nwin = (re - rb + L::kStage - 1) / L::kStage;
+            const int win = min(L::kStage, (re - rb + L::NW - 1) / L::NW);
+            const int nwin = (re - rb + win - 1) / win;
+            RowWindow<S, MODE> rw;
+            rw.clear();
             while (true) {
                 int wi = 0;
                 if (lane == 0) wi = atomicAdd(&ctl[1], 1);
                 wi = __shfl_sync(0xffffffffu, wi, 0);
                 if (wi >= nwin) break;
-                const int sl = r0 + lane;  // a round has at most 32 segments: one per lane
-                const bool starts = sl < rend && (segBeg[sl] - rb) / L::kStage == wi;
+                const int sl = r0 + lane;  // one segment of the round per lane
+                const bool starts = sl < rend && (segBeg[sl] - rb) / win == wi;
                 const unsigned own = __ballot_sync(0xffffffffu, starts);
                 if (!own) continue;
-                const int s_first = r0 + __ffs(own) - 1, s_last = r0 + 31 - __clz(own);
-                const int cb = segBeg[s_first], ce = segEnd[s_last];
-                int cur = s_first;  // segment being summed
-                NodeAcc acc[S];
-#pragma unroll
-                for (int c = 0; c < S; ++c) acc[c].zero();
-                for (int g0 = cb; g0 < ce; g0 += L::kStage) {
-                    const int np = min(L::kStage, ce - g0);
-                    if (lane < np) {
-                        p2gStageParticle<S, MODE, L::P, L::WB>(args, sc, pf, cap, dt, h, inv_h,
-                                                               i0 + (uint32_t)(g0 + lane), st + lane * L::P);
+                const int s_last = r0 + 31 - __clz(own);
+                int cur = r0 + __ffs(own) - 1;  // segment being summed
+                const int ce0 = segEnd[s_last];
+                // the loads of a pass are issued one pass ahead (the permutation
+                // entries and keys two)
+                const int gb = segBeg[cur];
+                P2GRaw<S, MODE> raw;
+                uint32_t cl = 0, ncl = 0, nperm = 0;
+                const bool stages = lane < L::kStage;
+                if (stages && gb + lane < ce0) {
+                    cl = keys[gb + lane] & 63u;
+                    raw.load(args, sc, pf, cap, perm[gb + lane]);
+                }
+                if (stages && gb + L::kStage + lane < ce0) {
+                    ncl = keys[gb + L::kStage + lane] & 63u;
+                    nperm = perm[gb + L::kStage + lane];
+                }
+                for (int g0 = gb; g0 < ce0; g0 += L::kStage) {
+                    const int np = min(L::kStage, ce0 - g0);
+                    if (lane < np) p2gStageParticle<S, MODE>(sc, raw, dt, h, inv_h, t0, cl, st + lane * L::P4);
+                    const uint32_t pcl = cl;  // this pass's cells
+                    const int next_x = (int)(__shfl_sync(0xffffffffu, ncl, 0) & 3u);  // only read where the segment goes on
+                    if (stages && g0 + L::kStage + lane < ce0) raw.load(args, sc, pf, cap, nperm);
+                    cl = ncl;
+                    if (stages && g0 + 2 * L::kStage + lane < ce0) {
+                        ncl = keys[g0 + 2 * L::kStage + lane] & 63u;
+                        nperm = perm[g0 + 2 * L::kStage + lane];
                     }
                     __syncwarp();
                     // the segments overlapping this pass, in order
                     while (cur <= s_last) {
-                    const int se = segEnd[cur];
-                    const int qlo = max(segBeg[cur], g0) - g0, qhi = min(se, g0 + np) - g0;
-                    // group grp sums the segment's particles j = grp (mod G), in
-                    // order, however the segment is cut into staging passes
-                    const int jlo = g0 + qlo - segBeg[cur];
-                    if (lane_on)
-                        p2gAccumulate<S, MODE, L::P, L::WB, L::G>(st, qlo + (grp - jlo % L::G + L::G) % L::G, qhi, na,
-                                                                  nb, acc);
-                    if (se > g0 + np) break;  // the segment continues in the next pass
-                    // Segment done: sum the groups' columns in group order into
-                    // group 0 (fixed order, so the partial does not depend on
-                    // timing), write its slot, start the next segment.
+                        const int sb = segBeg[cur], se = segEnd[cur];
+                        const int qlo = max(sb, g0) - g0, qhi = min(se, g0 + np) - g0;
+                        const bool ends = se <= g0 + np;
+                        float* slot = partial + (size_t)(cur - r0) * L::kSlotFloats;
+                        rw.pass(st, pcl, qlo, qhi, segRow[cur], g0 + qlo - sb, ends ? 4 : next_x, lane, ln,
+                                [&](int n, const float* v) {
 #pragma unroll
-                    for (int c = 0; c < S; ++c) {
-#pragma unroll
-                        for (int f = 0; f < F; ++f) {
-                            const float mine = acc[c].get(f);
-                            float sum = mine;
-#pragma unroll
-                            for (int g = 1; g < L::G; ++g)
-                                sum += __shfl_sync(0xffffffffu, mine, min(lane + g * L::PAIRS, 31));
-                            if (grp == 0)
-                                partial[(size_t)(cur - r0) * F * L::NS + f * L::NS + na + S * nb + L::PAIRS * c] = sum;
-                        }
-                        acc[c].zero();
-                    }
-                    ++cur;
+                                    for (int i = 0; i < LN::kOut; ++i)
+                                        if (off[i] >= 0) slot[off[i] + n * CS] = v ? v[i] : 0.f;
+                                });
+                        if (!ends) break;  // the segment continues in the next pass
+                        ++cur;
                     }
                     __syncwarp();
                 }
             }
+        };
+        for (int r0 = 0; r0 < nseg; r0 += L::kSlots) {
+            const int rend = min(nseg, r0 + L::kSlots);
+            particles(r0, rend);
             __syncthreads();
             if (threadIdx.x == 0) ctl[1] = 0;  // next round's dynamic counter (no warp reads it until the barrier below)
             // ---- gather phase: fixed-order merge of this round's segments ----
-#pragma unroll
+            // (a later round adds to the tile that the same thread wrote before)
+#pragma unroll 1
             for (int j = 0; j < L::TJ; ++j) {
                 const int tn = threadIdx.x + j * L::NT;
-                if (tn < L::TN) {
-                    const int tx = tn % (S + 3), ty = (tn / (S + 3)) % (S + 3), tz = tn / ((S + 3) * (S + 3));
-                    for (int sg = r0; sg < rend; ++sg) {
-                        const int cell = segCell[sg];
-                        const int dx = tx - (cell & 3), dy = ty - ((cell >> 2) & 3), dz = tz - (cell >> 4);
-                        if ((unsigned)dx >= (unsigned)S || (unsigned)dy >= (unsigned)S || (unsigned)dz >= (unsigned)S)
-                            continue;
-                        // stencil node index of the lane layout: a + S (b + S c)
-                        const float* pc = partial + (size_t)(sg - r0) * F * L::NS + dx + S * (dy + S * dz);
+                if (tn >= TN) break;
+                const int tx = tn % T, ty = (tn / T) % T, tz = tn / (T * T);
+                float sum[F];
 #pragma unroll
-                        for (int f = 0; f < F; ++f) tacc[j][f] += pc[f * L::NS];
-                    }
+                for (int f = 0; f < F; ++f) sum[f] = r0 ? tile[f * TN + tn] : 0.f;
+                for (int sg = r0; sg < rend; ++sg) {
+                    const int row = segRow[sg];
+                    const int dy = ty - (row & 3), dz = tz - (row >> 2);
+                    if ((unsigned)dy >= (unsigned)S || (unsigned)dz >= (unsigned)S) continue;
+                    const float* pc = partial + (size_t)(sg - r0) * L::kSlotFloats + tx * CS + dy + S * dz;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) sum[f] += pc[f * T * CS];
                 }
+#pragma unroll
+                for (int f = 0; f < F; ++f) tile[f * TN + tn] = sum[f];
             }
             __syncthreads();
-        }
-        float* tile = args.tiles + (size_t)w * args.tile_stride;
-#pragma unroll
-        for (int j = 0; j < L::TJ; ++j) {
-            const int tn = threadIdx.x + j * L::NT;
-            if (tn < L::TN)
-#pragma unroll
-                for (int f = 0; f < F; ++f) tile[f * L::TN + tn] = tacc[j][f];
         }
     }
     spanEnd(args.spans, SPAN_P2G);
@@ -905,46 +1113,51 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
 
 // ---------------------------------------------------------------------------
 // P2G by whole warps for the small items (the combination's warp list).  Each
-// warp takes an item and sums its particles segment by segment as p2gKernel
-// does -- cells in order, each cut into segments of at most kSeg particles; a
-// segment's particles summed per group in order, the groups then in lane
-// order (p2gStageParticle, p2gAccumulate) -- and adds each segment's sums
-// into its own shared-memory tile in segment order, the order of p2gKernel's
+// warp takes an item and sums its particles row by row as p2gKernel does (the
+// same segments, RowWindow) and adds the nodes that leave its window into its
+// own shared-memory tile, segment after segment, the order of p2gKernel's
 // merge: the tile is bitwise p2gKernel's, so which kernel takes an item
 // changes no result.  No CTA barrier: an item of a few particles per cell
-// spends most of p2gKernel's time in its per-item set-up, barriers and merge
-// rounds.
+// spends most of p2gKernel's time in its per-item set-up, barriers and merge.
 // ---------------------------------------------------------------------------
 template <int S, int MODE>
-struct P2GWarpLayout {
-    using D = P2GLayout<S, MODE, 16>;  // staging layout, column map and segment length
-    static constexpr int F = D::F, TN = D::TN, P = D::P, WB = D::WB, G = D::G, PAIRS = D::PAIRS;
-    static constexpr int kSeg = D::kSeg;
-    static constexpr int kStage = 16;  // particles staged per pass
-    static constexpr int NT = 256, NW = NT / 32;
-    // per warp: its item's scene entry, its tile [F][TN], its staging rows
-    // (field-major: a column's 16 lanes add to 16 different banks; a
+struct P2GWarpLayout : P2GStage<S, MODE> {
+    using R = P2GStage<S, MODE>;
+    static constexpr int kStage = 32;  // particles staged per pass (8.4M-particle slab P2G 1.02, 1.00 and 0.95 ms at 16, 24, 32)
+    // per warp: its item's scene entry, its tile [F][TN], its staging words
+    // (field-major: neighbouring columns add to neighbouring banks; a
     // node-major tile of 16-byte words had bank conflicts and was slower)
     static constexpr int kSceneFloats = (int)((sizeof(SceneDev) + 15) / 16 * 4);
-    static constexpr int kTileFloats = (F * TN + 3) / 4 * 4;
-    static constexpr int kWarpFloats = kSceneFloats + kTileFloats + kStage * P;
+    static constexpr int kTileFloats = (R::F * R::TN + 3) / 4 * 4;
+    static constexpr int kRowInts = 20;
+    static constexpr int kWarpFloats = kSceneFloats + kTileFloats + kStage * R::P4 * 4 + kRowInts;
+    // two CTAs per SM of as many warps as its shared memory holds, at most 24 in all
+    static constexpr int kWarpsPerSm = (int)(226u * 1024 / (kWarpFloats * 4));
+    static constexpr int NW = (kWarpsPerSm < 24 ? kWarpsPerSm : 24) / 2, NT = 32 * NW;
     static constexpr size_t smemBytes = (size_t)NW * kWarpFloats * 4;
-    static constexpr int MIN_CTAS = (smemBytes + 1024) * 3 <= 228 * 1024 ? 3 : 2;
+    static constexpr int MIN_CTAS = 2;
 };
 
 template <int S, int MODE>
 __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, MODE>::MIN_CTAS)
     p2gWarpKernel(StepArgs args) {
     using W = P2GWarpLayout<S, MODE>;
-    constexpr int F = W::F, T = S + 3, TN = W::TN, G = W::G, PAIRS = W::PAIRS;
+    constexpr int F = W::F, T = S + 3, TN = W::TN;
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* wbase = reinterpret_cast<float*>(smem4) + (size_t)warp * W::kWarpFloats;
     SceneDev& sc = *reinterpret_cast<SceneDev*>(wbase);
     float* tile = wbase + W::kSceneFloats;
-    float* st = tile + W::kTileFloats;
-    const int grp = lane / PAIRS, na = (lane % PAIRS) % S, nb = (lane % PAIRS) / S;
-    const bool lane_on = grp < G;
+    float4* st = reinterpret_cast<float4*>(tile + W::kTileFloats);
+    int* rowBeg = reinterpret_cast<int*>(st + W::kStage * W::P4);
+    using LN = P2GLanes<S, MODE>;
+    const LN ln(lane);
+    int off[LN::kOut];  // where the lane's share of a flushed node goes in the tile (-1: nowhere)
+#pragma unroll
+    for (int i = 0; i < LN::kOut; ++i) {
+        const int k = valueOf<F, 1, LN::G>(i, ln.grp);
+        off[i] = k < 0 || !ln.on ? -1 : k * TN + T * (ln.b + T * ln.c);
+    }
     const uint32_t* list = args.p2g_lists + (size_t)(2 * args.combo) * args.p2g_list_cap;
     const uint32_t nwork = args.counters[kP2GListWord + 2 * args.combo];
     // the warps' item scheduler: [0] hands out list indices, [1] counts the
@@ -954,25 +1167,7 @@ __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, M
     // nothing for warps (the scheduler is untouched): p2gKernel takes the
     // small items when the list is too short to fill the GPU with warps
     if (nwork == 0 || !p2gWarpTakesSmall(args.p2g_warp, nwork)) return;
-    NodeAcc acc[S];
-    // a segment done: the groups' columns summed in group order (as
-    // p2gKernel), added by group 0 into the tile nodes of the segment's cell
-    auto finish = [&](int cell) {
-        const int cx = cell & 3, cy = (cell >> 2) & 3, cz = cell >> 4;
-#pragma unroll
-        for (int c = 0; c < S; ++c) {
-#pragma unroll
-            for (int f = 0; f < F; ++f) {
-                const float mine = acc[c].get(f);
-                float sum = mine;
-#pragma unroll
-                for (int g = 1; g < G; ++g) sum += __shfl_sync(0xffffffffu, mine, min(lane + g * PAIRS, 31));
-                if (grp == 0) tile[f * TN + (na + cx) + T * ((nb + cy) + T * (c + cz))] += sum;
-            }
-            acc[c].zero();
-        }
-        __syncwarp();  // the next segment's sums may land on the same nodes from other lanes
-    };
+    RowWindow<S, MODE> win;
     spanBegin(args.spans, SPAN_P2G);
     for (;;) {
         uint32_t wi = 0;
@@ -1003,57 +1198,67 @@ __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, M
         const float dt = sc.dt, h = sc.h, inv_h = sc.inv_h;
         const uint32_t i0 = it.start;
         const int count = (int)it.count;
-#pragma unroll
-        for (int c = 0; c < S; ++c) acc[c].zero();
-        int seg_start = 0;     // item index of the open segment's first particle
-        int seg_cell = 0;      // its cell
-        int cell_start = 0;    // item index of the current cell's first particle
-        uint32_t last_cell = 0;  // cell of the previous pass's last particle
+        const uint32_t* keys = args.sorted_keys + i0;
+        const uint32_t* perm = args.perm + i0;
+        int t0[3];
+        tileOrigin(sc, it.block, t0);
+        win.clear();
+        findRows(keys, count, rowBeg, lane, 32);
+        __syncwarp();
+        // the open row [rb, re) and its open segment [sb, se), the j-th of n
+        int row = 0, rb = 0, re = 0, sb = 0, se = 0, j = 0, n = 0;
+        // the loads of a pass are issued one pass ahead (the permutation
+        // entries and keys two)
+        P2GRaw<S, MODE> raw;
+        uint32_t cl = 0, ncl = 0, nperm = 0;
+        const bool stages = lane < W::kStage;
+        if (stages && lane < count) {
+            cl = keys[lane] & 63u;
+            raw.load(args, sc, pf, cap, perm[lane]);
+        }
+        if (stages && W::kStage + lane < count) {
+            ncl = keys[W::kStage + lane] & 63u;
+            nperm = perm[W::kStage + lane];
+        }
         for (int g0 = 0; g0 < count; g0 += W::kStage) {
             const int np = min(W::kStage, count - g0);
-            uint32_t cl = 0;
-            if (lane < np) {
-                p2gStageParticle<S, MODE, W::P, W::WB>(args, sc, pf, cap, dt, h, inv_h, i0 + (uint32_t)(g0 + lane),
-                                                       st + lane * W::P);
-                cl = args.sorted_keys[i0 + (uint32_t)(g0 + lane)] & 63u;
+            if (lane < np) p2gStageParticle<S, MODE>(sc, raw, dt, h, inv_h, t0, cl, st + lane * W::P4);
+            const uint32_t pcl = cl;  // this pass's cells
+            const int next_x = (int)(__shfl_sync(0xffffffffu, ncl, 0) & 3u);  // only read where the segment goes on
+            if (stages && g0 + W::kStage + lane < count) raw.load(args, sc, pf, cap, nperm);
+            cl = ncl;
+            if (stages && g0 + 2 * W::kStage + lane < count) {
+                ncl = keys[g0 + 2 * W::kStage + lane] & 63u;
+                nperm = perm[g0 + 2 * W::kStage + lane];
             }
-            // segment starts of this pass: a particle that opens a cell, or
-            // one kSeg particles after its cell's first
-            uint32_t up = __shfl_up_sync(0xffffffffu, cl, 1);
-            if (lane == 0) up = last_cell;
-            const unsigned cells = __ballot_sync(0xffffffffu, lane < np && (g0 + lane == 0 || cl != up));
-            const unsigned upto = cells & (0xffffffffu >> (31 - lane));  // this lane's and the earlier lanes'
-            const int my_cell_start = upto ? g0 + 31 - __clz(upto) : cell_start;
-            const unsigned segs = __ballot_sync(0xffffffffu, lane < np && (g0 + lane - my_cell_start) % W::kSeg == 0);
-            if (cells) cell_start = g0 + 31 - __clz(cells);
-            last_cell = __shfl_sync(0xffffffffu, cl, np - 1);
-            const uint32_t cl0 = __shfl_sync(0xffffffffu, cl, 0);
-            __syncwarp();  // the staged rows are visible to the warp
-            if (g0 == 0) {
-                seg_cell = (int)cl0;
-            } else if (segs & 1u) {  // the open segment ended with the previous pass
-                finish(seg_cell);
-                seg_start = g0;
-                seg_cell = (int)cl0;
+            __syncwarp();  // the staged particles are visible to the warp
+            for (int q = 0; q < np;) {
+                if (g0 + q == se) {  // the next segment, as p2gKernel cuts them
+                    if (se == re) {
+                        row = (int)(__shfl_sync(0xffffffffu, pcl, q) >> 2);
+                        rb = rowBeg[row];
+                        re = rowBeg[row + 1];
+                        n = (re - rb + W::kSeg - 1) / W::kSeg;
+                        j = 0;
+                    }
+                    sb = se;
+                    se = rb + (re - rb) * ++j / n;
+                }
+                const int qhi = min(se - g0, np);
+                const bool ends = se <= g0 + np;
+                const int base = T * ((row & 3) + T * (row >> 2));
+                win.pass(st, pcl, q, qhi, row, g0 + q - sb, ends ? 4 : next_x, lane, ln,
+                         [&](int n, const float* v) {
+                             if (v)
+#pragma unroll
+                                 for (int i = 0; i < LN::kOut; ++i)
+                                     if (off[i] >= 0) tile[off[i] + base + n] += v[i];
+                         });
+                if (ends) __syncwarp();  // the next segment's sums may land on the same nodes from other lanes
+                q = qhi;
             }
-            int qa = 0;
-            for (;;) {
-                const unsigned rest = segs & ~((2u << qa) - 1u);  // starts after qa
-                const int qb = rest ? __ffs(rest) - 1 : np;
-                // group grp sums the segment's particles j = grp (mod G), in
-                // order, however the segment is cut into passes
-                const int jlo = g0 + qa - seg_start;
-                if (lane_on) p2gAccumulate<S, MODE, W::P, W::WB, G>(st, qa + (grp - jlo % G + G) % G, qb, na, nb, acc);
-                if (qb >= np) break;  // the open segment continues past this pass
-                const uint32_t cq = __shfl_sync(0xffffffffu, cl, qb);
-                finish(seg_cell);
-                seg_start = g0 + qb;
-                seg_cell = (int)cq;
-                qa = qb;
-            }
-            __syncwarp();  // the staged rows are read before the next pass overwrites them
+            __syncwarp();  // the staged particles are read before the next pass overwrites them
         }
-        finish(seg_cell);
         float* out = args.tiles + (size_t)w * args.tile_stride;
         for (int q = lane; q < F * TN; q += 32) out[q] = tile[q];
         __syncwarp();  // the tile is read before the next item clears it
@@ -1656,14 +1861,6 @@ __device__ __forceinline__ bool waitTile(uint64_t* bar, unsigned parity, uint32_
     return true;
 }
 
-// Origin (node index) of the (S+3)^3 tile of an active block: 4 B - 4 per axis.
-__device__ __forceinline__ void tileOrigin(const SceneDev& sc, uint32_t block, int* t0) {
-    const uint32_t lb = block - sc.block_base;
-    t0[0] = 4 * (int)(lb % (uint32_t)sc.nb[0]) - 4;
-    t0[1] = 4 * (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]) - 4;
-    t0[2] = 4 * (int)(lb / ((uint32_t)sc.nb[0] * (uint32_t)sc.nb[1])) - 4;
-}
-
 // Bulk copy (cp.async.bulk) of bytes from global to shared memory, completing
 // on bar; both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulkLoad(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
@@ -1699,7 +1896,6 @@ constexpr int kG2PWarps = kG2PThreads / 32;
 #endif
 template <int S, bool APIC>
 __global__ void __launch_bounds__(kG2PThreads, MPM_G2P_MIN_CTAS) g2pKernel(StepArgs args, int fused) {
-    constexpr int T = S + 3;
     constexpr int TN = tileNodes(S);
     constexpr int TNP = (TN + 7) & ~7;  // buffers 128-byte aligned
     constexpr unsigned kTileBytes = (unsigned)TN * 16u;
