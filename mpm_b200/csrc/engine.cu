@@ -396,7 +396,7 @@ public:
     void releaseScratch() {
         DevMem* all[] = {&cell_range_, &block_range_, &solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
                          &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &inc_scratch_,
-                         &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_,
+                         &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_, &tile_done_,
                          &tiles_, &scenes_dev_, &err_, &tmp_, &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
         for (DevMem* m : all) m->release();
     }
@@ -956,10 +956,10 @@ public:
         CUDA_TRY(cudaMemsetAsync(block_count_.p, 0, sizeof(uint32_t) * tb, stream_));
         MPM_TRY(grow(sbb_, sizeof(uint32_t) * (ns + 1), "scene block bases"));
         CUDA_TRY(cudaMemcpyAsync(sbb_.p, sbb.data(), sizeof(uint32_t) * (ns + 1), cudaMemcpyHostToDevice, stream_));
-        // work items: one per non-empty block plus one per further kBlockChunk particles
-        max_active_ = std::max<size_t>(1, std::min<size_t>(tb, nk) + nk / kBlockChunk + 1);
+        // work items: one per non-empty block plus at most one per kSplitChunk particles
+        max_active_ = std::max<size_t>(1, std::min<size_t>(tb, nk) + nk / kSplitChunk + 1);
         MPM_TRY(grow(active_, sizeof(BlockItem) * max_active_, "active blocks"));
-        MPM_TRY(grow(outside_, sizeof(BlockItem) * ((size_t)ns + nk / kBlockChunk + 1), "outside blocks"));
+        MPM_TRY(grow(outside_, sizeof(BlockItem) * ((size_t)ns + nk / kSplitChunk + 1), "outside blocks"));
         g2p_cap_ = (uint32_t)(std::min<size_t>(tb, nk) + nk / kMinG2PChunk + 1);
         MPM_TRY(grow(g2p_items_, sizeof(BlockItem) * g2p_cap_ * (size_t)combos().size(), "G2P items"));
         // P2G's two lists of item slots per combination (warp items, CTA items)
@@ -973,11 +973,13 @@ public:
             MPM_TRY(resetSpans());
         }
         CUDA_TRY(cudaMemsetAsync(counters_.p, 0, sizeof(uint32_t) * kCounterWords, stream_));
-        MPM_TRY(grow(block_slot_, sizeof(int32_t) * tb, "block slots"));
+        MPM_TRY(grow(block_slot_, sizeof(int2) * tb, "block slots"));
         int maxS = 2;
         for (auto& s : scenes_) maxS = std::max(maxS, s->S);
         tile_stride_ = (size_t)7 * tileNodes(maxS);
         MPM_TRY(grow(tiles_, sizeof(float) * tile_stride_ * max_active_, "P2G tiles"));
+        MPM_TRY(grow(tile_done_, sizeof(uint32_t) * max_active_, "P2G tile counts"));
+        CUDA_TRY(cudaMemsetAsync(tile_done_.p, 0, sizeof(uint32_t) * max_active_, stream_));
         MPM_TRY(grow(scenes_dev_, sizeof(SceneDev) * std::max(ns, 1), "scene table"));
         // Room in the pool for the download staging buffers (two float4 per
         // particle, taken at a scene's first download): taken and given back
@@ -1156,8 +1158,9 @@ public:
         a.combo = 0;
         a.counters = counters_.as<uint32_t>();
         a.outside = outside_.as<BlockItem>();
-        a.block_slot = block_slot_.as<int32_t>();
+        a.block_slot = block_slot_.as<int2>();
         a.tiles = tiles_.as<float>();
+        a.tile_done = tile_done_.as<uint32_t>();
         a.tile_stride = (uint32_t)tile_stride_;
         a.next_keys = next_keys;
         a.block_count = block_count_.as<uint32_t>();
@@ -1181,7 +1184,7 @@ public:
         bb.g2p_items = g2p_items_.as<BlockItem>();
         bb.g2p_cap = g2p_cap_;
         bb.counters = counters_.as<uint32_t>();
-        bb.block_slot = block_slot_.as<int32_t>();
+        bb.block_slot = block_slot_.as<int2>();
         bb.p2g_lists = p2g_lists_.as<uint32_t>();
         bb.p2g_list_cap = (uint32_t)max_active_;
         return bb;
@@ -1242,7 +1245,7 @@ public:
             CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
             LaunchCtx cc = ctx();
             cc.stream = compact_stream_;
-            launchCompactOnesweep(cc, blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), kBlockChunk, comboSplit(),
+            launchCompactOnesweep(cc, blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), comboSplit(),
                                   err_.as<uint32_t>());
             CUDA_TRY(cudaGetLastError());
             CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
@@ -1270,7 +1273,7 @@ public:
             CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
         } else {
             mark(KF_COMPACT, 0);
-            launchCompactOnesweep(ctx(), blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), kBlockChunk, comboSplit(),
+            launchCompactOnesweep(ctx(), blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), comboSplit(),
                                   err_.as<uint32_t>());
             mark(KF_COMPACT, 1);
             collect(KF_COMPACT);
@@ -2410,7 +2413,7 @@ private:
     uint32_t total_blocks_ = 0;
     int key_bits_ = 1;
     DevMem keys_[2], vals_[2], sort_scratch_, inc_scratch_, compact_scratch_, block_count_, sbb_, active_,
-        outside_, counters_, block_slot_, tiles_, scenes_dev_, err_, tmp_, g2p_items_, tmaps_, spans_, p2g_lists_;
+        outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, tmp_, g2p_items_, tmaps_, spans_, p2g_lists_;
     // Per combination: the first step after a change of the scene set found
     // fewer than kWarpAutoMinItems small P2G items, so the step does not
     // launch the warp kernel (see checkWarpItems, warpModeOf).
@@ -2819,7 +2822,7 @@ mpm_status mpm_sort_keys(const uint32_t* keys, size_t n, int32_t bits, uint32_t*
     cudaStreamDestroy(st);
     if (s != MPM_OK) return s;
     if (e != cudaSuccess) return mpm::fail(MPM_ERR_CUDA, std::string("mpm_sort_keys: ") + cudaGetErrorString(e));
-    if (flag) return mpm::fail(MPM_ERR_TIMEOUT, "mpm_sort_keys: a look-back wait gave up");
+    if (flag) return mpm::fail(MPM_ERR_TIMEOUT, "mpm_sort_keys: a wait gave up");
     return MPM_OK;
 }
 

@@ -22,14 +22,23 @@ namespace mpm {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSortTileKeys = kThreads * 8;  // keys per radix-sort tile (8 per thread)
-// Work items: a block's sorted particles are split into
-// ceil(count / kBlockChunk) P2G items of nearly equal size (each with its own
-// P2G tile, merged in item order), so that one crowded block cannot serialize
-// a step.  The split fixes the order of P2G's sums, so it is a constant.
-// (Splits of 2048 and 1024 particles were no faster on the dense two-ball
-// scene -- P2G 0.150 and 0.144 ms against 0.145 ms -- and slowed the grid
-// pass, which sums more tiles per node.)
-constexpr uint32_t kBlockChunk = 4096;
+// Work items: a block's sorted particles are one P2G item up to kBlockChunk of
+// them; a fuller block is split into ceil(count / kSplitChunk) items of nearly
+// equal size, so that a few crowded blocks cannot serialize a step.  Each item
+// has its own tile; the last of a block's items to finish adds their tiles up
+// in item order, so the grid pass reads one tile per block.  The split fixes
+// the order of P2G's sums, so both are constants.  Where the line lies: at 35
+// particles a cell (2,200 a full block) whole blocks are faster than items of
+// 2048 or 1024 (P2G 0.099, 0.105 and 0.121 ms), which have too few rows each;
+// a block above 40 a cell has long rows, and scenes of few such blocks need
+// the parallelism (six scenes of up to 60k particles, P2G: items of up to 4096
+// 0.146 ms, split above 4096 into 1024s 0.116, above 2560 into 1280s 0.092;
+// into 640s 0.088, but 64 scenes of up to 500k 0.88 -> 1.03 ms).
+constexpr uint32_t kBlockChunk = 2560;
+constexpr uint32_t kSplitChunk = 1280;
+__host__ __device__ inline uint32_t blockItems(uint32_t count) {
+    return count <= kBlockChunk ? (count ? 1u : 0u) : (count + kSplitChunk - 1) / kSplitChunk;
+}
 // Particles that a P2G warp stages at a time unless the caller sets it
 // (mpm_tuning.p2g_stage): a full warp.  16 and 24 were slower for every density
 // measured (two-ball P2G 0.128, 0.111 and 0.099 ms at 16, 24 and 32).
@@ -58,7 +67,7 @@ constexpr int kP2GSmallWord = kP2GListWord + 2 * kMaxCombos;
 // them) and the others from the back (counters[kP2GBackWord + k]), so that
 // the CTAs take the long items first and the short ones fill the tail.
 constexpr int kP2GBackWord = kP2GSmallWord + kMaxCombos;
-constexpr uint32_t kBigItem = 1024;
+constexpr uint32_t kBigItem = 768;
 constexpr uint32_t kWarpAutoMax = 256;
 constexpr uint32_t kWarpAutoMinItems = 1024;
 // Who takes the small P2G items (list 0) in a step: p2gKernel after its own
@@ -196,8 +205,9 @@ struct StepArgs {
     int combo;                   // the combination a G2P launch serves
     const uint32_t* counters;    // [0] active blocks, [1] outside blocks
     const BlockItem* outside;
-    const int32_t* block_slot;   // dense: block -> slot or -1
+    const int2* block_slot;      // dense: block -> (first slot or -1, work items)
     float* tiles;                // [slot][F][TN]
+    uint32_t* tile_done;         // [first slot of a block]: its items whose tiles are written (zero between launches)
     uint32_t tile_stride;        // floats per slot
     uint32_t* next_keys;         // N
     uint32_t* block_count;       // dense per block

@@ -31,7 +31,7 @@ struct BlockBuffers {
     BlockItem* g2p_items;             // G2P work items, g2p_cap per combination
     uint32_t g2p_cap;
     uint32_t* counters;               // see kG2PCountWord, kP2GListWord
-    int32_t* block_slot;              // total_blocks
+    int2* block_slot;                 // total_blocks
     uint32_t* p2g_lists;              // P2G item slots, 2 lists of p2g_list_cap per combination
     uint32_t p2g_list_cap;
 };
@@ -79,7 +79,7 @@ struct ComboSplit {
     uint32_t p2g_warp_max[kMaxCombos];
 };
 void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks,
-                           unsigned long long* scratch, uint32_t chunk, const ComboSplit& split, uint32_t* err);
+                           unsigned long long* scratch, const ComboSplit& split, uint32_t* err);
 void launchStress(const LaunchCtx& c, int parity);
 void launchP2G(const LaunchCtx& c, const StepArgs& a, int S, int mode, int want_transfer);
 // P2G of the combination a.combo's warp list (a.p2g_lists set): one warp per

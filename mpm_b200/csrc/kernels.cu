@@ -204,8 +204,8 @@ __device__ __forceinline__ void splitItems(BlockItem* out, uint32_t b, uint32_t 
 __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
     uint32_t* __restrict__ block_count, uint32_t total_blocks, const uint32_t* __restrict__ scene_block_base,
     int nscenes, BlockItem* __restrict__ active, BlockItem* __restrict__ outside, uint32_t* __restrict__ counters,
-    int32_t* __restrict__ block_slot, unsigned long long* __restrict__ status, uint32_t* __restrict__ tile_counter,
-    uint32_t ntiles, uint32_t chunk, BlockItem* __restrict__ g2p_items, uint32_t g2p_cap, ComboSplit split,
+    int2* __restrict__ block_slot, unsigned long long* __restrict__ status, uint32_t* __restrict__ tile_counter,
+    uint32_t ntiles, BlockItem* __restrict__ g2p_items, uint32_t g2p_cap, ComboSplit split,
     uint32_t* __restrict__ p2g_lists, uint32_t p2g_list_cap, const SceneDev* __restrict__ scenes,
     uint32_t* __restrict__ err) {
     __shared__ uint32_t tile_s;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
             const uint32_t c = block_count[b];
             const int s = sceneOfBlock(scene_block_base, nscenes, b);
             const bool out = (b == scene_block_base[s + 1] - 1);
-            const unsigned long long items = (c > 0 && !out) ? (unsigned long long)((c + chunk - 1) / chunk) : 0ull;
+            const unsigned long long items = out ? 0ull : (unsigned long long)blockItems(c);
             v = (items << 32) | (unsigned long long)c;
         }
         packed[j] = v;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
         if (items) {
             const uint32_t slot = (uint32_t)(run >> 32);
             splitItems(active + slot, b, start, count, items, (uint32_t)scene);
-            block_slot[b] = (int32_t)slot;
+            block_slot[b] = make_int2((int)slot, (int)items);
             // G2P's items of the block, in its combination's list at slots
             // taken from a counter (their order does not matter)
             const int k = scenes[scene].combo;
@@ -388,9 +388,9 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
                 }
             }
         } else {
-            block_slot[b] = -1;
+            block_slot[b] = make_int2(-1, 0);
             if (count > 0) {
-                const uint32_t nitems = (count + chunk - 1) / chunk;
+                const uint32_t nitems = blockItems(count);
                 const uint32_t o = atomicAdd(&counters[1], nitems);
                 splitItems(outside + o, b, start, count, nitems, (uint32_t)scene);
             }
@@ -618,7 +618,7 @@ struct P2GRaw {
 #pragma unroll
         for (int a = 0; a < 3; ++a) x[a] = ldg(pp + (F_X + a) * cap);
         m = ldg(pp + F_MASS * cap);
-        if constexpr (MODE == MODE_MASS) return;
+        if (MODE == MODE_MASS) return;
 #pragma unroll
         for (int a = 0; a < 3; ++a) v[a] = ldg(pp + (F_V + a) * cap);
 #pragma unroll
@@ -866,6 +866,28 @@ struct RowWindow {
     }
 };
 
+// A block of several items (slot = first slot, items): counts this item's tile
+// as written and says whether it was the last one; the count goes back to
+// zero for the next launch.  The caller's writes of the tile are fenced.
+__device__ __forceinline__ int lastOfBlock(const StepArgs& args, int2 slot) {
+    if (atomicAdd(&args.tile_done[slot.x], 1u) != (uint32_t)slot.y - 1u) return 0;
+    args.tile_done[slot.x] = 0u;
+    __threadfence();
+    return 1;
+}
+// Adds a block's tiles of N floats up in item order, into its first one
+// (thread t of nt; read from L2, where the other items' writes are).
+template <int N>
+__device__ __forceinline__ void mergeItemTiles(const StepArgs& args, int2 slot, int t, int nt) {
+    float* first = args.tiles + (size_t)slot.x * args.tile_stride;
+    for (int q = t; q < N; q += nt) {
+        float sum = __ldcg(first + q);
+#pragma unroll 8
+        for (int s = 1; s < slot.y; ++s) sum += __ldcg(first + (size_t)s * args.tile_stride + q);
+        first[q] = sum;
+    }
+}
+
 // Row starts of an item's `count` particles (keys sorted by cell): row r's
 // particles are [beg[r], beg[r + 1]), r < 16.  Thread t of nt writes those of
 // the rows that begin at its particles.
@@ -889,7 +911,7 @@ struct P2GLayout : P2GStage<S, MODE> {
     // 4 (linear) the gather's (x, y) neighbours fall in different banks.
     static constexpr int CS = S == 4 ? 18 : S * S;
     static constexpr int kSlotFloats = F * T * CS;
-    static constexpr int kMaxSeg = 48;                // >= 16 + kBlockChunk / kSeg + 1
+    static constexpr int kMaxSeg = 32;                // >= 16 + kBlockChunk / kSeg + 1
     static constexpr int kCtlInts = 17 + 3 * kMaxSeg + 4 + 3;
     // dynamic shared memory of nw warps: stage [nw][kStage][P4] 16-byte words,
     // partials [kSlots][F][T][CS] floats, then the control ints (rowBeg[17],
@@ -1106,6 +1128,16 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
             }
             __syncthreads();
         }
+        // the last of a block's items adds up their tiles
+        const int2 slot = args.block_slot[it.block];
+        if (slot.y > 1) {
+            __shared__ int last_s;
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) last_s = lastOfBlock(args, slot);
+            __syncthreads();
+            if (last_s) mergeItemTiles<F * TN>(args, slot, (int)threadIdx.x, L::NT);
+        }
     }
     spanEnd(args.spans, SPAN_P2G);
 }
@@ -1261,6 +1293,14 @@ __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, M
         }
         float* out = args.tiles + (size_t)w * args.tile_stride;
         for (int q = lane; q < F * TN; q += 32) out[q] = tile[q];
+        const int2 slot = args.block_slot[it.block];
+        if (slot.y > 1) {
+            __threadfence();
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) last = lastOfBlock(args, slot);
+            if (__shfl_sync(0xffffffffu, last, 0)) mergeItemTiles<F * TN>(args, slot, lane, 32);
+        }
         __syncwarp();  // the tile is read before the next item clears it
     }
     __syncthreads();  // every warp done: the CTA's span ends here
@@ -1286,7 +1326,7 @@ __device__ __forceinline__ void groupBarrier(int g) {
 
 __device__ __forceinline__ int blockSlotAt(const StepArgs& args, const SceneDev& sc, int x, int y, int z) {
     if (x < 0 || y < 0 || z < 0 || x >= sc.nb[0] || y >= sc.nb[1] || z >= sc.nb[2]) return -1;
-    return args.block_slot[sc.block_base + (uint32_t)((z * sc.nb[1] + y) * sc.nb[0] + x)];
+    return args.block_slot[sc.block_base + (uint32_t)((z * sc.nb[1] + y) * sc.nb[0] + x)].x;
 }
 
 // CTAs per SM: 4 (64 registers) where that costs at most a few bytes of
@@ -1307,11 +1347,11 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
     // items per CTA, each group of 64 threads merges its own blocks (four in
     // flight per CTA), group g taking items g, g + 4, ... of the CTA's share
     // and synchronising on its own named barrier; with fewer, the whole CTA
-    // merges one block, four node blocks at a time.  Per group, the first
-    // work item and number of work items of the 3^3 blocks around the
-    // current one, index (ox + 1) + 3 (oy + 1) + 9 (oz + 1).
+    // merges one block, four node blocks at a time.  Per group, the tile slots
+    // of the 3^3 blocks around the current one, index (ox + 1) + 3 (oy + 1) +
+    // 9 (oz + 1).
     constexpr int kGroups = kThreads / 64;
-    __shared__ int nbSlotAll[kGroups][27], nbItemsAll[kGroups][27];
+    __shared__ int nbSlotAll[kGroups][27];
     const uint32_t nact = args.counters[0];
     const bool grouped = nact >= 2u * gridDim.x;  // uniform over the CTA
     const int ngroups = grouped ? kGroups : 1;
@@ -1319,27 +1359,19 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
     const int gt = grouped ? (int)(threadIdx.x & 63) : (int)threadIdx.x;  // thread within the group
     const int dstep = grouped ? 1 : kGroups;  // node blocks per round
     int* nbSlot = nbSlotAll[grp];
-    int* nbItems = nbItemsAll[grp];
     spanBegin(args.spans, SPAN_GRID);
     for (uint32_t w = blockIdx.x * ngroups + grp; w < nact; w += gridDim.x * ngroups) {
         const BlockItem it = args.active[w];
         const SceneDev& sc = args.scenes[it.scene];
         if (sc.S != S || (want_transfer >= 0 && sc.transfer != want_transfer)) continue;
         if (MODE == MODE_MASS && !sc.init_pass) continue;
-        if (args.block_slot[it.block] != (int32_t)w) continue;  // a block's first work item does its nodes
+        if (args.block_slot[it.block].x != (int32_t)w) continue;  // a block's first work item does its nodes
         const uint32_t lb = it.block - sc.block_base;
         const int B[3] = {(int)(lb % (uint32_t)sc.nb[0]), (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]),
                           (int)(lb / ((uint32_t)sc.nb[0] * (uint32_t)sc.nb[1]))};
         if (gt < 27) {
             const int o[3] = {gt % 3 - 1, (gt / 3) % 3 - 1, gt / 9 - 1};
-            const int slot = blockSlotAt(args, sc, B[0] + o[0], B[1] + o[1], B[2] + o[2]);
-            int cnt = 0;
-            if (slot >= 0) {
-                const uint32_t blk = args.active[slot].block;
-                for (uint32_t s2 = (uint32_t)slot; s2 < nact && args.active[s2].block == blk; ++s2) ++cnt;
-            }
-            nbSlot[gt] = slot;
-            nbItems[gt] = cnt;
+            nbSlot[gt] = blockSlotAt(args, sc, B[0] + o[0], B[1] + o[1], B[2] + o[2]);
         }
         if (grouped) groupBarrier(grp);
         else __syncthreads();
@@ -1362,16 +1394,12 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
             float acc[F];
 #pragma unroll
             for (int f = 0; f < F; ++f) acc[f] = 0.f;
-            // The 8 tiles that overlap the node, in order e, and within each
-            // every work item of that block in item order.  The first item's
-            // values of Q tiles are loaded together (independent loads in
-            // flight), then summed in the same order as one by one.
-            constexpr int Q = F <= 4 ? 4 : 2;
+            // The 8 tiles that overlap the node, summed in order e; the loads of
+            // Q of them are in flight at once.
+            constexpr int Q = F <= 4 ? 8 : 4;
 #pragma unroll
             for (int hq = 0; hq < 8 / Q; ++hq) {
                 float v[Q][F];
-                const float* tp[Q];
-                int cnt[Q];
 #pragma unroll
                 for (int q = 0; q < Q; ++q) {
                     const int e = Q * hq + q;
@@ -1379,24 +1407,14 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
                     const int ix = L[0] + 4 * de[0], iy = L[1] + 4 * de[1], iz = L[2] + 4 * de[2];
                     const int nbi = (dd[0] - de[0] + 1) + 3 * (dd[1] - de[1] + 1) + 9 * (dd[2] - de[2] + 1);
                     const int slot = (ix < T && iy < T && iz < T) ? nbSlot[nbi] : -1;
-                    cnt[q] = slot >= 0 ? nbItems[nbi] : 0;
-                    tp[q] = args.tiles + (size_t)(slot >= 0 ? slot : 0) * args.tile_stride + ix + T * (iy + T * iz);
+                    const float* tp = args.tiles + (size_t)(slot >= 0 ? slot : 0) * args.tile_stride + ix + T * (iy + T * iz);
 #pragma unroll
-                    for (int f = 0; f < F; ++f) v[q][f] = cnt[q] > 0 ? tp[q][f * TN] : 0.f;
+                    for (int f = 0; f < F; ++f) v[q][f] = slot >= 0 ? tp[f * TN] : 0.f;
                 }
-                // A block's items are summed first (from its first item's
-                // tile), then the block's total is added to the node.
 #pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    if (cnt[q] <= 0) continue;
-                    for (int s2 = 1; s2 < cnt[q]; ++s2) {
-                        const float* tile = tp[q] + (size_t)s2 * args.tile_stride;
-#pragma unroll
-                        for (int f = 0; f < F; ++f) v[q][f] += tile[f * TN];
-                    }
+                for (int q = 0; q < Q; ++q)
 #pragma unroll
                     for (int f = 0; f < F; ++f) acc[f] += v[q][f];
-                }
             }
             const size_t node = (size_t)n[0] + (size_t)sc.res[0] * ((size_t)n[1] + (size_t)sc.res[1] * n[2]);
             const size_t nodes = (size_t)sc.res[0] * sc.res[1] * sc.res[2];
@@ -2274,7 +2292,7 @@ size_t compactScratchWords64(uint32_t total_blocks) {
 }
 
 void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks,
-                           unsigned long long* scratch, uint32_t chunk, const ComboSplit& split, uint32_t* err) {
+                           unsigned long long* scratch, const ComboSplit& split, uint32_t* err) {
     const uint32_t ntiles = (uint32_t)((total_blocks + kCompactTile - 1) / kCompactTile);
     ClearRanges cr;
     cr.p[0] = reinterpret_cast<uint32_t*>(scratch);
@@ -2289,7 +2307,7 @@ void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t 
     noteLaunches(1);
     compactOnesweepKernel<<<ntiles, kThreads, 0, c.stream>>>(
         bb.block_count, total_blocks, bb.scene_block_base, c.nscenes, bb.active, bb.outside, bb.counters,
-        bb.block_slot, scratch + 1, reinterpret_cast<uint32_t*>(scratch), ntiles, chunk, bb.g2p_items, bb.g2p_cap,
+        bb.block_slot, scratch + 1, reinterpret_cast<uint32_t*>(scratch), ntiles, bb.g2p_items, bb.g2p_cap,
         split, bb.p2g_lists, bb.p2g_list_cap, c.scenes, err);
 }
 
