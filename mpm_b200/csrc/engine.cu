@@ -395,7 +395,7 @@ public:
     // (called before the stream is destroyed).
     void releaseScratch() {
         DevMem* all[] = {&cell_range_, &block_range_, &solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
-                         &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &inc_scratch_,
+                         &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &range_[0], &range_[1], &emig_count_[0], &emig_count_[1], &emig_, &far_, &arrivals_, &far_count_, &sort_list_, &dense_list_,
                          &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_, &tile_done_,
                          &tiles_, &scenes_dev_, &err_, &tmp_, &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
         for (DevMem* m : all) m->release();
@@ -948,8 +948,24 @@ public:
             MPM_TRY(grow(vals_[k], sizeof(uint32_t) * nk, "values"));
         }
         MPM_TRY(grow(sort_scratch_, sizeof(uint32_t) * onesweepScratchWords(nk, key_bits_), "sort scratch"));
-        MPM_TRY(grow(inc_scratch_, sizeof(uint32_t) * incrementalSortScratchWords(nk, key_bits_),
-                                  "incremental sort scratch"));
+        // the block sort's lists: per block ranges and emigrant counts (by
+        // particle buffer: the compaction clears the next step's counts), per
+        // particle emigrants, far movers and the arrivals of crowded blocks
+        for (int k = 0; k < 2; ++k) {
+            MPM_TRY(grow(range_[k], sizeof(uint2) * tb, "block ranges"));
+            MPM_TRY(grow(emig_count_[k], sizeof(uint32_t) * tb, "emigrant counts"));
+        }
+        MPM_TRY(grow(emig_, sizeof(uint2) * nk, "emigrants"));
+        MPM_TRY(grow(far_, sizeof(uint2) * nk, "far movers"));
+        MPM_TRY(grow(arrivals_, sizeof(unsigned long long) * nk, "arrivals"));
+        MPM_TRY(grow(far_count_, sizeof(uint32_t) * 2, "far mover counts"));
+        for (int k = 0; k < 2; ++k)
+            CUDA_TRY(cudaMemsetAsync(emig_count_[k].p, 0, sizeof(uint32_t) * tb, stream_));
+        CUDA_TRY(cudaMemsetAsync(far_count_.p, 0, sizeof(uint32_t) * 2, stream_));
+        sort_list_cap_ = (uint32_t)std::min<size_t>(tb, nk);
+        MPM_TRY(grow(sort_list_, sizeof(BlockItem) * sort_list_cap_, "block sort list"));
+        dense_cap_ = (uint32_t)(nk / kDenseBlock);
+        MPM_TRY(grow(dense_list_, sizeof(BlockItem) * (dense_cap_ + 1), "dense block list"));
         MPM_TRY(grow(compact_scratch_, sizeof(unsigned long long) * compactScratchWords64((uint32_t)tb),
                                        "compaction scratch"));
         MPM_TRY(grow(block_count_, sizeof(uint32_t) * tb, "block counts"));
@@ -1187,6 +1203,12 @@ public:
         bb.block_slot = block_slot_.as<int2>();
         bb.p2g_lists = p2g_lists_.as<uint32_t>();
         bb.p2g_list_cap = (uint32_t)max_active_;
+        bb.block_range = range_[parity_].as<uint2>();
+        bb.emig_count = emig_count_[parity_ ^ 1].as<uint32_t>();
+        bb.far_count = far_count_.as<uint32_t>() + (parity_ ^ 1);
+        bb.sort_list = sort_list_.as<BlockItem>();
+        bb.sort_list_cap = sort_list_cap_;
+        bb.dense_list = dense_list_.as<BlockItem>();
         return bb;
     }
 
@@ -1223,6 +1245,10 @@ public:
 
     // Keys of the live order (if stale) + sort + compaction.
     mpm_status sortLive() {
+        // The block sort serves when the live order is the last sorted order
+        // and the keys are G2P's (the particles have moved by one step): every
+        // step but the first after an upload or a split call.
+        const bool by_blocks = incremental_ok_ && keys_valid_ && !full_sort_only_;
         if (!keys_valid_) {
             mark(KF_KEYS, 0);
             CUDA_TRY(cudaMemsetAsync(block_count_.p, 0, sizeof(uint32_t) * total_blocks_, stream_));
@@ -1231,53 +1257,98 @@ public:
             collect(KF_KEYS);
             keys_valid_ = true;
         }
-        const bool incremental =
-            incremental_ok_ && !full_sort_only_ && (ntot_ >= kIncrementalMinKeys || incremental_always_);
-        // The block compaction reads only the per-block counts, not the sorted
-        // keys: beside the full radix sort (both latency-bound) it runs on its
-        // own stream and joins before the caller's next launch (two-ball step
-        // 0.425 -> 0.418 ms).  Beside the incremental sort it costs more than
-        // it hides (64-scene batch 2.34 -> 2.38 ms), and profiling keeps the
-        // families in sequence so that each is timed alone.
-        const bool overlap = !profiling_ && !incremental;
-        if (overlap) {
-            CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
-            CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
+        auto compact = [&](cudaStream_t st) {
             LaunchCtx cc = ctx();
-            cc.stream = compact_stream_;
-            launchCompactOnesweep(cc, blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), comboSplit(),
-                                  err_.as<uint32_t>());
-            CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
-        }
-        mark(KF_SORT, 0);
-        if (incremental) {
-            // keys_[1 - kcur_] still holds the previous step's sorted keys,
-            // aligned with the live particle order: sort incrementally into it
-            const int out = 1 - kcur_;
-            CUDA_TRY(incrementalSort(keys_[kcur_].as<uint32_t>(), keys_[out].as<uint32_t>(), ntot_, key_bits_,
-                                     keys_[out].as<uint32_t>(), vals_[out].as<uint32_t>(), inc_scratch_.as<uint32_t>(),
-                                     err_.as<uint32_t>(), stream_));
-            sorted_ = out;
+            cc.stream = st;
+            launchCompact(cc, blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(),
+                                  comboSplit(), err_.as<uint32_t>());
+        };
+        if (by_blocks) {
+            BlockSortArgs b;
+            b.scenes = scenes_dev_.as<SceneDev>();
+            b.nscenes = (int)scenes_.size();
+            b.scene_block_base = sbb_.as<uint32_t>();
+            b.keys = keys_[kcur_].as<uint32_t>();
+            b.prev_keys = keys_[1 - kcur_].as<uint32_t>();
+            b.prev_range = range_[parity_ ^ 1].as<uint2>();
+            b.emig_count = emig_count_[parity_].as<uint32_t>();
+            b.emig = emig_.as<uint2>();
+            b.far = far_.as<uint2>();
+            b.far_count = far_count_.as<uint32_t>() + parity_;
+            b.list = sort_list_.as<BlockItem>();
+            b.list_cap = sort_list_cap_;
+            b.dense = dense_list_.as<BlockItem>();
+            b.counters = counters_.as<uint32_t>();
+            b.aux = arrivals_.as<unsigned long long>();
+            // (the sorted keys go where the previous ones were: read by the
+            // emigrant kernel only, which is done by then)
+            b.out_keys = keys_[1 - kcur_].as<uint32_t>();
+            b.out_perm = vals_[1 - kcur_].as<uint32_t>();
+            b.err = err_.as<uint32_t>();
+            // the emigrant lists beside the compaction (in sequence under
+            // profiling, so that each family is timed alone)
+            const bool overlap = !profiling_;
+            mark(KF_SORT, 0);
+            if (overlap) {
+                CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
+                CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
+            }
+            CUDA_TRY(launchEmigrants(b, ntot_, num_sms_, overlap ? compact_stream_ : stream_));
+            if (overlap) CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
+            mark(KF_SORT, 1);
+            collect(KF_SORT);
+            mark(KF_COMPACT, 0);
+            compact(stream_);
+            mark(KF_COMPACT, 1);
+            collect(KF_COMPACT);
+            mark(KF_SORT, 0);
+            if (overlap) CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
+            if (dense_cap_) {
+                if (overlap) {
+                    CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
+                    CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
+                }
+                CUDA_TRY(launchBlockSort(b, dense_cap_, true, num_sms_, overlap ? compact_stream_ : stream_));
+                if (overlap) CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
+            }
+            CUDA_TRY(launchBlockSort(b, sort_list_cap_, false, num_sms_, stream_));
+            if (dense_cap_ && overlap) CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
+            sorted_ = 1 - kcur_;
         } else {
+            // The compaction reads only the per-block counts, not the sorted
+            // keys: beside the radix sort it runs on its own stream and joins
+            // before the caller's next launch (profiling keeps the families
+            // in sequence so that each is timed alone).
+            const bool overlap = !profiling_;
+            if (overlap) {
+                CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
+                CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
+                compact(compact_stream_);
+                CUDA_TRY(cudaGetLastError());
+                CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
+            }
+            mark(KF_SORT, 0);
             bool inB = false;
             CUDA_TRY(radixSortOnesweep(keys_[kcur_].as<uint32_t>(), vals_[kcur_].as<uint32_t>(),
                                        keys_[1 - kcur_].as<uint32_t>(), vals_[1 - kcur_].as<uint32_t>(), ntot_,
                                        key_bits_, sort_scratch_.as<uint32_t>(), err_.as<uint32_t>(), &inB, stream_));
             sorted_ = inB ? 1 - kcur_ : kcur_;
+            if (overlap) {
+                CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
+            } else {
+                mark(KF_SORT, 1);
+                collect(KF_SORT);
+                mark(KF_COMPACT, 0);
+                compact(stream_);
+                mark(KF_COMPACT, 1);
+                collect(KF_COMPACT);
+            }
+        }
+        if (by_blocks) {
+            mark(KF_SORT, 1);
+            collect(KF_SORT);
         }
         incremental_ok_ = false;  // set again once G2P has reordered the particles by this sort
-        mark(KF_SORT, 1);
-        collect(KF_SORT);
-        if (overlap) {
-            CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
-        } else {
-            mark(KF_COMPACT, 0);
-            launchCompactOnesweep(ctx(), blockBuffers(), total_blocks_, compact_scratch_.as<unsigned long long>(), comboSplit(),
-                                  err_.as<uint32_t>());
-            mark(KF_COMPACT, 1);
-            collect(KF_COMPACT);
-        }
         CUDA_TRY(cudaGetLastError());
         sorted_valid_ = true;
         return MPM_OK;
@@ -2398,21 +2469,16 @@ private:
     std::vector<std::array<cudaEvent_t, 4>> tune_ev_;  // per combination: P2G start/end, G2P start/end
     bool warp_check_ = true;
     // the previous step's sorted keys are aligned with the live particle order
-    // (sortLive may sort incrementally); MPM_FULL_SORT=1 always sorts all keys,
-    // MPM_INCREMENTAL_SORT=1 sorts incrementally whatever the size (both for
-    // tests and measurements)
+    // (sortLive may use the block sort); MPM_FULL_SORT=1 always sorts all keys
+    // (for tests and measurements)
     bool incremental_ok_ = false;
     const bool full_sort_only_ = getenv("MPM_FULL_SORT") != nullptr;
-    const bool incremental_always_ = getenv("MPM_INCREMENTAL_SORT") != nullptr;
-    // Below this many keys the full radix sort is faster (the movers' sort
-    // costs a few fixed-latency passes): 1M keys 0.072 ms full vs 0.100 ms
-    // incremental, 8.5M keys 0.43 ms vs 0.30 ms on the B200.
-    static constexpr size_t kIncrementalMinKeys = (size_t)3 << 20;
+    uint32_t sort_list_cap_ = 0, dense_cap_ = 0;
     int parity_ = 0, kcur_ = 0, sorted_ = 0;
     size_t ntot_ = 0, max_nodes_ = 0, max_n_ = 0, max_active_ = 1, tile_stride_ = 0;
     uint32_t total_blocks_ = 0;
     int key_bits_ = 1;
-    DevMem keys_[2], vals_[2], sort_scratch_, inc_scratch_, compact_scratch_, block_count_, sbb_, active_,
+    DevMem keys_[2], vals_[2], sort_scratch_, range_[2], emig_count_[2], emig_, far_, arrivals_, far_count_, sort_list_, dense_list_, compact_scratch_, block_count_, sbb_, active_,
         outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, tmp_, g2p_items_, tmaps_, spans_, p2g_lists_;
     // Per combination: the first step after a change of the scene set found
     // fewer than kWarpAutoMinItems small P2G items, so the step does not

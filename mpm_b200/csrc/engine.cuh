@@ -67,6 +67,15 @@ constexpr int kP2GSmallWord = kP2GListWord + 2 * kMaxCombos;
 // them) and the others from the back (counters[kP2GBackWord + k]), so that
 // the CTAs take the long items first and the short ones fill the tail.
 constexpr int kP2GBackWord = kP2GSmallWord + kMaxCombos;
+// [kSortFrontWord], [kSortBackWord], [kSortDenseWord]: entries of the block
+// sort's lists (blocks of at least kBigItem particles from the front, smaller
+// ones from the back; blocks of at least kDenseBlock apart);
+// [kSortSchedWord] .. [+ 5]: its work-item schedulers (CTAs, warps, dense).
+constexpr int kSortFrontWord = kP2GBackWord + kMaxCombos;
+constexpr int kSortBackWord = kSortFrontWord + 1;
+constexpr int kSortDenseWord = kSortFrontWord + 2;
+constexpr int kSortSchedWord = kSortFrontWord + 3;
+constexpr uint32_t kDenseBlock = 4096;
 constexpr uint32_t kBigItem = 768;
 constexpr uint32_t kWarpAutoMax = 256;
 constexpr uint32_t kWarpAutoMinItems = 1024;
@@ -79,7 +88,7 @@ __host__ __device__ inline bool p2gWarpTakesSmall(int mode, uint32_t n_small) {
     return mode == P2G_WARP_ALWAYS || (mode == P2G_WARP_AUTO && n_small >= kWarpAutoMinItems);
 }
 constexpr int kCounterWords = 128;
-static_assert(kP2GBackWord + kMaxCombos <= kCounterWords, "counter words");
+static_assert(kSortSchedWord + 6 <= kCounterWords, "counter words");
 
 enum Field : int {
     F_X = 0,

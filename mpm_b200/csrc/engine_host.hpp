@@ -34,6 +34,12 @@ struct BlockBuffers {
     int2* block_slot;                 // total_blocks
     uint32_t* p2g_lists;              // P2G item slots, 2 lists of p2g_list_cap per combination
     uint32_t p2g_list_cap;
+    uint2* block_range;               // total_blocks: (first sorted particle, count)
+    uint32_t* emig_count;             // total_blocks: cleared for the next step
+    uint32_t* far_count;              // likewise
+    BlockItem* sort_list;             // see BlockSortArgs
+    uint32_t sort_list_cap;
+    BlockItem* dense_list;
 };
 
 // Host-side count of kernel launches issued by the library (kernels.cu).
@@ -58,12 +64,32 @@ size_t onesweepScratchWords(size_t n, int bits);
 cudaError_t radixSortOnesweep(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, size_t n,
                               int bits, uint32_t* scratch, uint32_t* err, bool* result_in_b, cudaStream_t st,
                               const uint32_t* n_dev = nullptr);
-// Incremental sort (sort.cu): the stable sort of `keys` (n, live order) given
-// that `prev` (the previous step's sorted keys, aligned with the same live
-// order) is ascending.  Output equals radixSortOnesweep's (keys, perm).
-size_t incrementalSortScratchWords(size_t n, int bits);
-cudaError_t incrementalSort(const uint32_t* keys, const uint32_t* prev, size_t n, int bits, uint32_t* out_keys,
-                            uint32_t* out_perm, uint32_t* scratch, uint32_t* err, cudaStream_t st);
+// Block sort (sort.cu): the stable sort of `keys` (live order) given that the
+// live order is the order of the previous sort: launchEmigrants lists the
+// particles that left their blocks (counts zero before), the compaction the
+// occupied blocks with their new ranges, then launchBlockSort sorts.  Output equals radixSortOnesweep's (keys, perm).
+struct BlockSortArgs {
+    const SceneDev* scenes;
+    int nscenes;
+    const uint32_t* scene_block_base;
+    const uint32_t* keys;        // live order
+    const uint32_t* prev_keys;   // live order: the previous step's sorted keys
+    const uint2* prev_range;     // per block: (first, count) in the live order
+    uint32_t* emig_count;        // per block: particles that left it for a neighbouring block
+    uint2* emig;                 // (live index, key) of those of block b from prev_range[b].x on
+    uint2* far;                  // (live index, key) of the other particles that left their block
+    uint32_t* far_count;
+    const BlockItem* list;       // occupied blocks and their new ranges, full ones from the front,
+    uint32_t list_cap;           // the others from the back (kSortFrontWord, kSortBackWord)
+    const BlockItem* dense;      // the blocks of at least kDenseBlock particles (kSortDenseWord)
+    uint32_t* counters;
+    unsigned long long* aux;     // one word per particle: arrivals that exceed shared memory
+    uint32_t *out_keys, *out_perm;
+    uint32_t* err;
+};
+cudaError_t launchEmigrants(const BlockSortArgs& a, size_t n, int num_sms, cudaStream_t st);
+// `dense`: the dense blocks (they may run beside the others, on another stream).
+cudaError_t launchBlockSort(const BlockSortArgs& a, unsigned max_blocks, bool dense, int num_sms, cudaStream_t st);
 cudaError_t radixSortPairsInto(const uint32_t* in_keys, uint32_t* out_keys, uint32_t* out_vals, uint32_t* tmp_keys,
                                uint32_t* tmp_vals, size_t n, int bits, uint32_t* hist, uint32_t* scan_partials,
                                cudaStream_t st);
@@ -78,7 +104,7 @@ struct ComboSplit {
     uint32_t g2p_chunk[kMaxCombos];
     uint32_t p2g_warp_max[kMaxCombos];
 };
-void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks,
+void launchCompact(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks,
                            unsigned long long* scratch, const ComboSplit& split, uint32_t* err);
 void launchStress(const LaunchCtx& c, int parity);
 void launchP2G(const LaunchCtx& c, const StepArgs& a, int S, int mode, int want_transfer);

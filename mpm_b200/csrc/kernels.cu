@@ -15,6 +15,7 @@
 //                   (src/mpm_solver3d.cu:316-391,428-445; apic :326-388)
 //   split-mode kernels for the reference's sub-step API.
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched at run time)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -150,18 +151,22 @@ __global__ void __launch_bounds__(kThreads) keyKernel(const SceneDev* __restrict
     }
 }
 
-// Block compaction in one kernel: each CTA scans a tile of 1024 block counts,
+// Block compaction in one kernel: each CTA scans a tile of 512 block counts,
 // publishes the tile's (work items, particles) sums and looks back over the
 // earlier tiles' published words (single-pass scan, dynamic tile ids, every
 // wait bounded), then writes the work items, slots and outside items of its
 // blocks and clears their counts.  Word layout: [63:62] flag, [61:32] items,
 // [31:0] particles.
-constexpr int kCompactPer = 4;
-constexpr int kCompactTile = kThreads * kCompactPer;
+// one block a thread, so that neighbouring threads write neighbouring words of
+// the dense tables (two-ball step 0.268 ms; four a thread 0.271 ms, four a
+// thread of 1024 0.277 ms)
+constexpr int kCompactPer = 1, kCompactThreads = 512;
+constexpr int kCompactTile = kCompactThreads * kCompactPer;
 constexpr unsigned long long kCFlagAgg = 1ull << 62, kCFlagPrefix = 2ull << 62, kCFlagMask = 3ull << 62;
 
+template <int W>  // warps of the CTA
 __device__ __forceinline__ unsigned long long blockExclusiveScanU64(unsigned long long x, unsigned long long* total) {
-    __shared__ unsigned long long wt[kWarps];
+    __shared__ unsigned long long wt[W];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long inc = x;
 #pragma unroll
@@ -172,14 +177,14 @@ __device__ __forceinline__ unsigned long long blockExclusiveScanU64(unsigned lon
     if (lane == 31) wt[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        unsigned long long t = lane < kWarps ? wt[lane] : 0ull, ti = t;
+        unsigned long long t = lane < W ? wt[lane] : 0ull, ti = t;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned long long y = __shfl_up_sync(0xffffffffu, ti, o);
             if (lane >= o) ti += y;
         }
-        if (lane < kWarps) wt[lane] = ti - t;
-        const unsigned long long tl = __shfl_sync(0xffffffffu, ti, kWarps - 1);
+        if (lane < W) wt[lane] = ti - t;
+        const unsigned long long tl = __shfl_sync(0xffffffffu, ti, W - 1);
         if (lane == 0) *total = tl;
     }
     __syncthreads();
@@ -201,13 +206,184 @@ __device__ __forceinline__ void splitItems(BlockItem* out, uint32_t b, uint32_t 
     }
 }
 
-__global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
-    uint32_t* __restrict__ block_count, uint32_t total_blocks, const uint32_t* __restrict__ scene_block_base,
-    int nscenes, BlockItem* __restrict__ active, BlockItem* __restrict__ outside, uint32_t* __restrict__ counters,
-    int2* __restrict__ block_slot, unsigned long long* __restrict__ status, uint32_t* __restrict__ tile_counter,
-    uint32_t ntiles, BlockItem* __restrict__ g2p_items, uint32_t g2p_cap, ComboSplit split,
-    uint32_t* __restrict__ p2g_lists, uint32_t p2g_list_cap, const SceneDev* __restrict__ scenes,
-    uint32_t* __restrict__ err) {
+struct CompactArgs {
+    uint32_t* block_count;
+    uint32_t total_blocks;
+    const uint32_t* scene_block_base;
+    int nscenes;
+    BlockItem *active, *outside;
+    uint32_t* counters;
+    int2* block_slot;
+    BlockItem* g2p_items;
+    uint32_t g2p_cap;
+    ComboSplit split;
+    uint32_t* p2g_lists;
+    uint32_t p2g_list_cap;
+    uint2* block_range;
+    uint32_t *emig_count, *far_count;
+    BlockItem* sort_list;
+    uint32_t sort_list_cap;
+    BlockItem* dense_list;
+    const SceneDev* scenes;
+    uint32_t* err;
+};
+
+// Block b's (work items << 32 | particles) and its scene.
+__device__ __forceinline__ unsigned long long blockLoad(const CompactArgs& a, uint32_t b, int* scene) {
+    *scene = 0;
+    if (b >= a.total_blocks) return 0ull;
+    const uint32_t c = a.block_count[b];
+    const int s = *scene = sceneOfBlock(a.scene_block_base, a.nscenes, b);
+    const bool out = b == a.scene_block_base[s + 1] - 1;
+    return ((out ? 0ull : (unsigned long long)blockItems(c)) << 32) | (unsigned long long)c;
+}
+
+// The work items, slots, ranges and list entries of the thread's PER blocks
+// from b0 on, `run` the (items, particles) of all blocks before them.
+template <int PER>
+__device__ __forceinline__ void placeBlocks(const CompactArgs& a, uint32_t b0, const unsigned long long (&packed)[PER],
+                                            const int (&scn)[PER], unsigned long long run) {
+    // Slots are aggregated per warp when every block of the warp that has
+    // items belongs to one combination (the common case), else taken per block.
+    uint32_t gtot = 0;
+    int gcombo = -1;
+    bool mixed = false;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t b = b0 + j;
+        if (b >= a.total_blocks) continue;
+        if ((packed[j] >> 32) == 0) continue;
+        const uint32_t count = (uint32_t)(packed[j] & 0xffffffffull);
+        const int k = a.scenes[scn[j]].combo;
+        gtot += (count + a.split.g2p_chunk[k] - 1) / a.split.g2p_chunk[k];
+        if (gcombo < 0) gcombo = k;
+        else mixed |= k != gcombo;
+    }
+    const int lane = threadIdx.x & 31;
+    const unsigned has = __ballot_sync(0xffffffffu, gtot > 0);
+    const int lead = __shfl_sync(0xffffffffu, gcombo, has ? __ffs(has) - 1 : 0);
+    const bool warp_fast = __all_sync(0xffffffffu, gtot == 0 || (!mixed && gcombo == lead));
+    // Slots of this thread's P2G items in their combination's lists: list 0
+    // for items of at most the combination's warp threshold (P2G by warps),
+    // list 1 for the others -- those of at least kBigItem particles from its
+    // front, the rest from its back (class 2); the items of at most
+    // kWarpAutoMax particles are counted as well (class 3).  Then of its
+    // blocks in the block sort's lists (classes 5 to 7).  Totals per warp, and
+    // the classes' atomics issued together, each by a lane of its own (one
+    // after another, each waited for, they took a third of the kernel).
+    constexpr int kClasses = 8;  // P2G 0..3, G2P 4, block sort 5, 6, 7
+    uint32_t ctot[kClasses] = {};
+    if (warp_fast) ctot[4] = gtot;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (b0 + j >= a.total_blocks) continue;
+        const uint32_t items = (uint32_t)(packed[j] >> 32), count = (uint32_t)(packed[j] & 0xffffffffull);
+        ctot[5] += count >= kBigItem && count < kDenseBlock ? 1u : 0u;
+        ctot[6] += count && count < kBigItem ? 1u : 0u;
+        ctot[7] += count >= kDenseBlock ? 1u : 0u;
+        if (!a.p2g_lists || !warp_fast || !items) continue;
+        const uint32_t size = (count + items - 1) / items;
+        const int cls = size <= a.split.p2g_warp_max[lead] ? 0 : (size >= kBigItem ? 1 : 2);
+        ctot[0] += cls == 0 ? items : 0u;
+        ctot[1] += cls == 1 ? items : 0u;
+        ctot[2] += cls == 2 ? items : 0u;
+        if (size <= kWarpAutoMax) ctot[3] += items;
+    }
+    uint32_t cnext[kClasses], want = 0;
+#pragma unroll
+    for (int cls = 0; cls < kClasses; ++cls) {
+        uint32_t inc = ctot[cls];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        cnext[cls] = inc - ctot[cls];
+        const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+        if (lane == cls) want = all;
+    }
+    {
+        const int word = lane < 2    ? kP2GListWord + 2 * lead + lane
+                         : lane == 2 ? kP2GBackWord + lead
+                         : lane == 3 ? kP2GSmallWord + lead
+                         : lane == 4 ? kG2PCountWord + lead
+                         : lane == 5 ? kSortFrontWord
+                         : lane == 6 ? kSortBackWord
+                                     : kSortDenseWord;
+        const uint32_t base = lane < kClasses && want ? atomicAdd(&a.counters[word], want) : 0u;
+#pragma unroll
+        for (int cls = 0; cls < kClasses; ++cls) cnext[cls] += __shfl_sync(0xffffffffu, base, cls);
+    }
+    uint32_t gnext = cnext[4];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t b = b0 + j;
+        if (b >= a.total_blocks) break;
+        const unsigned long long v = packed[j];
+        const uint32_t count = (uint32_t)(v & 0xffffffffull);
+        const uint32_t items = (uint32_t)(v >> 32);
+        const uint32_t start = (uint32_t)(run & 0xffffffffull);
+        const int scene = scn[j];
+        a.block_range[b] = make_uint2(start, count);
+        a.emig_count[b] = 0u;
+        if (count) {
+            const BlockItem e{b, start, count, (uint32_t)scene};
+            if (count >= kDenseBlock) a.dense_list[cnext[7]++] = e;
+            else if (count >= kBigItem) a.sort_list[cnext[5]++] = e;
+            else a.sort_list[a.sort_list_cap - 1 - cnext[6]++] = e;
+        }
+        // a block's items have count / items particles, the first
+        // count % items of them one more (sizes differ by at most one)
+        if (items) {
+            const uint32_t slot = (uint32_t)(run >> 32);
+            splitItems(a.active + slot, b, start, count, items, (uint32_t)scene);
+            a.block_slot[b] = make_int2((int)slot, (int)items);
+            // G2P's items of the block, in its combination's list at slots
+            // taken from a counter (their order does not matter)
+            const int k = a.scenes[scene].combo;
+            const uint32_t parts = (count + a.split.g2p_chunk[k] - 1) / a.split.g2p_chunk[k];
+            uint32_t g0;
+            if (warp_fast) {
+                g0 = gnext;
+                gnext += parts;
+            } else {
+                g0 = atomicAdd(&a.counters[kG2PCountWord + k], parts);
+            }
+            splitItems(a.g2p_items + (size_t)k * a.g2p_cap + g0, b, start, count, parts, (uint32_t)scene);
+            if (a.p2g_lists) {
+                const uint32_t size = (count + items - 1) / items;
+                const int cls = size <= a.split.p2g_warp_max[k] ? 0 : (size >= kBigItem ? 1 : 2);
+                uint32_t p0;
+                if (warp_fast) {
+                    p0 = cls == 0 ? cnext[0] : cls == 1 ? cnext[1] : cnext[2];
+                    cnext[0] += cls == 0 ? items : 0u;
+                    cnext[1] += cls == 1 ? items : 0u;
+                    cnext[2] += cls == 2 ? items : 0u;
+                } else {
+                    p0 = atomicAdd(&a.counters[cls == 2 ? kP2GBackWord + k : kP2GListWord + 2 * k + cls], items);
+                    if (size <= kWarpAutoMax) atomicAdd(&a.counters[kP2GSmallWord + k], items);
+                }
+                uint32_t* lst = a.p2g_lists + (size_t)(2 * k + (cls == 0 ? 0 : 1)) * a.p2g_list_cap;
+                for (uint32_t q = 0; q < items; ++q) {
+                    if (cls == 2) lst[a.p2g_list_cap - 1 - (p0 + q)] = slot + q;  // from the back
+                    else lst[p0 + q] = slot + q;
+                }
+            }
+        } else {
+            a.block_slot[b] = make_int2(-1, 0);
+            if (count > 0) {
+                const uint32_t nitems = blockItems(count);
+                const uint32_t o = atomicAdd(&a.counters[1], nitems);
+                splitItems(a.outside + o, b, start, count, nitems, (uint32_t)scene);
+            }
+        }
+        a.block_count[b] = 0;
+        run += v;
+    }
+}
+
+__global__ void __launch_bounds__(kCompactThreads) compactOnesweepKernel(CompactArgs a, unsigned long long* __restrict__ status,
+                                                                  uint32_t* __restrict__ tile_counter, uint32_t ntiles) {
     __shared__ uint32_t tile_s;
     __shared__ unsigned long long tot, excl_s;
     if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1u);
@@ -215,22 +391,11 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
     const uint32_t tile = tile_s;
     const uint32_t b0 = tile * kCompactTile + threadIdx.x * kCompactPer;
     unsigned long long packed[kCompactPer];
+    int scn[kCompactPer];
     unsigned long long sum = 0;
 #pragma unroll
-    for (int j = 0; j < kCompactPer; ++j) {
-        const uint32_t b = b0 + j;
-        unsigned long long v = 0;
-        if (b < total_blocks) {
-            const uint32_t c = block_count[b];
-            const int s = sceneOfBlock(scene_block_base, nscenes, b);
-            const bool out = (b == scene_block_base[s + 1] - 1);
-            const unsigned long long items = out ? 0ull : (unsigned long long)blockItems(c);
-            v = (items << 32) | (unsigned long long)c;
-        }
-        packed[j] = v;
-        sum += v;
-    }
-    unsigned long long run = blockExclusiveScanU64(sum, &tot);
+    for (int j = 0; j < kCompactPer; ++j) sum += packed[j] = blockLoad(a, b0 + j, &scn[j]);
+    unsigned long long run = blockExclusiveScanU64<kCompactThreads / 32>(sum, &tot);
     if (threadIdx.x == 0) {
         unsigned long long excl = 0;
         if (tile == 0) {
@@ -261,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
                 }
                 if (waiting) {
                     if (++polls > (1 << 22)) {  // never expected: give up instead of hanging
-                        atomicOr(err, 16u);
+                        atomicOr(a.err, 16u);
                         break;
                     }
                     __nanosleep(32);
@@ -270,134 +435,54 @@ __global__ void __launch_bounds__(kThreads) compactOnesweepKernel(
             atomicExch(&status[tile], kCFlagPrefix | (excl + tot));
         }
         excl_s = excl;
-        if (tile == ntiles - 1) counters[0] = (uint32_t)((excl + tot) >> 32);
+        if (tile == ntiles - 1) a.counters[0] = (uint32_t)((excl + tot) >> 32);
     }
     __syncthreads();
     run += excl_s;
-    // Slots of this thread's G2P items: one atomic per warp when every block
-    // of the warp that has items belongs to one combination (the common
-    // case), else one per block.
-    int scn[kCompactPer];
-    uint32_t gtot = 0;
-    int gcombo = -1;
-    bool mixed = false;
-#pragma unroll
-    for (int j = 0; j < kCompactPer; ++j) {
-        const uint32_t b = b0 + j;
-        scn[j] = 0;
-        if (b >= total_blocks) continue;
-        scn[j] = sceneOfBlock(scene_block_base, nscenes, b);
-        if ((packed[j] >> 32) == 0) continue;
-        const uint32_t count = (uint32_t)(packed[j] & 0xffffffffull);
-        const int k = scenes[scn[j]].combo;
-        gtot += (count + split.g2p_chunk[k] - 1) / split.g2p_chunk[k];
-        if (gcombo < 0) gcombo = k;
-        else mixed |= k != gcombo;
+    if (tile == 0 && threadIdx.x == 0) *a.far_count = 0u;
+    placeBlocks<kCompactPer>(a, b0, packed, scn, run);
+}
+
+// The same compaction by one cluster of eight CTAs of 1024 threads, one block a
+// thread, for scenes of at most kClusterBlocks blocks: the CTAs read one
+// another's totals from shared memory.  No status words to clear, no look-back
+// and no clear of the counters ahead of it (the first CTA zeroes them before
+// the cluster barrier).  What bounds both is the latency of a few dependent
+// reads and atomics (65k-particle cube, 5,833 blocks: clear and compaction
+// 13.5 us, this one 9.0).  With more blocks a thread, eight SMs write the
+// dense block table more slowly than the whole GPU does in the kernel above
+// (two-ball scene, 36k blocks: 0.020 ms more a step).
+constexpr int kClusterCtas = 8, kClusterThreads = 1024;
+constexpr uint32_t kClusterBlocks = kClusterCtas * kClusterThreads;
+
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
+    compactClusterKernel(CompactArgs a) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ unsigned long long tot;
+    const uint32_t rank = cluster.block_rank(), b0 = rank * kClusterThreads + threadIdx.x;
+    if (rank == 0) {
+        const int t = threadIdx.x;
+        if (t < 4) a.counters[t] = 0u;
+        if (t < kMaxCombos) a.counters[kG2PCountWord + t] = 0u;
+        if (t >= kP2GListWord && t < kSortSchedWord) a.counters[t] = 0u;
+        if (t == 0) *a.far_count = 0u;
     }
-    const int lane = threadIdx.x & 31;
-    const unsigned has = __ballot_sync(0xffffffffu, gtot > 0);
-    const int lead = __shfl_sync(0xffffffffu, gcombo, has ? __ffs(has) - 1 : 0);
-    const bool warp_fast = __all_sync(0xffffffffu, gtot == 0 || (!mixed && gcombo == lead));
-    uint32_t gnext = 0;
-    if (warp_fast && has) {
-        uint32_t inc = gtot;
+    unsigned long long packed[1];
+    int scn[1];
+    packed[0] = blockLoad(a, b0, &scn[0]);
+    unsigned long long run = blockExclusiveScanU64<kClusterThreads / 32>(packed[0], &tot), total = 0;
+    cluster.sync();  // every CTA's total is in its `tot`, the counters are zero
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
-        }
-        uint32_t base = 0;
-        if (lane == 31) base = atomicAdd(&counters[kG2PCountWord + lead], inc);
-        gnext = __shfl_sync(0xffffffffu, base, 31) + inc - gtot;
+    for (int r = 0; r < kClusterCtas; ++r) {
+        const unsigned long long x = *cluster.map_shared_rank(&tot, r);
+        if (r < (int)rank) run += x;
+        total += x;
     }
-    // Slots of this thread's P2G items in their combination's lists: list 0
-    // for items of at most the combination's warp threshold (P2G by warps),
-    // list 1 for the others -- those of at least kBigItem particles from its
-    // front, the rest from its back (class 2); aggregated per warp like the
-    // G2P items.  The items of at most kWarpAutoMax particles are counted
-    // as well (class 3).
-    uint32_t pnext[3] = {0u, 0u, 0u};
-    if (p2g_lists && warp_fast && has) {
-        uint32_t ptot[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int j = 0; j < kCompactPer; ++j) {
-            const uint32_t items = (uint32_t)(packed[j] >> 32);
-            if (b0 + j >= total_blocks || !items) continue;
-            const uint32_t size = ((uint32_t)(packed[j] & 0xffffffffull) + items - 1) / items;
-            ptot[size <= split.p2g_warp_max[lead] ? 0 : (size >= kBigItem ? 1 : 2)] += items;
-            if (size <= kWarpAutoMax) ptot[3] += items;
-        }
-        const int words[4] = {kP2GListWord + 2 * lead, kP2GListWord + 2 * lead + 1, kP2GBackWord + lead,
-                              kP2GSmallWord + lead};
-#pragma unroll
-        for (int cls = 0; cls < 4; ++cls) {
-            uint32_t inc = ptot[cls];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            uint32_t base = 0;
-            if (lane == 31 && inc) base = atomicAdd(&counters[words[cls]], inc);
-            if (cls < 3) pnext[cls] = __shfl_sync(0xffffffffu, base, 31) + inc - ptot[cls];
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kCompactPer; ++j) {
-        const uint32_t b = b0 + j;
-        if (b >= total_blocks) break;
-        const unsigned long long v = packed[j];
-        const uint32_t count = (uint32_t)(v & 0xffffffffull);
-        const uint32_t items = (uint32_t)(v >> 32);
-        const uint32_t start = (uint32_t)(run & 0xffffffffull);
-        const int scene = scn[j];
-        // a block's items have count / items particles, the first
-        // count % items of them one more (sizes differ by at most one)
-        if (items) {
-            const uint32_t slot = (uint32_t)(run >> 32);
-            splitItems(active + slot, b, start, count, items, (uint32_t)scene);
-            block_slot[b] = make_int2((int)slot, (int)items);
-            // G2P's items of the block, in its combination's list at slots
-            // taken from a counter (their order does not matter)
-            const int k = scenes[scene].combo;
-            const uint32_t parts = (count + split.g2p_chunk[k] - 1) / split.g2p_chunk[k];
-            uint32_t g0;
-            if (warp_fast) {
-                g0 = gnext;
-                gnext += parts;
-            } else {
-                g0 = atomicAdd(&counters[kG2PCountWord + k], parts);
-            }
-            splitItems(g2p_items + (size_t)k * g2p_cap + g0, b, start, count, parts, (uint32_t)scene);
-            if (p2g_lists) {
-                const uint32_t size = (count + items - 1) / items;
-                const int cls = size <= split.p2g_warp_max[k] ? 0 : (size >= kBigItem ? 1 : 2);
-                const int words[3] = {kP2GListWord + 2 * k, kP2GListWord + 2 * k + 1, kP2GBackWord + k};
-                uint32_t p0;
-                if (warp_fast) {
-                    p0 = pnext[cls];
-                    pnext[cls] += items;
-                } else {
-                    p0 = atomicAdd(&counters[words[cls]], items);
-                    if (size <= kWarpAutoMax) atomicAdd(&counters[kP2GSmallWord + k], items);
-                }
-                uint32_t* lst = p2g_lists + (size_t)(2 * k + (cls == 0 ? 0 : 1)) * p2g_list_cap;
-                for (uint32_t q = 0; q < items; ++q) {
-                    if (cls == 2) lst[p2g_list_cap - 1 - (p0 + q)] = slot + q;  // from the back
-                    else lst[p0 + q] = slot + q;
-                }
-            }
-        } else {
-            block_slot[b] = make_int2(-1, 0);
-            if (count > 0) {
-                const uint32_t nitems = blockItems(count);
-                const uint32_t o = atomicAdd(&counters[1], nitems);
-                splitItems(outside + o, b, start, count, nitems, (uint32_t)scene);
-            }
-        }
-        block_count[b] = 0;
-        run += v;
-    }
+    cluster.barrier_arrive();
+    if (rank == 0 && threadIdx.x == 0) a.counters[0] = (uint32_t)(total >> 32);
+    placeBlocks<1>(a, b0, packed, scn, run);
+    cluster.barrier_wait();  // the others have read this CTA's total
 }
 
 // ---------------------------------------------------------------------------
@@ -2291,8 +2376,18 @@ size_t compactScratchWords64(uint32_t total_blocks) {
     return (size_t)(total_blocks + kCompactTile - 1) / kCompactTile + 1;  // + the tile counter
 }
 
-void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks,
-                           unsigned long long* scratch, const ComboSplit& split, uint32_t* err) {
+void launchCompact(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_blocks, unsigned long long* scratch,
+                   const ComboSplit& split, uint32_t* err) {
+    const CompactArgs a{bb.block_count, total_blocks,     bb.scene_block_base, c.nscenes,        bb.active,
+                        bb.outside,     bb.counters,      bb.block_slot,       bb.g2p_items,     bb.g2p_cap,
+                        split,          bb.p2g_lists,     bb.p2g_list_cap,     bb.block_range,   bb.emig_count,
+                        bb.far_count,   bb.sort_list,     bb.sort_list_cap,    bb.dense_list,    c.scenes,
+                        err};
+    if (total_blocks <= kClusterBlocks) {
+        noteLaunches(1);
+        compactClusterKernel<<<kClusterCtas, kClusterThreads, 0, c.stream>>>(a);
+        return;
+    }
     const uint32_t ntiles = (uint32_t)((total_blocks + kCompactTile - 1) / kCompactTile);
     ClearRanges cr;
     cr.p[0] = reinterpret_cast<uint32_t*>(scratch);
@@ -2301,14 +2396,11 @@ void launchCompactOnesweep(const LaunchCtx& c, const BlockBuffers& bb, uint32_t 
     cr.n[1] = 4;
     cr.p[2] = bb.counters + kG2PCountWord;
     cr.n[2] = kMaxCombos;
-    cr.p[3] = bb.counters + kP2GListWord;  // lists, small, back
-    cr.n[3] = 4 * kMaxCombos;
+    cr.p[3] = bb.counters + kP2GListWord;  // lists, small, back, the block sort's lists
+    cr.n[3] = kSortSchedWord - kP2GListWord;
     launchClear(cr, c.stream);
     noteLaunches(1);
-    compactOnesweepKernel<<<ntiles, kThreads, 0, c.stream>>>(
-        bb.block_count, total_blocks, bb.scene_block_base, c.nscenes, bb.active, bb.outside, bb.counters,
-        bb.block_slot, scratch + 1, reinterpret_cast<uint32_t*>(scratch), ntiles, bb.g2p_items, bb.g2p_cap,
-        split, bb.p2g_lists, bb.p2g_list_cap, c.scenes, err);
+    compactOnesweepKernel<<<ntiles, kCompactThreads, 0, c.stream>>>(a, scratch + 1, reinterpret_cast<uint32_t*>(scratch), ntiles);
 }
 
 void launchStress(const LaunchCtx& c, int parity) {

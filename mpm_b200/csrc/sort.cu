@@ -12,6 +12,8 @@
 
 #include "engine_host.hpp"
 
+#include <algorithm>
+
 namespace mpm {
 
 namespace {
@@ -486,253 +488,387 @@ cudaError_t radixSortPairsInto(const uint32_t* in_keys, uint32_t* out_keys, uint
 }
 
 // ---------------------------------------------------------------------------
-// Incremental sort.  Between two steps most particles keep their cell key.
-// The live particle order is the previous step's sorted order, so the keys
-// that did not change ("stayers") already appear in ascending order; only the
-// particles whose key changed ("movers") need sorting.  Steps:
-//   1. partition (one pass, look-back over tiles): stayers (key, index) and
-//      movers (key, index), both in live order;
-//   2. radix-sort the movers by key (stable: ties stay in index order);
-//   3. merge the two sequences by (key, index).
-// Every sequence is ordered by (key, live index), so the result is exactly
-// the stable sort of all keys: the same keys and permutation as
-// radixSortOnesweep.
+// Block sort: the stable sort of the step's cell keys, given that the live order
+// is the previous step's sorted order.  Particles move a fraction of a cell per
+// step, so nearly all of a block's particles were in it before, in order.  One
+// kernel lists the particles that left their block (its emigrants, in the
+// block's own range of `emig`; those that went further than a neighbouring
+// block, or in or out of the grid, in `far`) beside the compaction, which gives
+// every block its new range; then every occupied block is put together on its
+// own: the particles that stayed in it, by a counting sort over its 64 cells,
+// and the arrivals, picked from the neighbours' lists and sorted by (cell, live
+// index).  Blocks are in key order, so an arrival from a lower block goes before
+// the cell's own particles and one from a higher block after them: the result
+// is exactly the stable sort of all keys, the same keys and permutation as
+// radixSortOnesweep's.
+// What bounds it is the latency of one block (list entry, ranges, keys: a few
+// dependent reads from L2), paid once where a radix sort pays a launch and a
+// look-back chain in every pass: blocks of at least kBigItem particles are taken
+// by CTAs, first, the others by single warps (by CTAs where they are few), and
+// blocks of at least kDenseBlock by CTAs of 1024 threads beside them.  Sort and
+// compaction per step, against the radix sort: 65k-particle cube 0.033 -> 0.023
+// ms, two-ball scene (1M) 0.064 -> 0.040 ms, 2M particles 0.090 -> 0.054 ms, and
+// against a sort of the particles that changed cells and a merge: slab (8.4M)
+// 0.19 -> 0.11 ms.  Six scenes of up to 60k particles in a few cells each lose
+// 0.006 ms of 0.123 (their crowded blocks are put together by one CTA each).
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kPartItems = 8;                        // consecutive keys per thread
-constexpr int kPartTile = kThreads * kPartItems;     // 2048
-constexpr int kMergeItems = 8;
-constexpr int kMergeTile = kThreads * kMergeItems;   // outputs per CTA
+constexpr int kBsThreads = 256, kBsWarps = kBsThreads / 32;
+constexpr uint32_t kBsFarScan = 4096; // far list read by every block up to this; above, the keys themselves
 
-// One tile of kPartTile keys: item j * kThreads + threadIdx.x of the tile is
-// this thread's j-th (coalesced loads and stores).  A key is a mover if it
-// differs from the previous step's key at the same position.  Movers keep
-// their order in b, stayers in a: the rank of an item among the movers of
-// its tile comes from per-warp ballots and one scan over (round, warp) in
-// item order, the tile's offset from the decoupled look-back.
-__global__ void __launch_bounds__(kThreads) moverPartitionKernel(
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ prev, uint32_t n, uint32_t* __restrict__ a_keys,
-    uint32_t* __restrict__ a_idx, uint32_t* __restrict__ b_keys, uint32_t* __restrict__ b_idx,
-    uint32_t* __restrict__ m_out, uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status, uint32_t ntiles,
-    uint32_t* __restrict__ err) {
-    constexpr int kW = kThreads / 32;
-    __shared__ uint32_t tile_s, excl_s;
-    __shared__ uint32_t wcnt[kPartItems * kW];  // movers per (round, warp), then their exclusive scan
-    if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1u);
-    __syncthreads();
-    const uint32_t tile = tile_s;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t t0 = (size_t)tile * kPartTile;
-    uint32_t k[kPartItems], ball[kPartItems];
-#pragma unroll
-    for (int j = 0; j < kPartItems; ++j) {
-        const size_t i = t0 + (size_t)j * kThreads + threadIdx.x;
-        const bool valid = i < n;
-        k[j] = valid ? keys[i] : 0u;
-        const uint32_t pk = valid ? prev[i] : 0u;
-        ball[j] = __ballot_sync(0xffffffffu, valid && k[j] != pk);
-        if (lane == 0) wcnt[j * kW + warp] = (uint32_t)__popc(ball[j]);
-    }
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan of the kPartItems * kW counts, in item order
-        static_assert(kPartItems * kW == 64, "two counts per lane");
-        const uint32_t c0 = wcnt[2 * lane], c1 = wcnt[2 * lane + 1];
-        uint32_t x = c0 + c1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
-        wcnt[2 * lane] = x - c0 - c1;
-        wcnt[2 * lane + 1] = x - c1;
-        if (lane == 0) {
-            uint32_t excl = 0;
-            if (tile == 0) {
-                atomicExch(&status[0], kFlagPrefix | tot);
-            } else {
-                atomicExch(&status[tile], kFlagAgg | tot);
-                // kLookWidth predecessor words per round trip, as in the radix passes
-                int t = (int)tile - 1;
-                int polls = 0;
-                bool done = false;
-                while (!done && t >= 0) {
-                    uint32_t w[kLookWidth];
-#pragma unroll
-                    for (int q = 0; q < kLookWidth; ++q)
-                        w[q] = (t - q >= 0) ? *(volatile const uint32_t*)(status + (t - q)) : kFlagPrefix;
-                    bool waiting = false;
-#pragma unroll
-                    for (int q = 0; q < kLookWidth; ++q) {
-                        if (done || waiting) continue;
-                        const uint32_t f = w[q] & ~kCountMask;
-                        if (f == 0) {  // not published yet: poll again from this tile
-                            waiting = true;
-                            continue;
-                        }
-                        excl += w[q] & kCountMask;
-                        --t;
-                        if (f == kFlagPrefix) done = true;
-                    }
-                    if (waiting) {
-                        if (++polls > kLookbackLimit) {  // never expected: give up instead of hanging
-                            atomicOr(err, 8u);
-                            break;
-                        }
-                        __nanosleep(32);
-                    }
-                }
-                atomicExch(&status[tile], kFlagPrefix | (excl + tot));
-            }
-            excl_s = excl;
-            if (tile == ntiles - 1) *m_out = excl + tot;
-        }
-    }
-    __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int j = 0; j < kPartItems; ++j) {
-        const size_t i = t0 + (size_t)j * kThreads + threadIdx.x;
-        if (i >= n) break;
-        const uint32_t mb = excl_s + wcnt[j * kW + warp] + (uint32_t)__popc(ball[j] & lt);  // movers before it
-        if (ball[j] >> lane & 1u) {
-            b_keys[mb] = k[j];
-            b_idx[mb] = (uint32_t)i;
-        } else {
-            const uint32_t pa = (uint32_t)i - mb;  // stayers before it
-            a_keys[pa] = k[j];
-            a_idx[pa] = (uint32_t)i;
-        }
-    }
-}
-
-__device__ __forceinline__ unsigned long long composite(uint32_t key, uint32_t idx) {
-    return ((unsigned long long)key << 32) | idx;
-}
-
-// Number of stayers among the first d outputs of the merge (merge path).
-__device__ __forceinline__ uint32_t mergePath(const uint32_t* a_keys, const uint32_t* a_idx, uint32_t na,
-                                              const uint32_t* b_keys, const uint32_t* b_idx, uint32_t nb, uint32_t d) {
-    uint32_t lo = d > nb ? d - nb : 0u, hi = d < na ? d : na;
+__device__ __forceinline__ int blockScene(const uint32_t* base, int nscenes, uint32_t b) {
+    int lo = 0, hi = nscenes - 1;
     while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        const uint32_t bj = d - 1 - mid;
-        if (composite(a_keys[mid], a_idx[mid]) < composite(b_keys[bj], b_idx[bj])) lo = mid + 1;
-        else hi = mid;
+        const int mid = (lo + hi + 1) >> 1;
+        if (base[mid] <= b) lo = mid;
+        else hi = mid - 1;
     }
     return lo;
 }
 
-// Split points of the merge: split[c] = stayers among the first c * kMergeTile outputs.
-__global__ void __launch_bounds__(kThreads) mergeSplitKernel(const uint32_t* __restrict__ a_keys,
-                                                              const uint32_t* __restrict__ a_idx,
-                                                              const uint32_t* __restrict__ b_keys,
-                                                              const uint32_t* __restrict__ b_idx, uint32_t n,
-                                                              const uint32_t* __restrict__ m_dev,
-                                                              uint32_t* __restrict__ split, uint32_t nsplit) {
-    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
-    if (c >= nsplit) return;
-    const uint32_t m = *m_dev, na = n - m;
-    const uint32_t d = (uint32_t)min((size_t)c * kMergeTile, (size_t)n);
-    split[c] = mergePath(a_keys, a_idx, na, b_keys, b_idx, m, d);
+__global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s, uint32_t n) {
+    const uint32_t stride = gridDim.x * kBsThreads * 4;
+    for (uint32_t i0 = (blockIdx.x * kBsThreads + threadIdx.x) * 4; i0 < n; i0 += stride) {
+        uint32_t key[4], old[4];
+        if (i0 + 4 <= n) {  // (the buffers are 256-byte aligned)
+            *reinterpret_cast<uint4*>(key) = *reinterpret_cast<const uint4*>(s.keys + i0);
+            *reinterpret_cast<uint4*>(old) = *reinterpret_cast<const uint4*>(s.prev_keys + i0);
+        } else {
+            for (int j = 0; j < 4; ++j) {
+                key[j] = i0 + j < n ? s.keys[i0 + j] : 0u;
+                old[j] = i0 + j < n ? s.prev_keys[i0 + j] : 0u;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t home = old[j] >> 6, blk = key[j] >> 6;
+            if (blk == home) continue;
+            const SceneDev& sc = s.scenes[blockScene(s.scene_block_base, s.nscenes, home)];
+            const uint32_t out = sc.nblocks, lh = home - sc.block_base, lb = blk - sc.block_base;
+            bool near = lh < out && lb < out;
+            if (near) {
+                const int X = sc.nb[0], Y = sc.nb[1];
+                const int dx = (int)(lh % X) - (int)(lb % X), dy = (int)(lh / X % Y) - (int)(lb / X % Y),
+                          dz = (int)(lh / (X * Y)) - (int)(lb / (X * Y));
+                near = abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
+            }
+            const uint2 e = make_uint2(i0 + j, key[j]);
+            if (near) s.emig[s.prev_range[home].x + atomicAdd(&s.emig_count[home], 1u)] = e;
+            else s.far[atomicAdd(s.far_count, 1u)] = e;
+        }
+    }
 }
 
-// One CTA merges kMergeTile outputs: its stayer and mover ranges are staged in
-// shared memory, each thread finds its own split there and merges 8 outputs
-// into a shared output tile, which the CTA then stores with unit stride.
-__global__ void __launch_bounds__(kThreads) mergeKernel(const uint32_t* __restrict__ a_keys,
-                                                         const uint32_t* __restrict__ a_idx,
-                                                         const uint32_t* __restrict__ b_keys,
-                                                         const uint32_t* __restrict__ b_idx, uint32_t n,
-                                                         const uint32_t* __restrict__ m_dev,
-                                                         const uint32_t* __restrict__ split,
-                                                         uint32_t* __restrict__ out_keys,
-                                                         uint32_t* __restrict__ out_perm) {
-    __shared__ unsigned long long sa[kMergeTile], sb[kMergeTile];
-    __shared__ uint32_t ok[kMergeTile], op[kMergeTile];
-    const uint32_t d0 = blockIdx.x * kMergeTile;
-    if (d0 >= n) return;
-    const uint32_t d1 = min(n, d0 + (uint32_t)kMergeTile);
-    const uint32_t a0 = split[blockIdx.x], a1 = split[blockIdx.x + 1];
-    const uint32_t b0 = d0 - a0, b1 = d1 - a1;
-    const uint32_t la = a1 - a0, lb = b1 - b0;  // la + lb = d1 - d0 <= kMergeTile
-    for (uint32_t i = threadIdx.x; i < la; i += kThreads) sa[i] = composite(a_keys[a0 + i], a_idx[a0 + i]);
-    for (uint32_t i = threadIdx.x; i < lb; i += kThreads) sb[i] = composite(b_keys[b0 + i], b_idx[b0 + i]);
-    __syncthreads();
-    const uint32_t dl = threadIdx.x * kMergeItems;
-    if (dl < la + lb) {
-        uint32_t lo = dl > lb ? dl - lb : 0u, hi = dl < la ? dl : la;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (sa[mid] < sb[dl - 1 - mid]) lo = mid + 1;
-            else hi = mid;
-        }
-        uint32_t ia = lo, ib = dl - lo;
-        const uint32_t dend = min(dl + (uint32_t)kMergeItems, la + lb);
-        for (uint32_t dd = dl; dd < dend; ++dd) {
-            const bool takeA = ib >= lb || (ia < la && sa[ia] < sb[ib]);
-            const unsigned long long v = takeA ? sa[ia++] : sb[ib++];
-            ok[dd] = (uint32_t)(v >> 32);
-            op[dd] = (uint32_t)v;
+// A group of NW warps (a whole CTA, or one warp) that puts blocks together.
+template <int NW>
+struct BlockSorter {
+    static constexpr int N = NW * 32;
+    static constexpr uint32_t kCap = NW == 1 ? 192 : NW == 32 ? 8192 : 4096;  // arrivals sorted in shared memory; more in aux
+    struct Smem {
+        unsigned long long arr[kCap];
+        uint32_t cnt[NW][64];  // own particles per warp and cell, then their first positions
+        uint32_t arrLo[64], arrHi[64], own[64], ownBelow[64], cellStart[64];
+        uint32_t nbStart[27], nbOff[28], narr, stayed, wsum[NW];
+    };
+    Smem& m;
+    const BlockSortArgs& s;
+    int t, lane, warp;  // thread and warp within the group
+    __device__ __forceinline__ BlockSorter(Smem& m_, const BlockSortArgs& s_, int t_)
+        : m(m_), s(s_), t(t_), lane(t_ & 31), warp(t_ >> 5) {}
+    __device__ __forceinline__ void sync() const {
+        if (NW == 1) __syncwarp();
+        else __syncthreads();
+    }
+
+    // Ascending sort of a[0..n): bitonic network in the form whose comparators
+    // all point the same way, so that elements past n act as infinity.
+    __device__ __forceinline__ void sort(unsigned long long* a, uint32_t n) const {
+        for (uint32_t k = 2; k / 2 < n; k <<= 1) {
+            for (uint32_t j = k; j > 1; j >>= 1) {
+                const uint32_t half = j >> 1;
+                for (uint32_t p = t;; p += N) {
+                    const uint32_t o = p & (half - 1), b = (p / half) * j;
+                    const uint32_t l = b + o, r = j == k ? b + k - 1 - o : l + half;
+                    if (l >= n) break;
+                    if (r < n) {
+                        const unsigned long long x = a[l], y = a[r];
+                        if (x > y) {
+                            a[l] = y;
+                            a[r] = x;
+                        }
+                    }
+                }
+                sync();
+            }
         }
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < la + lb; i += kThreads) {
-        out_keys[d0 + i] = ok[i];
-        out_perm[d0 + i] = op[i];
+
+    // The keys of particles [i, i + 128) of the warp's part [w0, w1) that stayed,
+    // as cells (64: not this block's); f(live index, cell, key) for each 32.
+    template <class Fn>
+    __device__ __forceinline__ void forOwn(uint2 prev, uint32_t w0, uint32_t w1, uint32_t blk, Fn&& f) const {
+        for (uint32_t i = w0; i < w1; i += 128) {
+            uint32_t key[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                key[j] = i + 32 * j + lane < w1 ? s.keys[prev.x + i + 32 * j + lane] : 0xffffffffu;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (i + 32 * j >= w1) break;
+                const bool mine = i + 32 * j + lane < w1 && (key[j] >> 6) == blk;
+                f(prev.x + i + 32 * j + lane, mine ? key[j] & 63u : 64u, key[j]);
+            }
+        }
     }
-    (void)m_dev;
+
+    __device__ __forceinline__ void run(const BlockItem& it, uint2 prev, uint32_t nfar) const {
+        const SceneDev& sc = s.scenes[it.scene];
+        const uint32_t blk = it.block, lt = (1u << lane) - 1u;
+        const bool outside = blk == sc.block_base + sc.nblocks;
+        for (int q = t; q < NW * 64; q += N) (&m.cnt[0][0])[q] = 0u;
+        for (int q = t; q < 64; q += N) m.arrLo[q] = m.arrHi[q] = 0u;
+        if (t == 0) m.narr = 0u;
+        if (warp == NW - 1) {
+            // the neighbouring blocks' emigrant lists
+            uint32_t c = 0, start = 0;
+            if (lane < 27 && lane != 13 && !outside) {
+                const uint32_t lb = blk - sc.block_base;
+                const int x = (int)(lb % (uint32_t)sc.nb[0]) + lane % 3 - 1;
+                const int y = (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]) + (lane / 3) % 3 - 1;
+                const int z = (int)(lb / ((uint32_t)sc.nb[0] * (uint32_t)sc.nb[1])) + lane / 9 - 1;
+                if (x >= 0 && y >= 0 && z >= 0 && x < sc.nb[0] && y < sc.nb[1] && z < sc.nb[2]) {
+                    const uint32_t nb = sc.block_base + (uint32_t)((z * sc.nb[1] + y) * sc.nb[0] + x);
+                    c = s.emig_count[nb];
+                    start = s.prev_range[nb].x;
+                }
+            }
+            uint32_t inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane < 27) {
+                m.nbStart[lane] = start;
+                m.nbOff[lane + 1] = inc;
+            }
+            if (lane == 0) m.nbOff[0] = 0u;
+        }
+        sync();
+        // ---- own particles: each warp a part of the block's previous range ----
+        const uint32_t per = ((prev.y + N - 1) / N) * 32;
+        const uint32_t w0 = min(prev.y, warp * per), w1 = min(prev.y, w0 + per);
+        forOwn(prev, w0, w1, blk, [&](uint32_t, uint32_t c, uint32_t) {
+            const uint32_t peers = __match_any_sync(0xffffffffu, c);
+            if (c < 64u && lane == __ffs(peers) - 1) m.cnt[warp][c] += (uint32_t)__popc(peers);
+            __syncwarp();
+        });
+        sync();
+        if (warp == 0) {  // cells 2 lane and 2 lane + 1
+            uint32_t tot[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t run = 0;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    const uint32_t c = m.cnt[w][2 * lane + h];
+                    m.cnt[w][2 * lane + h] = run;
+                    run += c;
+                }
+                m.own[2 * lane + h] = tot[h] = run;
+            }
+            uint32_t inc = tot[0] + tot[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            m.ownBelow[2 * lane] = inc - tot[0] - tot[1];
+            m.ownBelow[2 * lane + 1] = inc - tot[1];
+            if (lane == 31) m.stayed = inc;
+        }
+        sync();
+        const uint32_t stayed = m.stayed;
+        const uint32_t A = it.count >= stayed ? it.count - stayed : 0u;
+        uint32_t na = 0;
+        unsigned long long* arr = A <= kCap ? m.arr : s.aux + it.start;
+        if (A || it.count < stayed) {
+            // ---- arrivals ----
+            auto add = [&](uint32_t slot, uint2 e) {
+                if (slot < A) arr[slot] = ((unsigned long long)(e.y & 63u) << 32) | e.x;
+            };
+            const bool ordered = nfar > kBsFarScan;
+            if (ordered) {
+                // many far movers: every particle of the scene, in live order
+                const uint32_t n_round = (sc.n + N - 1) / N * N;
+                uint32_t found = 0;
+                for (uint32_t i = t; i < n_round && found < A; i += N) {
+                    const uint32_t g = sc.key_offset + i;
+                    const uint32_t key = i < sc.n ? s.keys[g] : 0xffffffffu;
+                    const bool hit = i < sc.n && (key >> 6) == blk && g - prev.x >= prev.y;
+                    const unsigned b = __ballot_sync(0xffffffffu, hit);
+                    if (lane == 0) m.wsum[warp] = (uint32_t)__popc(b);
+                    sync();
+                    uint32_t before = 0, all = 0;
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) {
+                        before += w < warp ? m.wsum[w] : 0u;
+                        all += m.wsum[w];
+                    }
+                    if (hit) add(found + before + __popc(b & lt), make_uint2(g, key));
+                    found += all;
+                    sync();
+                }
+                if (t == 0) m.narr = found;
+            } else {
+                const uint32_t E = m.nbOff[27], F = E + nfar;
+                for (uint32_t e = t; e < F; e += N) {
+                    uint2 v;
+                    if (e < E) {
+                        int q = 0;
+#pragma unroll
+                        for (int h = 16; h > 0; h >>= 1)
+                            if (q + h < 27 && m.nbOff[q + h] <= e) q += h;
+                        v = s.emig[m.nbStart[q] + (e - m.nbOff[q])];
+                    } else {
+                        v = s.far[e - E];
+                    }
+                    if ((v.y >> 6) == blk) add(atomicAdd(&m.narr, 1u), v);
+                }
+            }
+            sync();
+            if (t == 0 && (m.narr != A || it.count < stayed)) atomicOr(s.err, ERR_INDEX);  // never expected
+            na = min(m.narr, A);
+            if (!(ordered && outside)) sort(arr, na);  // (the outside block has one cell)
+            for (uint32_t q = t; q < na; q += N) {
+                const uint32_t c = (uint32_t)(arr[q] >> 32), g = (uint32_t)arr[q];
+                atomicAdd(g < prev.x ? &m.arrLo[c] : &m.arrHi[c], 1u);
+            }
+            sync();
+        }
+        if (warp == 0) {
+            const uint32_t a0 = m.arrLo[2 * lane] + m.arrHi[2 * lane];
+            const uint32_t a1 = m.arrLo[2 * lane + 1] + m.arrHi[2 * lane + 1];
+            uint32_t inc = a0 + a1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            m.cellStart[2 * lane] = m.ownBelow[2 * lane] + inc - a0 - a1;
+            m.cellStart[2 * lane + 1] = m.ownBelow[2 * lane + 1] + inc - a1;
+        }
+        sync();
+        // ---- positions ----
+        auto put = [&](uint32_t pos, uint32_t key, uint32_t g) {
+            if (pos >= it.count) return;  // never expected
+            s.out_keys[it.start + pos] = key;
+            s.out_perm[it.start + pos] = g;
+        };
+        // the q-th arrival of all is the r-th of its cell
+        for (uint32_t q = t; q < na; q += N) {
+            const uint32_t c = (uint32_t)(arr[q] >> 32), g = (uint32_t)arr[q];
+            const uint32_t r = q - (m.cellStart[c] - m.ownBelow[c]);
+            put(m.cellStart[c] + r + (r < m.arrLo[c] ? 0u : m.own[c]), (blk << 6) | c, g);
+        }
+        forOwn(prev, w0, w1, blk, [&](uint32_t g, uint32_t c, uint32_t key) {
+            const uint32_t peers = __match_any_sync(0xffffffffu, c);
+            uint32_t before = 0;
+            if (c < 64u) before = m.cnt[warp][c];
+            __syncwarp();
+            if (c < 64u) {
+                put(m.cellStart[c] + m.arrLo[c] + before + __popc(peers & lt), key, g);
+                if (lane == __ffs(peers) - 1) m.cnt[warp][c] = before + (uint32_t)__popc(peers);
+            }
+            __syncwarp();
+        });
+        sync();
+    }
+};
+
+constexpr size_t kBsSmem = std::max(sizeof(BlockSorter<kBsWarps>::Smem), kBsWarps * sizeof(BlockSorter<1>::Smem));
+constexpr size_t kBsDenseSmem = sizeof(BlockSorter<32>::Smem);
+
+__global__ void __launch_bounds__(kBsThreads) blockSortKernel(BlockSortArgs s) {
+    extern __shared__ unsigned long long bs_smem[];
+    __shared__ uint32_t item_s;
+    const uint32_t nfront = s.counters[kSortFrontWord], nback = s.counters[kSortBackWord];
+    const uint32_t nfar = *s.far_count;
+    // few small blocks: by CTAs as well, whose latency is a third of a warp's
+    const bool all = nback <= 2 * gridDim.x;
+    const uint32_t ncta = nfront + (all ? nback : 0u);
+    {
+        auto& m = *reinterpret_cast<BlockSorter<kBsWarps>::Smem*>(bs_smem);
+        const BlockSorter<kBsWarps> g(m, s, threadIdx.x);
+        const bool fixed = ncta <= gridDim.x;  // at most one each: no scheduler
+        for (uint32_t wi = blockIdx.x;;) {
+            if (!fixed) wi = nextWorkItem(s.counters + kSortSchedWord, ncta, &item_s);
+            if (wi >= ncta) break;
+            const BlockItem it = s.list[wi < nfront ? wi : s.list_cap - 1 - (wi - nfront)];
+            g.run(it, s.prev_range[it.block], nfar);
+            if (fixed) break;
+        }
+    }
+    if (all) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    auto& m = reinterpret_cast<BlockSorter<1>::Smem*>(bs_smem)[warp];
+    const BlockSorter<1> g(m, s, lane);
+    uint32_t* sched = s.counters + kSortSchedWord + 2;
+    for (;;) {
+        uint32_t wi = 0;
+        if (lane == 0) {
+            wi = atomicAdd(&sched[0], 1u);
+            if (wi >= nback && atomicAdd(&sched[1], 1u) == gridDim.x * kBsWarps - 1) {
+                sched[0] = 0u;
+                sched[1] = 0u;
+            }
+        }
+        wi = __shfl_sync(0xffffffffu, wi, 0);
+        if (wi >= nback) return;
+        const BlockItem it = s.list[s.list_cap - 1 - wi];
+        g.run(it, s.prev_range[it.block], nfar);
+    }
+}
+
+// Blocks of at least kDenseBlock particles, by CTAs of 1024 threads.
+__global__ void __launch_bounds__(1024) blockSortDenseKernel(BlockSortArgs s) {
+    extern __shared__ unsigned long long bs_smem[];
+    __shared__ uint32_t item_s;
+    const uint32_t ndense = s.counters[kSortDenseWord];
+    if (ndense == 0) return;
+    const uint32_t nfar = *s.far_count;
+    auto& m = *reinterpret_cast<BlockSorter<32>::Smem*>(bs_smem);
+    const BlockSorter<32> g(m, s, threadIdx.x);
+    for (;;) {
+        const uint32_t wi = nextWorkItem(s.counters + kSortSchedWord + 4, ndense, &item_s);
+        if (wi >= ndense) return;
+        const BlockItem it = s.dense[wi];
+        g.run(it, s.prev_range[it.block], nfar);
+    }
 }
 
 }  // namespace
 
-// Scratch layout (u32 words): a_keys, a_idx, b_keys, b_idx, b_keys2, b_idx2
-// (n each), mover count, partition tile counter and status words, merge
-// split points, then the movers' radix-sort scratch.
-static size_t partitionTiles(size_t n) { return (n + kPartTile - 1) / kPartTile; }
-static size_t mergeSplits(size_t n) { return (n + kMergeTile - 1) / kMergeTile + 1; }
-
-size_t incrementalSortScratchWords(size_t n, int bits) {
-    return 6 * n + 2 + partitionTiles(n) + mergeSplits(n) + onesweepScratchWords(n, bits) + 64;
+cudaError_t launchEmigrants(const BlockSortArgs& a, size_t n, int num_sms, cudaStream_t st) {
+    noteLaunches(1);
+    const unsigned grid = (unsigned)std::min<size_t>((n + kBsThreads * 4 - 1) / (kBsThreads * 4), (size_t)num_sms * 8);
+    emigrantKernel<<<std::max(1u, grid), kBsThreads, 0, st>>>(a, (uint32_t)n);
+    return cudaGetLastError();
 }
 
-cudaError_t incrementalSort(const uint32_t* keys, const uint32_t* prev, size_t n, int bits, uint32_t* out_keys,
-                            uint32_t* out_perm, uint32_t* scratch, uint32_t* err, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    if (n > kCountMask) return cudaErrorInvalidValue;
-    uint32_t* a_keys = scratch;
-    uint32_t* a_idx = a_keys + n;
-    uint32_t* b_keys = a_idx + n;
-    uint32_t* b_idx = b_keys + n;
-    uint32_t* b_keys2 = b_idx + n;
-    uint32_t* b_idx2 = b_keys2 + n;
-    uint32_t* m_dev = b_idx2 + n;
-    uint32_t* tile_counter = m_dev + 1;
-    uint32_t* status = tile_counter + 1;
-    const size_t ptiles = partitionTiles(n);
-    uint32_t* split = status + ptiles;
-    const size_t nsplit = mergeSplits(n);
-    uint32_t* sort_scratch = split + nsplit;
-    {
-        ClearRanges cr;
-        cr.p[0] = m_dev;
-        cr.n[0] = 2 + ptiles;
-        launchClear(cr, st);
+cudaError_t launchBlockSort(const BlockSortArgs& a, unsigned max_blocks, bool dense, int num_sms, cudaStream_t st) {
+    static_assert(kBsSmem <= 47 * 1024, "dynamic shared memory without an attribute");
+    noteLaunches(1);
+    if (dense) {
+        const cudaError_t e = cudaFuncSetAttribute(blockSortDenseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)kBsDenseSmem);
+        if (e != cudaSuccess) return e;
+        blockSortDenseKernel<<<std::max(1u, std::min(max_blocks, (unsigned)num_sms)), 1024, kBsDenseSmem, st>>>(a);
+    } else {
+        blockSortKernel<<<std::max(1u, std::min(max_blocks, (unsigned)num_sms * 5u)), kBsThreads, kBsSmem, st>>>(a);
     }
-    cudaError_t e = cudaSuccess;
-    noteLaunches(3);
-    moverPartitionKernel<<<(unsigned)ptiles, kThreads, 0, st>>>(keys, prev, (uint32_t)n, a_keys, a_idx, b_keys, b_idx,
-                                                                m_dev, tile_counter, status, (uint32_t)ptiles, err);
-    bool inB = false;
-    e = radixSortOnesweep(b_keys, b_idx, b_keys2, b_idx2, n, bits, sort_scratch, err, &inB, st, m_dev);
-    if (e != cudaSuccess) return e;
-    const uint32_t* mk = inB ? b_keys2 : b_keys;
-    const uint32_t* mi = inB ? b_idx2 : b_idx;
-    mergeSplitKernel<<<(unsigned)((nsplit + kThreads - 1) / kThreads), kThreads, 0, st>>>(
-        a_keys, a_idx, mk, mi, (uint32_t)n, m_dev, split, (uint32_t)nsplit);
-    mergeKernel<<<(unsigned)(nsplit - 1), kThreads, 0, st>>>(a_keys, a_idx, mk, mi, (uint32_t)n, m_dev, split, out_keys,
-                                                             out_perm);
     return cudaGetLastError();
 }
 
