@@ -46,7 +46,9 @@ __device__ __forceinline__ void cpAsync4(float* smem_dst, const float* gsrc) {
 __device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cpAsyncWaitAll() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-constexpr int kPreStride = 19;  // odd: rows of consecutive threads fall in different banks
+// G2P's prefetch row of a thread (floats): Fe, Fp, V0, x, mass, pid, and v
+// (PIC-FLIP); odd, so that rows of consecutive threads fall in different banks.
+constexpr int kPreVol = 18, kPreX = 19, kPreMass = 22, kPrePid = 23, kPreV = 24, kPreStride = 27;
 
 
 __device__ __forceinline__ uint32_t outsideKey(const SceneDev& sc) { return (sc.block_base + sc.nblocks) << 6; }
@@ -1572,35 +1574,39 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
 // (S+3)^3 node tile of v* (and v) is staged in shared memory, then one thread
 // per particle.  Writes the particle to its sorted slot of the other buffer.
 // ---------------------------------------------------------------------------
-// The first loads of a particle's update, issued one particle ahead: the
-// permutation entry, x and v into registers, and Fe, Fp, V0 into the thread's
+// The loads of a particle's update, issued one particle ahead into the thread's
 // shared-memory row by cp.async (one commit group per particle, possibly
-// empty), so their latency overlaps the previous particle's update.
+// empty), so that their latency overlaps the previous particle's update; its
+// permutation entry and key, which they wait for, two ahead.  (Holding x and v
+// in registers instead, and reading mass and pid where they are stored, left
+// the loads of a permutation entry, of mass and of pid exposed in every
+// update.)
 struct G2PIn {
-    uint32_t old;
+    uint32_t old, cell;
     bool ok;
-    float x[3], v[3];
 };
-__device__ __forceinline__ G2PIn g2pFetch(const StepArgs& args, const SceneDev& sc, uint32_t gs, float* pre) {
+template <bool APIC>
+__device__ __forceinline__ G2PIn g2pFetch(const StepArgs& args, const SceneDev& sc, uint32_t gs, uint32_t perm,
+                                          uint32_t key, float* pre) {
     G2PIn p;
-    const float* pf = sc.buf[args.parity].f;
     const size_t cap = sc.cap;
-    const uint32_t old = args.perm[gs] - sc.key_offset;
+    const uint32_t old = perm - sc.key_offset;
     const uint32_t dst = gs - sc.key_offset;
     p.ok = old < sc.n && dst < sc.n;  // range check: never expected, skip instead of faulting
     p.old = p.ok ? old : 0u;
+    p.cell = key & 63u;
     if (p.ok) {
+        const float* pf = sc.buf[args.parity].f + old;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            cpAsync4(pre + k, pf + (F_FE + k) * cap + old);
-            cpAsync4(pre + 9 + k, pf + (F_FP + k) * cap + old);
-        }
-        cpAsync4(pre + 18, pf + F_VOL * cap + old);
+        for (int a = 0; a < 3; ++a) cpAsync4(pre + kPreX + a, pf + (F_X + a) * cap);
+        if (!APIC)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            p.x[a] = ldg(pf + (F_X + a) * cap + old);
-            p.v[a] = ldg(pf + (F_V + a) * cap + old);
-        }
+            for (int a = 0; a < 3; ++a) cpAsync4(pre + kPreV + a, pf + (F_V + a) * cap);
+#pragma unroll
+        for (int k = 0; k < 18; ++k) cpAsync4(pre + k, pf + (F_FE + k) * cap);  // Fe, Fp
+        cpAsync4(pre + kPreVol, pf + F_VOL * cap);
+        cpAsync4(pre + kPreMass, pf + F_MASS * cap);
+        cpAsync4(pre + kPrePid, reinterpret_cast<const float*>(sc.buf[args.parity].pid + old));
     } else {
         atomicOr(args.err, ERR_INDEX);
     }
@@ -1614,46 +1620,27 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
                                                bool next_pending, const float4* tvs, const float4* tvo, const int* t0,
                                                bool fused, float* pre, const MaterialDev& mat0) {
     constexpr int T = S + 3;
-    const float* pf = sc.buf[args.parity].f;
     float* nf = sc.buf[args.parity ^ 1].f;
     const size_t cap = sc.cap;
-    if (!in.ok) {
-        if (next_pending) cpAsyncWaitPrevious();
-        else cpAsyncWaitAll();
-        return;
-    }
+    if (next_pending) cpAsyncWaitPrevious();  // this particle's group; the next one's may still run
+    else cpAsyncWaitAll();
+    if (!in.ok) return;
     const uint32_t old = in.old;
     const uint32_t dst = gs - sc.key_offset;
     const float h = sc.h, dt = sc.dt;
-    float x[3], v[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        x[a] = in.x[a];
-        v[a] = in.v[a];
-    }
     float vpic[3] = {0.f, 0.f, 0.f}, dflip[3] = {0.f, 0.f, 0.f};
     float gv[9], K[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) gv[k] = K[k] = 0.f;
-    float delta[3] = {0.f, 0.f, 0.f};
-    int base[3];
-    bool in_tile = false;
     if (tvs) {
-        in_tile = stencilBase(sc, x, base);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) in_tile = in_tile && base[a] - t0[a] >= 0 && base[a] - t0[a] <= 3;
-        if (!in_tile) atomicOr(args.err, ERR_INDEX);  // key and position disagree: never expected
-    }
-    if (in_tile) {
+        // the stencil base comes from the cell, which the key was formed from
+        const int lo[3] = {(int)(in.cell & 3u), (int)((in.cell >> 2) & 3u), (int)(in.cell >> 4)};
         float w[3][S], dw[3][S];
-        int lo[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            lo[a] = base[a] - t0[a];
-            float gp0 = __fadd_rn(sc.origin[a], __fmul_rn(h, (float)base[a]));
-            delta[a] = x[a] - gp0;
+            float gp0 = __fadd_rn(sc.origin[a], __fmul_rn(h, (float)(t0[a] + lo[a])));
             float dk[S];
-            dk[0] = __fdiv_rn(delta[a], h);
+            dk[0] = quotient(pre[kPreX + a] - gp0, h, sc.inv_h);
 #pragma unroll
             for (int k = 1; k < S; ++k) dk[k] = dk[0] - (float)k;  // exact subtraction
             splineWeights<S>(dk, w[a], dw[a]);
@@ -1662,90 +1649,83 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
                 dw[a][k] *= sc.inv_h;
             }
         }
-        // Separable gather in packed FP32 pairs: the x and y components of
-        // every sum go through one __ffma2_rn (two exactly rounded FMAs, the
-        // same results as fmaf), z through fmaf.  Column j of grad v and of
-        // the APIC moment K is held as (row 0, row 1) pair + row 2.
-        float2 wp[S], dwp[S], wap[S];
-#pragma unroll
-        for (int a = 0; a < S; ++a) {
-            wp[a] = make_float2(w[0][a], w[0][a]);
-            dwp[a] = make_float2(dw[0][a], dw[0][a]);
-            const float wa = w[0][a] * (float)a;
-            wap[a] = make_float2(wa, wa);
-        }
-        float2 vp_xy = make_float2(0.f, 0.f), df_xy = make_float2(0.f, 0.f), gv_xy[3], K_xy[3];
-        float vp_z = 0.f, df_z = 0.f, gv_z[3], K_z[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            gv_xy[j] = K_xy[j] = make_float2(0.f, 0.f);
-            gv_z[j] = K_z[j] = 0.f;
-        }
+        // Separable gather, one axis after another: along x for every row (b,
+        // c) of the stencil, along y for every plane c, then along z.  In
+        // packed FP32 pairs: the x and y components of every sum go through
+        // one __ffma2_rn (two exactly rounded FMAs, the same results as
+        // fmaf), z through fmaf.  Sums of v* with the weights N_x N_y N_z (the
+        // velocity), N'_x N_y N_z and so on (the columns of grad v), a N_x N_y
+        // N_z and so on (those of the APIC moment K); PIC-FLIP's of v* - v.
+        // Instruction issue and load latency bound the kernel: summing the rows
+        // straight into the results took seven scaled additions a row (with
+        // the loads two particles ahead and the base from the cell: two-ball
+        // G2P 0.118 -> 0.106 ms and 62M -> 56M warp instructions, slab 1.14 ->
+        // 0.98 ms).
+        struct V3 {
+            float2 xy;
+            float z;
+        };
+        auto fma3 = [](float k, const V3& v, V3& sum) {
+            sum.xy = __ffma2_rn(make_float2(k, k), v.xy, sum.xy);
+            sum.z = fmaf(k, v.z, sum.z);
+        };
+        const V3 zero{make_float2(0.f, 0.f), 0.f};
+        V3 sv = zero, sg[3] = {zero, zero, zero}, sk[3] = {zero, zero, zero}, sf = zero;
 #pragma unroll
         for (int c = 0; c < S; ++c) {
+            // plane sums: y weight N_y of the rows' N_x, N'_x and a N_x (or
+            // v* - v) sums, and N'_y and b N_y of the first
+            V3 p0 = zero, pd = zero, p1 = zero, py = zero, pb = zero;
 #pragma unroll
             for (int b = 0; b < S; ++b) {
-                float2 r0 = make_float2(0.f, 0.f), r1 = r0, rd = r0, rv = r0;
-                float r0z = 0.f, r1z = 0.f, rdz = 0.f, rvz = 0.f;
+                V3 r0 = zero, rd = zero, r1 = zero;
                 const int rowbase = lo[0] + T * ((lo[1] + b) + T * (lo[2] + c));
 #pragma unroll
                 for (int a = 0; a < S; ++a) {
                     const float4 g = tvs[rowbase + a];
-                    const float2 gxy = make_float2(g.x, g.y);
-                    r0 = __ffma2_rn(wp[a], gxy, r0);
-                    r0z = fmaf(w[0][a], g.z, r0z);
-                    rd = __ffma2_rn(dwp[a], gxy, rd);
-                    rdz = fmaf(dw[0][a], g.z, rdz);
+                    const V3 gv3{make_float2(g.x, g.y), g.z};
+                    fma3(w[0][a], gv3, r0);
+                    fma3(dw[0][a], gv3, rd);
                     if (APIC) {
-                        r1 = __ffma2_rn(wap[a], gxy, r1);
-                        r1z = fmaf(wap[a].x, g.z, r1z);
+                        if (a) fma3(w[0][a] * (float)a, gv3, r1);
                     } else {
                         const float4 o = tvo[rowbase + a];
-                        const float2 d = __fadd2_rn(gxy, make_float2(-o.x, -o.y));  // g - o, exactly
-                        rv = __ffma2_rn(wp[a], d, rv);
-                        rvz = fmaf(w[0][a], g.z - o.z, rvz);
+                        const V3 d{__fadd2_rn(gv3.xy, make_float2(-o.x, -o.y)), g.z - o.z};  // g - o, exactly
+                        fma3(w[0][a], d, r1);
                     }
                 }
-                const float wyz = w[1][b] * w[2][c];
-                const float dy = dw[1][b] * w[2][c];
-                const float dz = w[1][b] * dw[2][c];
-                const float2 wyz2 = make_float2(wyz, wyz), dy2 = make_float2(dy, dy), dz2 = make_float2(dz, dz);
-                vp_xy = __ffma2_rn(wyz2, r0, vp_xy);
-                vp_z = fmaf(wyz, r0z, vp_z);
-                gv_xy[0] = __ffma2_rn(wyz2, rd, gv_xy[0]);
-                gv_z[0] = fmaf(wyz, rdz, gv_z[0]);
-                gv_xy[1] = __ffma2_rn(dy2, r0, gv_xy[1]);
-                gv_z[1] = fmaf(dy, r0z, gv_z[1]);
-                gv_xy[2] = __ffma2_rn(dz2, r0, gv_xy[2]);
-                gv_z[2] = fmaf(dz, r0z, gv_z[2]);
-                if (APIC) {
-                    const float wb = wyz * (float)b, wc = wyz * (float)c;
-                    K_xy[0] = __ffma2_rn(wyz2, r1, K_xy[0]);
-                    K_z[0] = fmaf(wyz, r1z, K_z[0]);
-                    K_xy[1] = __ffma2_rn(make_float2(wb, wb), r0, K_xy[1]);
-                    K_z[1] = fmaf(wb, r0z, K_z[1]);
-                    K_xy[2] = __ffma2_rn(make_float2(wc, wc), r0, K_xy[2]);
-                    K_z[2] = fmaf(wc, r0z, K_z[2]);
-                } else {
-                    df_xy = __ffma2_rn(wyz2, rv, df_xy);
-                    df_z = fmaf(wyz, rvz, df_z);
-                }
+                fma3(w[1][b], r0, p0);
+                fma3(w[1][b], rd, pd);
+                fma3(w[1][b], r1, p1);
+                fma3(dw[1][b], r0, py);
+                if (APIC && b) fma3(w[1][b] * (float)b, r0, pb);
+            }
+            fma3(w[2][c], p0, sv);
+            fma3(w[2][c], pd, sg[0]);
+            fma3(w[2][c], py, sg[1]);
+            fma3(dw[2][c], p0, sg[2]);
+            if (APIC) {
+                fma3(w[2][c], p1, sk[0]);
+                fma3(w[2][c], pb, sk[1]);
+                if (c) fma3(w[2][c] * (float)c, p0, sk[2]);
+            } else {
+                fma3(w[2][c], p1, sf);
             }
         }
-        vpic[0] = vp_xy.x;
-        vpic[1] = vp_xy.y;
-        vpic[2] = vp_z;
-        dflip[0] = df_xy.x;
-        dflip[1] = df_xy.y;
-        dflip[2] = df_z;
+        vpic[0] = sv.xy.x;
+        vpic[1] = sv.xy.y;
+        vpic[2] = sv.z;
+        dflip[0] = sf.xy.x;
+        dflip[1] = sf.xy.y;
+        dflip[2] = sf.z;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            gv[0 * 3 + j] = gv_xy[j].x;
-            gv[1 * 3 + j] = gv_xy[j].y;
-            gv[2 * 3 + j] = gv_z[j];
-            K[0 * 3 + j] = K_xy[j].x;
-            K[1 * 3 + j] = K_xy[j].y;
-            K[2 * 3 + j] = K_z[j];
+            gv[0 * 3 + j] = sg[j].xy.x;
+            gv[1 * 3 + j] = sg[j].xy.y;
+            gv[2 * 3 + j] = sg[j].z;
+            K[0 * 3 + j] = sk[j].xy.x;
+            K[1 * 3 + j] = sk[j].xy.y;
+            K[2 * 3 + j] = sk[j].z;
         }
     }
     // New velocity (src/mpm_solver3d.cu:362-363; apic :366-374).
@@ -1756,12 +1736,10 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
     } else {
         const float al = sc.blend, om = 1.0f - sc.blend;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) vn[i] = al * (v[i] + dflip[i]) + om * vpic[i];
+        for (int i = 0; i < 3; ++i) vn[i] = al * (pre[kPreV + i] + dflip[i]) + om * vpic[i];
     }
     // Fe <- (I + dt grad v) Fe ; F = Fe Fp ; SVD clamp (src/material_point3d.cu:53-70).
     float Fe[9], Fp[9], A[9], Fn[9];
-    if (next_pending) cpAsyncWaitPrevious();  // this particle's group; the next one's may still run
-    else cpAsyncWaitAll();
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         Fe[k] = pre[k];
@@ -1772,7 +1750,7 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
     const uint16_t mid = sc.nmat > 1 ? sc.buf[args.parity].mat[old] : (uint16_t)0;
     const MaterialDev m = sc.nmat > 1 ? sc.mats[mid] : mat0;
     const float hi = 1.0f + m.theta_s, lo = 1.0f - m.theta_c;
-    const float V0 = pre[18];
+    const float V0 = pre[kPreVol];
     float mu, la, tau[6];
     // Elastic fast path: no singular value can be clamped, so Fe = Fn and Fp
     // stay as they are, and the stress comes from the polar rotation of Fn
@@ -1859,6 +1837,15 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
     }
     tauFromSvd(m.model, U, s, mu, la, V0, tau);
     }
+    // the position, read again (held in registers across the update it would
+    // spill others)
+    float x[3], delta[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        x[a] = *(volatile const float*)(pre + kPreX + a);
+        const int lo = (int)((in.cell >> (2 * a)) & 3u);
+        delta[a] = tvs ? x[a] - __fadd_rn(sc.origin[a], __fmul_rn(h, (float)(t0[a] + lo))) : 0.f;
+    }
     if (fused) {
         if (sc.pcoll) {  // particlesCollision (src/mpm_solver3d.cu:428-445)
             float pos[3];
@@ -1900,9 +1887,9 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
     }
 #pragma unroll
     for (int k = 0; k < 6; ++k) nf[(F_TAU + k) * cap + dst] = tau[k];
-    nf[F_MASS * cap + dst] = ldg(pf + F_MASS * cap + old);
+    nf[F_MASS * cap + dst] = pre[kPreMass];
     nf[F_VOL * cap + dst] = V0;
-    sc.buf[args.parity ^ 1].pid[dst] = sc.buf[args.parity].pid[old];
+    sc.buf[args.parity ^ 1].pid[dst] = __float_as_uint(pre[kPrePid]);
     if (sc.nmat > 1) sc.buf[args.parity ^ 1].mat[dst] = mid;
 }
 
@@ -2114,11 +2101,26 @@ __global__ void __launch_bounds__(kG2PThreads, MPM_G2P_MIN_CTAS) g2pKernel(StepA
             // each thread's particles of the item, the next one's loads in
             // flight during the current one's update (rows alternate)
             int row = 0;
-            G2PIn cur = g2pFetch(args, sc, it.start + threadIdx.x, &pre[0][threadIdx.x * kPreStride]);
-            for (uint32_t i = threadIdx.x; i < it.count; i += kG2PThreads) {
+            const uint32_t* perm = args.perm + it.start;
+            const uint32_t* keys = args.sorted_keys + it.start;
+            uint32_t i = threadIdx.x;
+            uint32_t np = 0, nk = 0;  // permutation entry and key of the particle to fetch next
+            if (i + kG2PThreads < it.count) {
+                np = perm[i + kG2PThreads];
+                nk = keys[i + kG2PThreads];
+            }
+            G2PIn cur = g2pFetch<APIC>(args, sc, it.start + i, perm[i], keys[i], &pre[0][threadIdx.x * kPreStride]);
+            for (; i < it.count; i += kG2PThreads) {
                 const bool more = i + kG2PThreads < it.count;
                 G2PIn nxt;
-                if (more) nxt = g2pFetch(args, sc, it.start + i + kG2PThreads, &pre[row ^ 1][threadIdx.x * kPreStride]);
+                if (more) {
+                    nxt = g2pFetch<APIC>(args, sc, it.start + i + kG2PThreads, np, nk,
+                                         &pre[row ^ 1][threadIdx.x * kPreStride]);
+                    if (i + 2 * kG2PThreads < it.count) {
+                        np = perm[i + 2 * kG2PThreads];
+                        nk = keys[i + 2 * kG2PThreads];
+                    }
+                }
                 particleUpdate<S, APIC>(args, sc, it.start + i, cur, more, inside ? &tvs[b][0] : nullptr,
                                         APIC ? nullptr : &tvo[b][0], t0, fused != 0,
                                         &pre[row][threadIdx.x * kPreStride], mat0[b]);
@@ -2495,7 +2497,7 @@ static void g2pLaunch(const LaunchCtx& c, const StepArgs& a, int fused) {
         return true;
     }();
     (void)attr;
-    g2pKernel<S, APIC><<<c.persistent_blocks * (256 / kG2PThreads), kG2PThreads, kG2PDynSmem, c.stream>>>(a, fused);
+    g2pKernel<S, APIC><<<(c.persistent_blocks * 256 + kG2PThreads - 1) / kG2PThreads, kG2PThreads, kG2PDynSmem, c.stream>>>(a, fused);
 }
 
 void launchG2P(const LaunchCtx& c, const StepArgs& args, int S, bool apic, bool fused, int combo) {
