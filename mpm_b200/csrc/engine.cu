@@ -227,7 +227,7 @@ struct SceneHost {
     // semi-implicit update (beta > 0) and its solver buffers (implicit.cu)
     float beta = 0.f, solve_tol = 1e-5f;
     int solve_max_iter = 50;
-    DevMem solve_m, solve_vec, solve_list, solve_part, solve_status;
+    DevMem solve_m, solve_vec, solve_part, solve_status;
     size_t nodes() const { return (size_t)desc.resolution[0] * desc.resolution[1] * desc.resolution[2]; }
     ~SceneHost() {
         for (int k = 0; k < 2; ++k) {
@@ -394,7 +394,7 @@ public:
     // Returns the engine's own buffers to the pool in the stream's order
     // (called before the stream is destroyed).
     void releaseScratch() {
-        DevMem* all[] = {&cell_range_, &block_range_, &solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
+        DevMem* all[] = {&solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
                          &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &range_[0], &range_[1], &emig_count_[0], &emig_count_[1], &emig_, &far_, &arrivals_, &far_count_, &sort_list_, &dense_list_,
                          &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_, &tile_done_,
                          &tiles_, &scenes_dev_, &err_, &tmp_, &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
@@ -1049,19 +1049,17 @@ public:
         d.beta = s.beta;
         d.solve_tol = s.solve_tol;
         d.solve_max_iter = s.solve_max_iter;
-        d.solve = SolveDev{s.solve_m.as<float>(), s.solve_vec.as<float4>(), s.solve_list.as<int>(),
+        d.solve = SolveDev{s.solve_m.as<float>(), s.solve_vec.as<float4>(),
                            s.solve_part.as<double>(), s.solve_status.as<SolveStatus>()};
     }
     // Batch-wide buffers over the sorted particles and the cell keys.
     mpm_status ensureSolveBuffers() {
         if (!any_implicit_ || dirty_) return MPM_OK;
         const size_t n = std::max<size_t>(ntot_, 1);
-        MPM_TRY(grow(cell_range_, sizeof(uint2) * (size_t)total_blocks_ * 64, "solver cell ranges"));
-        MPM_TRY(grow(block_range_, sizeof(uint2) * (size_t)total_blocks_, "solver block ranges"));
         MPM_TRY(grow(solve_pofs_, sizeof(float4) * n, "solver stencil offsets"));
         MPM_TRY(grow(solve_prep_, sizeof(float) * kSolvePrepPlanes * n, "solver particle data"));
         MPM_TRY(grow(solve_T_, sizeof(float4) * 3 * n, "solver particle stress differentials"));
-        MPM_TRY(grow(solve_iter_, sizeof(int), "solver iteration counter"));
+        MPM_TRY(grow(solve_iter_, 2 * sizeof(int), "solver iteration counter"));
         MPM_TRY(ensureSideStreams(1));  // the loop body of a captured solve is captured on side_[0]
         return MPM_OK;
     }
@@ -1080,7 +1078,6 @@ public:
             const size_t nodes = s.nodes();
             MPM_TRY(grow(s.solve_m, sizeof(float) * nodes, "solver node masses"));
             MPM_TRY(grow(s.solve_vec, sizeof(float4) * kSolveVectors * nodes, "solver node vectors"));
-            MPM_TRY(grow(s.solve_list, sizeof(int) * nodes, "solver node list"));
             MPM_TRY(grow(s.solve_part, sizeof(double) * solvePartialDoubles(max_iter), "solver partial sums"));
             MPM_TRY(grow(s.solve_status, sizeof(SolveStatus), "solver status"));
             CUDA_TRY(cudaMemset(s.solve_status.p, 0, sizeof(SolveStatus)));
@@ -1116,12 +1113,11 @@ public:
         return m;
     }
     mpm_status launchSolveAll(bool split) {
-        SolveBuffers b{keys_[sorted_].as<uint32_t>(), vals_[sorted_].as<uint32_t>(), cell_range_.as<uint2>(),
-                       (size_t)total_blocks_ * 64, block_range_.as<uint2>(), (size_t)total_blocks_,
-                       solve_pofs_.as<float4>(), solve_prep_.as<float>(), solve_T_.as<float4>(), (uint32_t)ntot_,
-                       solve_iter_.as<int>()};
+        SolveBuffers b{keys_[sorted_].as<uint32_t>(), vals_[sorted_].as<uint32_t>(), solve_pofs_.as<float4>(),
+                       solve_prep_.as<float>(), solve_T_.as<float4>(), (uint32_t)ntot_, solve_iter_.as<int>()};
+        const StepArgs step = args(keys_[sorted_].as<uint32_t>(), vals_[sorted_].as<uint32_t>(), nullptr);
         const std::vector<int> S = stencilSizes();
-        CUDA_TRY(launchSolve(ctx(), b, parity_, S.data(), (int)S.size(), maxSolveIters(), split, side_[0]));
+        CUDA_TRY(launchSolve(ctx(), step, b, parity_, S.data(), (int)S.size(), maxSolveIters(), split, side_[0]));
         return MPM_OK;
     }
     // Split API: solveLinearSystem(dt) on the split-mode grid (v* of
@@ -1184,6 +1180,8 @@ public:
         a.stats = counters_.as<uint32_t>();
         a.sched = counters_.as<uint32_t>() + 8;
         a.tmaps = tmaps_.as<unsigned char>();
+        a.solve_pofs = a.solve_T = nullptr;  // set by the semi-implicit solve
+        a.solve_iter = nullptr;
         a.spans = nullptr;  // set per combination by the step
         a.p2g_lists = nullptr;  // the step's P2G launches take their combination's lists
         a.p2g_list_cap = (uint32_t)max_active_;
@@ -1901,6 +1899,12 @@ public:
     // is the step captured as a CUDA graph (a change would drop it).
     mpm_status checkWarpItems() {
         if (!warp_check_) return MPM_OK;
+        if (any_implicit_ && !warp_pending_) {
+            // not worth waiting for: without a graph a step launches every
+            // iteration of the solve up to its limit
+            warp_check_ = false;
+            return MPM_OK;
+        }
         if (!warp_pending_) {
             if (!host_word_) {
                 host_word_ = g_pinned_words.take();
@@ -2474,7 +2478,7 @@ private:
     bool dirty_ = true, keys_valid_ = false, sorted_valid_ = false;
     bool any_cfl_ = false;     // some scene steps with a CFL dt (two more launches per step)
     bool any_implicit_ = false;  // some scene solves the semi-implicit update
-    DevMem cell_range_, block_range_, solve_pofs_, solve_prep_, solve_T_, solve_iter_;
+    DevMem solve_pofs_, solve_prep_, solve_T_, solve_iter_;
     uint32_t g2p_cap_ = 1;   // G2P items per combination (rebuild)
     // launch settings per (stencil, transfer) combination (mpm_tuning)
     std::map<std::pair<int, int>, mpm_tuning> tuning_;

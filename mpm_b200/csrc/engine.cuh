@@ -136,20 +136,17 @@ struct CflState {
     double time;
 };
 
-// Semi-implicit solve of one scene (see implicit.cu).  vec holds seven
-// dense node vectors of float4 (x, r, z, p, Ap, Az, h; .w unused); list the
-// nodes with mass; part the per-block FP64 partial sums of the dot
-// products, [quantity][slot][block].
+// Semi-implicit solve of one scene (see implicit.cu).  vec holds six dense
+// node vectors of float4 (x, r, z, p, Ap, Az; .w unused); part the per-block
+// FP64 partial sums of the dot products, [quantity][slot][block].
 struct SolveStatus {
     int done_at;     // first iteration whose test found convergence (INT_MAX while running)
     int iters;
     float residual;  // |r| / |M v*| at the end
-    int nactive;     // nodes in list
 };
 struct SolveDev {
     float* m;
     float4* vec;
-    int* list;
     double* part;
     SolveStatus* status;
 };
@@ -230,6 +227,11 @@ struct StepArgs {
     uint32_t p2g_list_cap;
     int p2g_warp;                // who takes list 0 (the small items): P2G_WARP_NONE, _ALWAYS or _AUTO
     const unsigned char* tmaps;  // kTensorMapBytes x 2 per scene (64-byte aligned): TMA maps of v*, v
+    // MODE_HESS: per sorted particle its stencil offsets and the rows of T; the
+    // solver's device iteration counter and its "all converged" flag (null:
+    // before the first iteration)
+    const float4 *solve_pofs, *solve_T;
+    const int* solve_iter;
     unsigned long long* spans;   // this combination's kernel time spans (see KernelSpan), or null
 };
 
@@ -287,11 +289,12 @@ enum P2GMode : int {
     MODE_APIC_FUSED = 0,  // fields: m, p + dt f        (F = 4)
     MODE_FLIP = 1,        // fields: m, p, f            (F = 7)
     MODE_SPLIT = 2,       // fields: m, p, f (any transfer, split API, F = 7)
-    MODE_MASS = 3         // fields: m                  (F = 1)
+    MODE_MASS = 3,        // fields: m                  (F = 1)
+    MODE_HESS = 4         // fields: f of the semi-implicit solver (P2G only, F = 3)
 };
 
 __host__ __device__ constexpr int modeFields(int mode) {
-    return mode == MODE_APIC_FUSED ? 4 : (mode == MODE_MASS ? 1 : 7);
+    return mode == MODE_APIC_FUSED ? 4 : (mode == MODE_MASS ? 1 : (mode == MODE_HESS ? 3 : 7));
 }
 __host__ __device__ constexpr int tileNodes(int S) { return (S + 3) * (S + 3) * (S + 3); }
 

@@ -133,10 +133,6 @@ void launchDensity(const LaunchCtx& c, const float4* vstar, size_t nodes, float 
 struct SolveBuffers {
     const uint32_t* sorted_keys;  // ntot
     const uint32_t* perm;         // ntot
-    uint2* cell_range;            // nkeys: first and end sorted position of each cell key
-    size_t nkeys;
-    uint2* block_range;           // nblocks: the same per 4^3 block of cells (key >> 6)
-    size_t nblocks;
     float4* pofs;                 // ntot: stencil offsets (x - (o + h base)) / h (sorted order)
     float* prep;                  // kSolvePrepPlanes x ntot
     float4* T;                    // 3 x ntot: V0 dP Fe^T rows
@@ -144,14 +140,15 @@ struct SolveBuffers {
     int* iter;                    // device iteration counter
 };
 constexpr int kSolvePrepPlanes = 44;
-constexpr int kSolveVectors = 7;
+constexpr int kSolveVectors = 6;
 constexpr int kSolveBlocks = 512;  // node-kernel blocks per scene = partial sums per dot product
 inline size_t solvePartialDoubles(int max_iter) { return (size_t)4 * (size_t)(max_iter + 2) * kSolveBlocks; }
 // split: v* from and to the split-mode dense planes (no collision after);
 // else from and to the fused step's v* grid, with the grid collision after.
 // aux: an idle stream on which, inside a stream capture, the iteration body
 // is captured as the body of a conditional while node.
-cudaError_t launchSolve(const LaunchCtx& c, const SolveBuffers& b, int parity, const int* stencils, int nstencils,
+// step: the arguments of the step's P2G (work items, tiles, schedulers).
+cudaError_t launchSolve(const LaunchCtx& c, const StepArgs& step, const SolveBuffers& b, int parity, const int* stencils, int nstencils,
                         int max_iter, bool split, cudaStream_t aux);
 
 // CFL time step of the scenes with cfl > 0: max |v|^2 over their live

@@ -8,28 +8,29 @@
 //     H u = sum_p V0 (dP/dF : (sum_j u_j grad w_jp^T) Fe) Fe^T grad w_ip,
 // and solved by conjugate residual preconditioned with the node masses.
 //
-//   cellRangeKernel    first and end sorted position of every cell key and
-//                      of every 4^3 block of cells
 //   solvePrepKernel    per sorted particle: Fe, its SVD, cofactor, J, ln J,
 //                      V0 mu and V0 la (hardened), model; the offsets
 //                      (x - (o + h base)) / h of its stencil
 //   solveInitKernel    node masses (the transfer's), x0 = v*, the other
-//                      vectors 0, |M v*|^2, list of the nodes with mass
-//   solveGatherKernel  per particle: G = sum_j u_j grad w^T, T = V0 dP(G Fe) Fe^T
-//   solveScatterKernel per listed node: h = sum_p T_p grad w_ip
+//                      vectors 0, |M v*|^2
+//   solveGatherKernel  per work item: the tile of u in shared memory, then per
+//                      particle G = sum_j u_j grad w^T, T = V0 dP(G Fe) Fe^T
+//   p2gKernel (MODE_HESS)  tiles of sum_p T_p grad w_ip, the transfer's scatter
 //   solveResidualKernel, solveAzKernel, solveUpdateKernel, solveDirKernel
-//                      the elementwise vector updates and dot products
+//                      the elementwise vector updates and dot products; the
+//                      first two merge a node's tiles into (H u)_i
 //   solveFinalKernel   v* = x (and the grid collision again in the fused step)
 //
-// A node's sum h is formed by one warp: the lanes share out the
-// particles of the S^3 cells around the node (flattened, in sorted order) and
-// the lane sums meet in a fixed shuffle tree, so a node's value does not
-// depend on which warp computes it.  Dot products come from the elementwise
-// kernels as per-block FP64 partials over a fixed node partition, which every
-// consumer block reduces in block order.  The solve is bitwise reproducible
-// and a scene's result does not depend on its batch-mates.  Convergence
-// (|r| <= tol |M v*|) is decided on the device; a scene that converged skips
-// the remaining launches of the step.
+// The scatter sums in the transfer's fixed order, so a node's value does not
+// depend on which CTA takes an item.  (It was one warp per node over the
+// particles of the S^3 cells around the node: every particle's weights formed
+// S^3 times.  120k particles, cubic, 17 a cell, per iteration: scatter 94 -> 
+// MEASURE us, gather from global memory 37 -> MEASURE.)  Dot products come from the
+// elementwise kernels as per-block FP64 partials over a fixed node partition,
+// which every consumer block reduces in block order.  The solve is bitwise
+// reproducible and a scene's result does not depend on its batch-mates.
+// Convergence (|r| <= tol |M v*|) is decided on the device; a scene that
+// converged skips the remaining launches of the step.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -44,9 +45,9 @@ namespace mpm {
 
 namespace {
 
-enum { VX = 0, VR = 1, VZ = 2, VP = 3, VAP = 4, VAZ = 5, VH = 6 };  // node vectors
+enum { VX = 0, VR = 1, VZ = 2, VP = 3, VAP = 4, VAZ = 5 };         // node vectors
 enum { QRR = 0, QZAZ = 1, QAPQ = 2, QBB = 3 };                      // dot products
-static_assert(VH + 1 == kSolveVectors, "node vector count");
+static_assert(VAZ + 1 == kSolveVectors, "node vector count");
 
 static_assert(kSolveBlocks == 2 * kThreads, "partials are reduced two per thread");
 
@@ -54,15 +55,19 @@ struct SolveArgs {
     const SceneDev* scenes;
     const uint32_t* sorted_keys;
     const uint32_t* perm;
-    const uint2* cell_range;
-    const uint2* block_range;
+    const BlockItem* items;     // G2P's work items, combination q's at items + q * items_cap,
+    uint32_t items_cap;         // counters[kG2PCountWord + q] of them
+    const uint32_t* counters;
+    const int2* block_slot;     // block -> (first tile slot or -1, items)
+    const float* tiles;
+    uint32_t tile_stride;
     float4* pofs;  // per sorted particle: stencil offsets d0 (xyz)
     float* prep;
     float4* T;
     uint32_t ntot;
     int parity;
     int split;
-    int* iter;  // device iteration counter of the loop
+    int* iter;  // [0] device iteration counter of the loop, [1] no scene iterates any more
 };
 
 // Prep planes (stride ntot): F 0..8, U 9..17, V 18..26, s 27..29, cof F
@@ -116,89 +121,32 @@ __device__ __forceinline__ void nodeCoords(const SceneDev& sc, size_t node, int*
 }
 __device__ __forceinline__ float3 ld3(const float4& v) { return make_float3(v.x, v.y, v.z); }
 
-// Weight and gradient of stencil node k of a particle with stencil offsets
-// d0 = (x - (o + h base)) / h (the distance is d0 - k, as in G2P).
-template <int S>
-__device__ __forceinline__ void nodeWeight(const SceneDev& sc, const float4& d0, const int* k, float* w, float* dw) {
-    const float d[3] = {d0.x - (float)k[0], d0.y - (float)k[1], d0.z - (float)k[2]};
+// (H u)_i at node n: the sum of the up to 8 tiles that overlap it, in the grid
+// pass's order (a block of the particles' cells covers S + 3 nodes an axis).
+__device__ __forceinline__ float3 tileSum(const SolveArgs& a, const SceneDev& sc, const int* n) {
+    const int T = sc.S + 3, TN = T * T * T;
+    const int N[3] = {(n[0] + 4) >> 2, (n[1] + 4) >> 2, (n[2] + 4) >> 2};
+    float3 h = make_float3(0.f, 0.f, 0.f);
+    int slot[8], at[8];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        w[a] = splineN<S>(d[a]);
-        dw[a] = splineNDot<S>(d[a]) * sc.inv_h;
-    }
-}
-// Stencil base of a particle from its cell key (key = block << 6 | cell,
-// base + 4 = 4 block + cell per axis).
-__device__ __forceinline__ void keyBase(const SceneDev& sc, uint32_t key, int* base) {
-    const uint32_t lb = (key >> 6) - sc.block_base, c = key & 63u;
-    base[0] = 4 * (int)(lb % (uint32_t)sc.nb[0]) - 4 + (int)(c & 3u);
-    base[1] = 4 * (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]) - 4 + (int)((c >> 2) & 3u);
-    base[2] = 4 * (int)(lb / ((uint32_t)sc.nb[0] * sc.nb[1])) - 4 + (int)(c >> 4);
-}
-
-// Sum fn(p, base, k) over the particles whose stencil covers node n, by one
-// warp: the S^3 base cells n - S + 1 .. n (always inside the key range) in a
-// fixed order, their particles in sorted order, flattened and dealt to the
-// lanes round-robin; the lane sums meet in a fixed shuffle tree.  Every lane
-// returns the total.  sh: this warp's 2 S^3 + 1 ints of shared memory.
-template <int S, int C, class Fn>
-__device__ __forceinline__ void warpNodeSum(const SceneDev& sc, const SolveArgs& a, const int* n, int* sh, float* out,
-                                            Fn&& fn) {
-    constexpr int NC = S * S * S;
-    const int lane = threadIdx.x & 31;
-    int* first = sh;       // NC
-    int* start = sh + NC;  // NC + 1: flattened offset of each cell
-    int cnt[2] = {0, 0};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int ci = lane + 32 * h;
-        if (ci < NC) {
-            const int c[3] = {ci % S, (ci / S) % S, ci / (S * S)};
-            const int base[3] = {n[0] - S + 1 + c[0], n[1] - S + 1 + c[1], n[2] - S + 1 + c[2]};
-            const uint2 rg = a.cell_range[makeKey(sc, base)];
-            first[ci] = (int)rg.x;
-            cnt[h] = (int)(rg.y - rg.x);
-        }
-    }
-    // exclusive offsets in cell order: cells lane and 32 + lane
-    int v0 = cnt[0], v1 = cnt[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t0 = __shfl_up_sync(0xffffffffu, v0, o), t1 = __shfl_up_sync(0xffffffffu, v1, o);
-        if (lane >= o) {
-            v0 += t0;
-            v1 += t1;
-        }
-    }
-    const int tot0 = __shfl_sync(0xffffffffu, v0, 31);
-    if (lane < NC) start[lane] = v0 - cnt[0];
-    if (32 + lane < NC) start[32 + lane] = tot0 + v1 - cnt[1];
-    const int total = tot0 + __shfl_sync(0xffffffffu, v1, 31);
-    if (lane == 0) start[NC] = total;
-    __syncwarp();
-    float acc[C];
-#pragma unroll
-    for (int q = 0; q < C; ++q) acc[q] = 0.f;
-    for (int f = lane; f < total; f += 32) {
-        int lo = 0, hi = NC - 1;  // the cell with start[ci] <= f < start[ci + 1]
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (start[mid] <= f) lo = mid;
-            else hi = mid - 1;
-        }
-        const int c[3] = {lo % S, (lo / S) % S, lo / (S * S)};
-        const int base[3] = {n[0] - S + 1 + c[0], n[1] - S + 1 + c[1], n[2] - S + 1 + c[2]};
-        const int k[3] = {S - 1 - c[0], S - 1 - c[1], S - 1 - c[2]};
-        fn((uint32_t)(first[lo] + (f - start[lo])), base, k, acc);
+    for (int e = 0; e < 8; ++e) {
+        const int d[3] = {e & 1, (e >> 1) & 1, (e >> 2) & 1};
+        const int B[3] = {N[0] - d[0], N[1] - d[1], N[2] - d[2]};
+        const int i[3] = {((n[0] + 4) & 3) + 4 * d[0], ((n[1] + 4) & 3) + 4 * d[1], ((n[2] + 4) & 3) + 4 * d[2]};
+        const bool in = i[0] < T && i[1] < T && i[2] < T && B[0] >= 0 && B[1] >= 0 && B[2] >= 0 && B[0] < sc.nb[0] &&
+                        B[1] < sc.nb[1] && B[2] < sc.nb[2];
+        slot[e] = in ? a.block_slot[sc.block_base + (uint32_t)((B[2] * sc.nb[1] + B[1]) * sc.nb[0] + B[0])].x : -1;
+        at[e] = i[0] + T * (i[1] + T * i[2]);
     }
 #pragma unroll
-    for (int q = 0; q < C; ++q) {
-        float v = acc[q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        out[q] = __shfl_sync(0xffffffffu, v, 0);  // lane 0's tree order
+    for (int e = 0; e < 8; ++e) {
+        if (slot[e] < 0) continue;
+        const float* t = a.tiles + (size_t)slot[e] * a.tile_stride + at[e];
+        h.x += t[0];
+        h.y += t[TN];
+        h.z += t[2 * TN];
     }
-    __syncwarp();  // sh is reused by the warp's next node
+    return h;
 }
 
 __device__ __forceinline__ void ldMat(const float* prep, size_t stride, size_t i, int plane, float* m) {
@@ -258,22 +206,10 @@ __device__ __forceinline__ void mTm3(const float* A, const float* B, float* C) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-__global__ void cellRangeKernel(const uint32_t* __restrict__ keys, uint32_t n, uint2* __restrict__ range,
-                                uint2* __restrict__ block_range) {
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-        const uint32_t k = keys[i];
-        const uint32_t kp = i > 0 ? keys[i - 1] : 0xffffffffu, kn = i + 1 < n ? keys[i + 1] : 0xffffffffu;
-        if (kp != k) range[k].x = i;
-        if (kn != k) range[k].y = i + 1;
-        if (i == 0 || (kp >> 6) != (k >> 6)) block_range[k >> 6].x = i;
-        if (i + 1 == n || (kn >> 6) != (k >> 6)) block_range[k >> 6].y = i + 1;
-    }
-}
-
 __global__ void __launch_bounds__(kThreads) solvePrepKernel(SolveArgs a) {
     const SceneDev& sc = a.scenes[blockIdx.y];
     if (!solving(sc)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *sc.solve.status = SolveStatus{INT_MAX, 0, 0.f, 0};
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sc.solve.status = SolveStatus{INT_MAX, 0, 0.f};
     const float* f = sc.buf[a.parity].f;
     const uint16_t* mat = sc.buf[a.parity].mat;
     const size_t cap = sc.cap, st = a.ntot;
@@ -323,8 +259,7 @@ __global__ void __launch_bounds__(kThreads) solvePrepKernel(SolveArgs a) {
     }
 }
 
-// Node masses, x0 = v*, the other vectors 0, |M v*|^2, and the list of the
-// nodes with mass.  The masses are the transfer's own: the split-mode grid
+// Node masses, x0 = v*, the other vectors 0 and |M v*|^2.  The masses are the transfer's own: the split-mode grid
 // holds them densely; in the fused step the grid pass wrote (v*, m) for the
 // node blocks N (nodes 4N - 4 + L) next to a particle block N - (0|1, 0|1,
 // 0|1) that holds particles, and the other nodes have no mass this step.
@@ -350,8 +285,8 @@ __global__ void __launch_bounds__(kThreads) solveInitKernel(SolveArgs a) {
             for (int d = 0; d < 8; ++d) {
                 const int B[3] = {N[0] - (d & 1), N[1] - ((d >> 1) & 1), N[2] - (d >> 2)};
                 if (B[0] >= 0 && B[1] >= 0 && B[2] >= 0 && B[0] < sc.nb[0] && B[1] < sc.nb[1] && B[2] < sc.nb[2]) {
-                    const uint2 r = a.block_range[sc.block_base + (uint32_t)((B[2] * sc.nb[1] + B[1]) * sc.nb[0] + B[0])];
-                    written |= r.y > r.x;
+                    written |=
+                        a.block_slot[sc.block_base + (uint32_t)((B[2] * sc.nb[1] + B[1]) * sc.nb[0] + B[0])].x >= 0;
                 }
             }
             if (written) {
@@ -363,76 +298,107 @@ __global__ void __launch_bounds__(kThreads) solveInitKernel(SolveArgs a) {
             }
         }
         const bool act = m > kFltEps;
-        if (act) {
+        if (act)
             acc += (double)(m * vs[0]) * (m * vs[0]) + (double)(m * vs[1]) * (m * vs[1]) +
                    (double)(m * vs[2]) * (m * vs[2]);
-            sc.solve.list[atomicAdd(&sc.solve.status->nactive, 1)] = (int)node;
-        }
         sc.solve.m[node] = act ? m : 0.f;
         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
         vec[(size_t)VX * nodes + node] = act ? make_float4(vs[0], vs[1], vs[2], 0.f) : z4;
 #pragma unroll
-        for (int v = VR; v <= VH; ++v) vec[(size_t)v * nodes + node] = z4;
+        for (int v = VR; v <= VAZ; ++v) vec[(size_t)v * nodes + node] = z4;
     }
     writePartial(acc, partSlot(sc, QBB, 0));
 }
 
+// The particles of a work item: G from the item's tile of u, staged in shared
+// memory (nodes outside the grid as zeros), then T = V0 dP(G Fe) Fe^T.
 template <int S>
 __global__ void __launch_bounds__(kThreads) solveGatherKernel(SolveArgs a, int src, const int* kp, int k0) {
-    const SceneDev& sc = a.scenes[blockIdx.y];
-    const int k = kp ? *kp : k0;
-    if (!solving(sc) || sc.S != S || blockDoneAt(sc) <= k) return;
-    const size_t nodes = sceneNodes(sc), st = a.ntot;
-    const float4* u = sc.solve.vec + (size_t)src * nodes;
-    const uint32_t outside = sc.block_base + sc.nblocks;
-    for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < sc.n; j += gridDim.x * kThreads) {
-        const size_t i = (size_t)sc.key_offset + j;
-        float4* To = a.T + 3 * i;
-        const uint32_t key = a.sorted_keys[i];
-        if ((key >> 6) >= outside) {
-            To[0] = To[1] = To[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-            continue;
+    constexpr int T = S + 3, TN = tileNodes(S);
+    __shared__ float4 tile[TN];
+    __shared__ uint32_t first[kMaxCombos + 1];  // items of the combinations before each
+    const int k = kp ? kp[0] : k0;
+    if (kp && kp[1]) return;
+    if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        for (int q = 0; q < kMaxCombos; ++q) {
+            first[q] = run;
+            run += a.counters[kG2PCountWord + q];
         }
-        int base[3];
-        keyBase(sc, key, base);
-        const float4 q = a.pofs[i];
-        const float d0[3] = {q.x, q.y, q.z};
-        float w[3][S], dw[3][S];
+        first[kMaxCombos] = run;
+    }
+    __syncthreads();
+    const size_t st = a.ntot;
+    for (uint32_t w = blockIdx.x; w < first[kMaxCombos]; w += gridDim.x) {
+        int q = 0;
+        while (w >= first[q + 1]) ++q;
+        const BlockItem it = a.items[(size_t)q * a.items_cap + (w - first[q])];
+        const SceneDev& sc = a.scenes[it.scene];
+        if (!solving(sc) || sc.S != S || sc.solve.status->done_at <= k) continue;  // the same for the whole CTA
+        const float4* u = sc.solve.vec + (size_t)src * sceneNodes(sc);
+        const uint32_t lb = it.block - sc.block_base;
+        const int t0[3] = {4 * (int)(lb % (uint32_t)sc.nb[0]) - 4,
+                           4 * (int)((lb / (uint32_t)sc.nb[0]) % (uint32_t)sc.nb[1]) - 4,
+                           4 * (int)(lb / ((uint32_t)sc.nb[0] * (uint32_t)sc.nb[1])) - 4};
+        __syncthreads();  // the previous item's tile is no longer read
+        for (int e = threadIdx.x; e < TN; e += kThreads) {
+            const int n[3] = {t0[0] + e % T, t0[1] + (e / T) % T, t0[2] + e / (T * T)};
+            const bool in = n[0] >= 0 && n[1] >= 0 && n[2] >= 0 && n[0] < sc.res[0] && n[1] < sc.res[1] && n[2] < sc.res[2];
+            tile[e] = in ? u[(size_t)n[0] + (size_t)sc.res[0] * ((size_t)n[1] + (size_t)sc.res[1] * n[2])]
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < it.count; j += kThreads) {
+        const size_t i = (size_t)it.start + j;
+        float4* To = a.T + 3 * i;
+        const uint32_t cell = a.sorted_keys[i] & 63u;
+        const float4* origin = tile + (cell & 3u) + T * (((cell >> 2) & 3u) + T * (cell >> 4));
+        const float4 q0 = a.pofs[i];
+        const float d0[3] = {q0.x, q0.y, q0.z};
+        float w3[3][S], dw[3][S];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
             float dk[S];
             dk[0] = d0[ax];
 #pragma unroll
             for (int kk = 1; kk < S; ++kk) dk[kk] = dk[0] - (float)kk;
-            splineWeights<S>(dk, w[ax], dw[ax]);
+            splineWeights<S>(dk, w3[ax], dw[ax]);
 #pragma unroll
             for (int kk = 0; kk < S; ++kk) dw[ax][kk] *= sc.inv_h;
         }
+        // axis by axis: rows along x, planes along y, then z; column c of G is
+        // the sum with the derivative along axis c
         float G[9];
 #pragma unroll
         for (int e = 0; e < 9; ++e) G[e] = 0.f;
 #pragma unroll
         for (int c = 0; c < S; ++c) {
-            const int nz = base[2] + c;
-            if (nz < 0 || nz >= sc.res[2]) continue;
+            float p0[3] = {0.f, 0.f, 0.f}, pd[3] = {0.f, 0.f, 0.f}, py[3] = {0.f, 0.f, 0.f};
 #pragma unroll
             for (int b = 0; b < S; ++b) {
-                const int ny = base[1] + b;
-                if (ny < 0 || ny >= sc.res[1]) continue;
+                float r0[3] = {0.f, 0.f, 0.f}, rd[3] = {0.f, 0.f, 0.f};
 #pragma unroll
                 for (int ai = 0; ai < S; ++ai) {
-                    const int nx = base[0] + ai;
-                    if (nx < 0 || nx >= sc.res[0]) continue;
-                    const float3 uv = ld3(u[(size_t)nx + (size_t)sc.res[0] * ((size_t)ny + (size_t)sc.res[1] * nz)]);
-                    const float g[3] = {dw[0][ai] * w[1][b] * w[2][c], w[0][ai] * dw[1][b] * w[2][c],
-                                        w[0][ai] * w[1][b] * dw[2][c]};
+                    const float4 uv = origin[ai + T * (b + T * c)];
+                    const float v[3] = {uv.x, uv.y, uv.z};
 #pragma unroll
-                    for (int col = 0; col < 3; ++col) {
-                        G[col] += uv.x * g[col];
-                        G[3 + col] += uv.y * g[col];
-                        G[6 + col] += uv.z * g[col];
+                    for (int r = 0; r < 3; ++r) {
+                        r0[r] = fmaf(w3[0][ai], v[r], r0[r]);
+                        rd[r] = fmaf(dw[0][ai], v[r], rd[r]);
                     }
                 }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    p0[r] = fmaf(w3[1][b], r0[r], p0[r]);
+                    pd[r] = fmaf(w3[1][b], rd[r], pd[r]);
+                    py[r] = fmaf(dw[1][b], r0[r], py[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                G[3 * r] = fmaf(w3[2][c], pd[r], G[3 * r]);
+                G[3 * r + 1] = fmaf(w3[2][c], py[r], G[3 * r + 1]);
+                G[3 * r + 2] = fmaf(dw[2][c], p0[r], G[3 * r + 2]);
             }
         }
         float F[9], C[9], dF[9], dP[9];
@@ -483,35 +449,6 @@ __global__ void __launch_bounds__(kThreads) solveGatherKernel(SolveArgs a, int s
         To[1] = make_float4(Tm[3], Tm[4], Tm[5], 0.f);
         To[2] = make_float4(Tm[6], Tm[7], Tm[8], 0.f);
     }
-}
-
-// h = sum_p T_p grad w_ip at the listed nodes (one warp per node).
-template <int S>
-__global__ void __launch_bounds__(kThreads) solveScatterKernel(SolveArgs a, const int* kp, int k0) {
-    const SceneDev& sc = a.scenes[blockIdx.y];
-    const int k = kp ? *kp : k0;
-    if (!solving(sc) || sc.S != S || blockDoneAt(sc) <= k) return;
-    __shared__ int sh[kThreads / 32][2 * S * S * S + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t nodes = sceneNodes(sc);
-    float4* h = sc.solve.vec + (size_t)VH * nodes;
-    const int na = sc.solve.status->nactive;
-    for (int li = blockIdx.x * (kThreads / 32) + warp; li < na; li += gridDim.x * (kThreads / 32)) {
-        const size_t node = (size_t)sc.solve.list[li];
-        int n[3];
-        nodeCoords(sc, node, n);
-        float out[3];
-        warpNodeSum<S, 3>(sc, a, n, sh[warp], out, [&](uint32_t p, const int* base, const int* kk, float* acc) {
-            float w[3], dw[3];
-            nodeWeight<S>(sc, a.pofs[p], kk, w, dw);
-            const float g[3] = {dw[0] * w[1] * w[2], w[0] * dw[1] * w[2], w[0] * w[1] * dw[2]};
-            const float4* Tp = a.T + 3 * (size_t)p;
-            const float4 t0 = Tp[0], t1 = Tp[1], t2 = Tp[2];
-            acc[0] += t0.x * g[0] + t0.y * g[1] + t0.z * g[2];
-            acc[1] += t1.x * g[0] + t1.y * g[1] + t1.z * g[2];
-            acc[2] += t2.x * g[0] + t2.y * g[1] + t2.z * g[2];
-        });
-        if (lane == 0) h[node] = make_float4(out[0], out[1], out[2], 0.f);
     }
 }
 
@@ -527,7 +464,9 @@ __global__ void __launch_bounds__(kThreads) solveResidualKernel(SolveArgs a) {
          node += (size_t)kSolveBlocks * kThreads) {
         const float m = sc.solve.m[node];
         if (!(m > 0.f)) continue;
-        const float3 h = ld3(vec[(size_t)VH * nodes + node]);
+        int n[3];
+        nodeCoords(sc, node, n);
+        const float3 h = tileSum(a, sc, n);
         const float r[3] = {-c * h.x, -c * h.y, -c * h.z};
         vec[(size_t)VR * nodes + node] = make_float4(r[0], r[1], r[2], 0.f);
         vec[(size_t)VZ * nodes + node] = make_float4(r[0] / m, r[1] / m, r[2] / m, 0.f);
@@ -549,7 +488,9 @@ __global__ void __launch_bounds__(kThreads) solveAzKernel(SolveArgs a, const int
          node += (size_t)kSolveBlocks * kThreads) {
         const float m = sc.solve.m[node];
         if (!(m > 0.f)) continue;
-        const float3 z = ld3(vec[(size_t)VZ * nodes + node]), h = ld3(vec[(size_t)VH * nodes + node]);
+        int n[3];
+        nodeCoords(sc, node, n);
+        const float3 z = ld3(vec[(size_t)VZ * nodes + node]), h = tileSum(a, sc, n);
         const float Az[3] = {m * z.x + c * h.x, m * z.y + c * h.y, m * z.z + c * h.z};
         vec[(size_t)VAZ * nodes + node] = make_float4(Az[0], Az[1], Az[2], 0.f);
         acc += (double)z.x * Az[0] + (double)z.y * Az[1] + (double)z.z * Az[2];
@@ -633,7 +574,8 @@ __global__ void solveCondKernel(SolveArgs a, int nscenes, cudaGraphConditionalHa
     }
     running = __syncthreads_or(running);
     if (threadIdx.x == 0) {
-        *a.iter = k + 1;
+        a.iter[0] = k + 1;
+        a.iter[1] = !running;
         if (use_cond) cudaGraphSetConditional(h, running ? 1u : 0u);
     }
 }
@@ -668,20 +610,18 @@ __global__ void __launch_bounds__(kThreads) solveFinalKernel(SolveArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-cudaError_t launchSolve(const LaunchCtx& c, const SolveBuffers& b, int parity, const int* stencils, int nstencils,
-                        int max_iter, bool split, cudaStream_t aux) {
-    SolveArgs a{c.scenes, b.sorted_keys, b.perm, b.cell_range, b.block_range, b.pofs, b.prep, b.T, b.ntot, parity,
-                split ? 1 : 0, b.iter};
+cudaError_t launchSolve(const LaunchCtx& c, const StepArgs& step, const SolveBuffers& b, int parity,
+                        const int* stencils, int nstencils, int max_iter, bool split, cudaStream_t aux) {
+    SolveArgs a{c.scenes, b.sorted_keys, b.perm, step.g2p_items, step.g2p_cap, step.counters, step.block_slot,
+                step.tiles, step.tile_stride, b.pofs, b.prep, b.T, b.ntot, parity, split ? 1 : 0, b.iter};
+    StepArgs sa = step;
+    sa.solve_pofs = b.pofs;
+    sa.solve_T = b.T;
     const dim3 pgrid(c.particle_blocks, (unsigned)c.nscenes), ngrid(kSolveBlocks, (unsigned)c.nscenes);
-    const dim3 wgrid((unsigned)c.num_sms * 8, (unsigned)c.nscenes);  // warp-per-node kernels
+    const unsigned igrid = (unsigned)c.num_sms * 4;  // CTAs of the work-item kernels
     uint64_t launches = 0;
-    cudaMemsetAsync(b.cell_range, 0, sizeof(uint2) * b.nkeys, c.stream);
-    cudaMemsetAsync(b.block_range, 0, sizeof(uint2) * b.nblocks, c.stream);
-    const unsigned kb = (unsigned)std::max<size_t>(
-        1, std::min<size_t>((b.ntot + kThreads - 1) / kThreads, (size_t)c.num_sms * 8));
-    cellRangeKernel<<<kb, kThreads, 0, c.stream>>>(b.sorted_keys, b.ntot, b.cell_range, b.block_range);
     solvePrepKernel<<<pgrid, kThreads, 0, c.stream>>>(a);
-    launches += 2;
+    ++launches;
     auto perS = [&](auto launch) {
         for (int i = 0; i < nstencils; ++i) {
             switch (stencils[i]) {
@@ -694,9 +634,15 @@ cudaError_t launchSolve(const LaunchCtx& c, const SolveBuffers& b, int parity, c
     };
     cudaStream_t st = c.stream;  // the stream of the iteration kernels
     const int* kp = nullptr;
-    auto gatherX = [&](auto S) { solveGatherKernel<decltype(S)::value><<<pgrid, kThreads, 0, st>>>(a, VX, nullptr, -1); };
-    auto gatherZ = [&](auto S) { solveGatherKernel<decltype(S)::value><<<pgrid, kThreads, 0, st>>>(a, VZ, kp, -1); };
-    auto scatter = [&](auto S) { solveScatterKernel<decltype(S)::value><<<wgrid, kThreads, 0, st>>>(a, kp, -1); };
+    auto gatherX = [&](auto S) { solveGatherKernel<decltype(S)::value><<<igrid, kThreads, 0, st>>>(a, VX, nullptr, -1); };
+    auto gatherZ = [&](auto S) { solveGatherKernel<decltype(S)::value><<<igrid, kThreads, 0, st>>>(a, VZ, kp, -1); };
+    auto scatter = [&](auto S) {
+        LaunchCtx cc = c;
+        cc.stream = st;
+        sa.solve_iter = kp;
+        launchP2G(cc, sa, decltype(S)::value, MODE_HESS, -1);
+        --launches;  // counted there
+    };
     solveInitKernel<<<ngrid, kThreads, 0, st>>>(a);
     perS(gatherX);
     perS(scatter);
@@ -705,7 +651,7 @@ cudaError_t launchSolve(const LaunchCtx& c, const SolveBuffers& b, int parity, c
     perS(scatter);
     solveAzKernel<<<ngrid, kThreads, 0, st>>>(a, nullptr, 0, -1);
     solveDirKernel<<<ngrid, kThreads, 0, st>>>(a, nullptr, 0, -1);
-    cudaMemsetAsync(b.iter, 0, sizeof(int), st);
+    cudaMemsetAsync(b.iter, 0, 2 * sizeof(int), st);
     launches += 4;
     kp = b.iter;
     auto body = [&](cudaGraphConditionalHandle h, int use_cond) {

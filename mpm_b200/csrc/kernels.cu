@@ -560,6 +560,8 @@ __global__ void __launch_bounds__(kThreads) stressKernel(const SceneDev* __restr
 //                momentum w X_a m v, force X'_a w T_i0 + X_a R^i
 //   SPLIT      : the first with T = 0, then X' | T_i0 | (Y'_b T_i1, -) [S] | (Z'_c T_i2, -) [S]
 //   MASS       : m X_0.. | Y_0.. | Z_0..
+//   HESS       : PIC-FLIP's without the first (the force of the semi-implicit
+//                solver's T = V0 dP Fe^T, not symmetric)
 // ---------------------------------------------------------------------------
 // One lane's sums for one stencil node, in packed FP32 pairs so that two
 // components go through one __ffma2_rn (two exactly rounded FMAs):
@@ -584,9 +586,10 @@ struct P2GStage {
     static constexpr int T = S + 3;                   // nodes of a row along x
     static constexpr int TN = tileNodes(S);
     static constexpr bool kC = MODE == MODE_APIC_FUSED || MODE == MODE_SPLIT;  // XX words
-    static constexpr bool kSepF = MODE == MODE_FLIP || MODE == MODE_SPLIT;     // force apart from momentum
+    static constexpr bool kMom = MODE != MODE_HESS;                            // mass and momentum
+    static constexpr bool kSepF = MODE == MODE_FLIP || MODE == MODE_SPLIT || MODE == MODE_HESS;  // force apart from momentum
     static constexpr int WXX = 0;                     // XX (or m v, m)
-    static constexpr int WX = MODE == MODE_MASS ? 0 : (kC ? S : 1);
+    static constexpr int WX = MODE == MODE_MASS || !kMom ? 0 : (kC ? S : 1);
     static constexpr int WXD = WX + 1;                // X' (kSepF), then T_i0
     static constexpr int WT = WXD + 1;
     static constexpr int WY = MODE == MODE_MASS ? 1 : (kSepF ? WT + 1 : WX + 1);
@@ -694,7 +697,17 @@ struct P2GRaw {
     float x[3], m, v[3], t[6], B[9];
     bool bad;  // range check failed: the particle contributes nothing
     __device__ __forceinline__ void load(const StepArgs& args, const SceneDev& sc, const float* pf, size_t cap,
-                                         uint32_t perm) {
+                                         uint32_t perm, uint32_t at) {
+        if constexpr (MODE == MODE_HESS) {  // by sorted position: x holds the stencil offsets, B the matrix T
+            const float4 q = args.solve_pofs[at];
+            x[0] = q.x, x[1] = q.y, x[2] = q.z;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const float4 row = args.solve_T[3 * (size_t)at + r];
+                B[3 * r] = row.x, B[3 * r + 1] = row.y, B[3 * r + 2] = row.z;
+            }
+            return;
+        }
         uint32_t old = perm - sc.key_offset;
         bad = old >= sc.n;
         if (bad) {
@@ -729,9 +742,9 @@ __device__ __forceinline__ void p2gStageParticle(const SceneDev& sc, const P2GRa
     using R = P2GStage<S, MODE>;
     const float (&x)[3] = raw.x;
     const float (&v)[3] = raw.v;
-    const float m = raw.bad ? 0.f : raw.m;
+    const float m = MODE == MODE_HESS || raw.bad ? 0.f : raw.m;
     float t[6], mC[9];
-    if (MODE != MODE_MASS) {
+    if (MODE != MODE_MASS && MODE != MODE_HESS) {
         const float ts = raw.bad ? 0.f : (MODE == MODE_APIC_FUSED ? -dt : -1.0f);
 #pragma unroll
         for (int k = 0; k < 6; ++k) t[k] = ts * raw.t[k];
@@ -752,7 +765,10 @@ __device__ __forceinline__ void p2gStageParticle(const SceneDev& sc, const P2GRa
         // (x_p - (o + h i)) / h; the B-splines are smooth there and use
         // d0 - k (exact subtraction).
         float dk[S];
-        if (S == 2) {
+        if (MODE == MODE_HESS) {
+#pragma unroll
+            for (int k = 0; k < S; ++k) dk[k] = x[a] - (float)k;
+        } else if (S == 2) {
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 const float gp = __fadd_rn(sc.origin[a], __fmul_rn(h, (float)(base[a] + k)));
@@ -807,10 +823,20 @@ __device__ __forceinline__ void p2gStageParticle(const SceneDev& sc, const P2GRa
             my[R::WY + k] = make_float4(yy[0], yy[1], yy[2], wk[1][k]);
             my[R::WZ + k] = make_float4(zz[0], zz[1], zz[2], wk[2][k]);
         }
-    } else {
+    } else if (R::kMom) {
         my[R::WXX] = make_float4(m * v[0], m * v[1], m * v[2], m);
     }
-    if (R::kSepF) {
+    if (MODE == MODE_HESS) {
+        const float (&B)[9] = raw.B;
+        my[R::WXD] = row4(dwk[0]);
+        my[R::WT] = make_float4(B[0], B[3], B[6], 0.f);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            const float dy = dwk[1][k], dz = dwk[2][k];
+            my[R::WYF + k] = make_float4(dy * B[1], dy * B[4], dy * B[7], wk[1][k]);
+            my[R::WZF + k] = make_float4(dz * B[2], dz * B[5], dz * B[8], wk[2][k]);
+        }
+    } else if (R::kSepF) {
         my[R::WXD] = row4(dwk[0]);
         my[R::WT] = make_float4(t[0], t[3], t[4], 0.f);
 #pragma unroll
@@ -856,7 +882,7 @@ __device__ __forceinline__ void p2gAccumulate(const float4* st, int q0, int qhi,
                 n.pxy = __ffma2_rn(w2, make_float2(xx.x, xx.y), __ffma2_rn(xa, Rxy, n.pxy));
                 n.pzm = __ffma2_rn(w2, make_float2(xx.z, xx.w), __ffma2_rn(xa, Rz0, n.pzm));
             }
-        } else {
+        } else if (R::kMom) {
             const float4 mv = pq[R::WXX];
             const float2 Pxy = __fmul2_rn(w2, make_float2(mv.x, mv.y)), Pzm = __fmul2_rn(w2, make_float2(mv.z, mv.w));
 #pragma unroll
@@ -910,7 +936,7 @@ struct RowWindow {
         if (cells & touch) {
             float v[L::F];
 #pragma unroll
-            for (int f = 0; f < L::F; ++f) v[f] = acc[N % S].get(f);
+            for (int f = 0; f < L::F; ++f) v[f] = acc[N % S].get(MODE == MODE_HESS ? 4 + f : f);
             acc[N % S].zero();
             groupReduce<L::F, 1, L::G>(v, lane);
             out(N, v);
@@ -1048,6 +1074,8 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
     const uint32_t nwork = !list ? args.counters[0]
                                  : nlist1 + (p2gWarpTakesSmall(args.p2g_warp, nsmall) ? 0u : nsmall);
     const uint32_t* small = list ? args.p2g_lists + (size_t)(2 * args.combo) * args.p2g_list_cap : nullptr;
+    const int solve_k = MODE == MODE_HESS && args.solve_iter ? args.solve_iter[0] : -1;
+    if (MODE == MODE_HESS && args.solve_iter && args.solve_iter[1]) return;  // every scene has converged
     spanBegin(args.spans, SPAN_P2G);
     __shared__ uint32_t item_s;
     __shared__ SceneDev sc_s;
@@ -1063,6 +1091,7 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
             const SceneDev& scg = args.scenes[it.scene];
             if (scg.S != S || (want_transfer >= 0 && scg.transfer != want_transfer)) continue;
             if (MODE == MODE_MASS && !scg.init_pass) continue;
+            if (MODE == MODE_HESS && !(scg.beta > 0.f && scg.solve.status->done_at > solve_k)) continue;
         }
         const uint32_t i0 = it.start;
         const int icount = (int)it.count;
@@ -1150,7 +1179,7 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
                 const bool stages = lane < L::kStage;
                 if (stages && gb + lane < ce0) {
                     cl = keys[gb + lane] & 63u;
-                    raw.load(args, sc, pf, cap, perm[gb + lane]);
+                    raw.load(args, sc, pf, cap, perm[gb + lane], i0 + (uint32_t)(gb + lane));
                 }
                 if (stages && gb + L::kStage + lane < ce0) {
                     ncl = keys[gb + L::kStage + lane] & 63u;
@@ -1161,7 +1190,8 @@ __global__ void __launch_bounds__(P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MO
                     if (lane < np) p2gStageParticle<S, MODE>(sc, raw, dt, h, inv_h, t0, cl, st + lane * L::P4);
                     const uint32_t pcl = cl;  // this pass's cells
                     const int next_x = (int)(__shfl_sync(0xffffffffu, ncl, 0) & 3u);  // only read where the segment goes on
-                    if (stages && g0 + L::kStage + lane < ce0) raw.load(args, sc, pf, cap, nperm);
+                    if (stages && g0 + L::kStage + lane < ce0)
+                        raw.load(args, sc, pf, cap, nperm, i0 + (uint32_t)(g0 + L::kStage + lane));
                     cl = ncl;
                     if (stages && g0 + 2 * L::kStage + lane < ce0) {
                         ncl = keys[g0 + 2 * L::kStage + lane] & 63u;
@@ -1333,7 +1363,7 @@ __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, M
         const bool stages = lane < W::kStage;
         if (stages && lane < count) {
             cl = keys[lane] & 63u;
-            raw.load(args, sc, pf, cap, perm[lane]);
+            raw.load(args, sc, pf, cap, perm[lane], i0 + (uint32_t)lane);
         }
         if (stages && W::kStage + lane < count) {
             ncl = keys[W::kStage + lane] & 63u;
@@ -1344,7 +1374,8 @@ __global__ void __launch_bounds__(P2GWarpLayout<S, MODE>::NT, P2GWarpLayout<S, M
             if (lane < np) p2gStageParticle<S, MODE>(sc, raw, dt, h, inv_h, t0, cl, st + lane * W::P4);
             const uint32_t pcl = cl;  // this pass's cells
             const int next_x = (int)(__shfl_sync(0xffffffffu, ncl, 0) & 3u);  // only read where the segment goes on
-            if (stages && g0 + W::kStage + lane < count) raw.load(args, sc, pf, cap, nperm);
+            if (stages && g0 + W::kStage + lane < count)
+                raw.load(args, sc, pf, cap, nperm, i0 + (uint32_t)(g0 + W::kStage + lane));
             cl = ncl;
             if (stages && g0 + 2 * W::kStage + lane < count) {
                 ncl = keys[g0 + 2 * W::kStage + lane] & 63u;
@@ -2467,6 +2498,7 @@ void launchP2G(const LaunchCtx& c, const StepArgs& a, int S, int mode, int want_
             case MODE_APIC_FUSED: p2gOne<SS, MODE_APIC_FUSED>(c, a, want_transfer); break; \
             case MODE_FLIP: p2gOne<SS, MODE_FLIP>(c, a, want_transfer); break;         \
             case MODE_SPLIT: p2gOne<SS, MODE_SPLIT>(c, a, want_transfer); break;       \
+            case MODE_HESS: p2gLaunch<SS, MODE_HESS, 32>(c, a, want_transfer); break;  \
             default: p2gOne<SS, MODE_MASS>(c, a, want_transfer); break;                \
         }                                                                              \
     }
