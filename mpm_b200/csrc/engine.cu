@@ -991,10 +991,12 @@ public:
         CUDA_TRY(cudaMemsetAsync(block_count_.p, 0, sizeof(uint32_t) * tb, stream_));
         MPM_TRY(grow(sbb_, sizeof(uint32_t) * (ns + 1), "scene block bases"));
         CUDA_TRY(cudaMemcpyAsync(sbb_.p, sbb.data(), sizeof(uint32_t) * (ns + 1), cudaMemcpyHostToDevice, stream_));
-        // work items: one per non-empty block plus at most one per kSplitChunk particles
-        max_active_ = std::max<size_t>(1, std::min<size_t>(tb, nk) + nk / kSplitChunk + 1);
+        // work items: one per non-empty block plus at most one per split chunk of particles
+        size_t split_items = 0;
+        for (auto& s : scenes_) split_items += s->n / splitChunk((uint32_t)s->n) + 1;
+        max_active_ = std::max<size_t>(1, std::min<size_t>(tb, nk) + split_items);
         MPM_TRY(grow(active_, sizeof(BlockItem) * max_active_, "active blocks"));
-        MPM_TRY(grow(outside_, sizeof(BlockItem) * ((size_t)ns + nk / kSplitChunk + 1), "outside blocks"));
+        MPM_TRY(grow(outside_, sizeof(BlockItem) * ((size_t)ns + split_items), "outside blocks"));
         g2p_cap_ = (uint32_t)(std::min<size_t>(tb, nk) + nk / kMinG2PChunk + 1);
         MPM_TRY(grow(g2p_items_, sizeof(BlockItem) * g2p_cap_ * (size_t)combos().size(), "G2P items"));
         // P2G's two lists of item slots per combination (warp items, CTA items)

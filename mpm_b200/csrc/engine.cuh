@@ -27,17 +27,28 @@ constexpr int kSortTileKeys = kThreads * 8;  // keys per radix-sort tile (8 per 
 // equal size, so that a few crowded blocks cannot serialize a step.  Each item
 // has its own tile; the last of a block's items to finish adds their tiles up
 // in item order, so the grid pass reads one tile per block.  The split fixes
-// the order of P2G's sums, so both are constants.  Where the line lies: at 35
-// particles a cell (2,200 a full block) whole blocks are faster than items of
-// 2048 or 1024 (P2G 0.099, 0.105 and 0.121 ms), which have too few rows each;
+// the order of P2G's sums, so it depends on nothing but the block's and its
+// scene's particle counts.  Where the line lies: at 35 particles a cell (2,200
+// a full block) whole blocks are faster than items of 2048 or 1024 (P2G 0.099,
+// 0.105 and 0.121 ms), which have too few rows each;
 // a block above 40 a cell has long rows, and scenes of few such blocks need
 // the parallelism (six scenes of up to 60k particles, P2G: items of up to 4096
 // 0.146 ms, split above 4096 into 1024s 0.116, above 2560 into 1280s 0.092;
 // into 640s 0.088, but 64 scenes of up to 500k 0.88 -> 1.03 ms).
 constexpr uint32_t kBlockChunk = 2560;
 constexpr uint32_t kSplitChunk = 1280;
-__host__ __device__ inline uint32_t blockItems(uint32_t count) {
-    return count <= kBlockChunk ? (count ? 1u : 0u) : (count + kSplitChunk - 1) / kSplitChunk;
+// A scene of at most kFewParticles cannot fill the chip with such items: its
+// crowded blocks are split above kFewBlockChunk into kFewSplitChunks (the six
+// scenes' step 0.123 -> 0.107 ms, P2G 0.095 -> 0.063; 512s above 1024 the same,
+// 512s above 640 0.115; the 64 scenes, of which few are that small, 1.718 ->
+// 1.725).  The line is the scene's own count, not the batch's, so that a scene
+// in a batch keeps the bits it has alone.
+constexpr uint32_t kFewParticles = 65536, kFewBlockChunk = 1280, kFewSplitChunk = 640;
+__host__ __device__ inline uint32_t splitChunk(uint32_t n) { return n <= kFewParticles ? kFewSplitChunk : kSplitChunk; }
+// The work items of a block of `count` particles of a scene of n.
+__host__ __device__ inline uint32_t blockItems(uint32_t count, uint32_t n) {
+    const uint32_t whole = n <= kFewParticles ? kFewBlockChunk : kBlockChunk, split = splitChunk(n);
+    return count <= whole ? (count ? 1u : 0u) : (count + split - 1) / split;
 }
 // Particles that a P2G warp stages at a time unless the caller sets it
 // (mpm_tuning.p2g_stage): a full warp.  16 and 24 were slower for every density

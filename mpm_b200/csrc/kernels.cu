@@ -238,7 +238,7 @@ __device__ __forceinline__ unsigned long long blockLoad(const CompactArgs& a, ui
     if (c == 0) return 0ull;
     const int s = *scene = sceneOfBlock(a.scene_block_base, a.nscenes, b);
     const bool out = b == a.scene_block_base[s + 1] - 1;
-    return ((out ? 0ull : (unsigned long long)blockItems(c)) << 32) | (unsigned long long)c;
+    return ((out ? 0ull : (unsigned long long)blockItems(c, a.scenes[s].n)) << 32) | (unsigned long long)c;
 }
 
 // The work items, slots, ranges and list entries of the thread's PER blocks
@@ -392,7 +392,7 @@ __device__ __forceinline__ void placeBlocks(const CompactArgs& a, uint32_t b0, c
         } else {
             a.block_slot[b] = make_int2(-1, 0);
             if (count > 0) {
-                const uint32_t nitems = blockItems(count);
+                const uint32_t nitems = blockItems(count, a.scenes[scene].n);
                 const uint32_t o = atomicAdd(&a.counters[1], nitems);
                 splitItems(a.outside + o, b, start, count, nitems, (uint32_t)scene);
             }
