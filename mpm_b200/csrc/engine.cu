@@ -390,10 +390,28 @@ public:
     // engines that are created and destroyed (solvers of a server, the
     // benchmark's repeated constructions) reuse memory without cudaMalloc or
     // the implicit device synchronization of cudaFree.
-    mpm_status alloc(DevMem& m, size_t b, const char* what) { return m.allocPooled(b, what, pool_, stream_); }
+    mpm_status alloc(DevMem& m, size_t b, const char* what) {
+        if (m.p && m.bytes >= b) return MPM_OK;
+        const mpm_status st = m.allocPooled(b, what, pool_, stream_);
+        return st == MPM_ERR_OOM && releaseUploads() ? m.allocPooled(b, what, pool_, stream_) : st;
+    }
     mpm_status grow(DevMem& m, size_t b, const char* what) {
         if (m.p && m.bytes >= b) return MPM_OK;
-        return m.allocPooled(std::max(b, m.bytes + m.bytes / 2), what, pool_, stream_);
+        return alloc(m, std::max(b, m.bytes + m.bytes / 2), what);
+    }
+    // The upload buffers stay with the engine between scenes: given back at
+    // each rebuild, the step's scratch took their memory and the next
+    // construction waited for the pool to map more (one of ten two-ball
+    // constructions 4 to 15 ms instead of 1.0).  Where memory runs out they
+    // are given back, except the one that a scene is being added from.
+    bool releaseUploads() {
+        bool any = false;
+        for (int k = 0; k < 2; ++k) {
+            if (!upload_[k].p || k == upload_busy_) continue;
+            upload_[k].release();
+            any = true;
+        }
+        return any;
     }
     // Returns the engine's own buffers to the pool in the stream's order
     // (called before the stream is destroyed).
@@ -580,6 +598,11 @@ public:
             const int u = staged_bytes <= kUploadTwice ? upload_next_ : 0;
             upload_next_ = u ^ 1;
             const bool fresh = upload_[u].bytes < staged_bytes;
+            upload_busy_ = u;
+            struct Busy {
+                int& b;
+                ~Busy() { b = -1; }
+            } busy{upload_busy_};
             MPM_TRY(grow(upload_[u], staged_bytes, "particle upload buffer"));
             float* staged = upload_[u].as<float>();
             uint16_t* staged_mat = p.material ? (uint16_t*)((char*)upload_[u].p + mat_off) : nullptr;
@@ -610,7 +633,9 @@ public:
                 CUDA_TRY(cudaMemcpyAsync(staged_mat, p.material, sizeof(uint16_t) * n, cudaMemcpyHostToDevice,
                                          compact_stream_));
             CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
-            MPM_TRY(newScene(d, p.materials, p.nmaterials, p.n, &sc));
+            mpm_status made = newScene(d, p.materials, p.nmaterials, p.n, &sc);
+            if (made == MPM_ERR_OOM && releaseUploads()) made = newScene(d, p.materials, p.nmaterials, p.n, &sc);
+            MPM_TRY(made);
             const uint32_t* perm = nullptr;
             DevMem sk[2], sv[2], sscr;  // back to the pool in the stream's order on return
             if (sorted) {
@@ -959,7 +984,6 @@ public:
         total_blocks_ = (uint32_t)tb;
         key_bits_ = 1;
         while (((uint64_t)1 << key_bits_) < tb * 64) ++key_bits_;
-        for (auto& m : upload_) m.release();  // back to the pool until the next scene is added
         // batch scratch
         const size_t nk = std::max<size_t>(ntot, 1);
         for (int k = 0; k < 2; ++k) {
@@ -2519,7 +2543,7 @@ private:
     DevMem keys_[2], vals_[2], sort_scratch_, range_[2], emig_count_[2], emig_, far_, arrivals_, far_count_, sort_list_, dense_list_, compact_scratch_, block_count_, sbb_, active_,
         outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, tmp_, upload_[2], g2p_items_, tmaps_, spans_, p2g_lists_;
     cudaEvent_t upload_free_[2] = {};  // the scene staged in upload_[k] has been written
-    int upload_next_ = 0;
+    int upload_next_ = 0, upload_busy_ = -1;  // the buffer of the next scene; of the scene being added, or -1
     // Per combination: the first step after a change of the scene set found
     // fewer than kWarpAutoMinItems small P2G items, so the step does not
     // launch the warp kernel (see checkWarpItems, warpModeOf).
