@@ -308,7 +308,7 @@ def peaks():
 TRAFFIC_SOURCE = ("ncu capture of one launch of the kernel in a separate run of this bench on the same workload "
                   "(dram__bytes_read.sum + dram__bytes_write.sum)")
 NCU_TRAFFIC = {
-    "two_balls": {"p2g": 104.8e6, "g2p": 240.4e6, "grid": 4.45e6},
+    "two_balls": {"p2g": 105.7e6, "g2p": 245.1e6, "grid": 4.45e6},
 }
 
 
@@ -323,7 +323,7 @@ def traffic_of(family, workload):
 FP32_SOURCE = ("ncu capture of one launch of the kernel in a separate run of this bench on the same workload "
                "(sm__pipe_fma_cycles_active.avg.pct_of_peak_sustained_active / 100)")
 NCU_FP32 = {
-    "two_balls": {"p2g": 0.401, "g2p": 0.447, "grid": 0.048},
+    "two_balls": {"p2g": 0.353, "g2p": 0.445, "grid": 0.066},
 }
 
 

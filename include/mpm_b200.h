@@ -359,7 +359,9 @@ MPM_API mpm_status mpm_solver_stats(mpm_solver* s, mpm_step_stats* out);
  * work is spread over the GPU and never the order of any sum, so every result
  * is bitwise the same for any setting.
  *   g2p_chunk:    particles per G2P work item, MPM_G2P_CHUNK_MIN..MPM_G2P_CHUNK_MAX
- *                 (a grid block's particles are split into items of this size);
+ *                 (a grid block's particles are split into items of this size;
+ *                 until it is set or tuned the engine takes a quarter of the
+ *                 particles per SM, within 256 (linear: 512) and 1024);
  *   p2g_stage:    particles staged per P2G warp pass, 16, 24 or 32 (0: 32);
  *   p2g_warp_max: P2G work items of at most this many particles are taken by
  *                 single warps instead of whole CTAs, 0..MPM_P2G_WARP_MAX_MAX

@@ -2470,7 +2470,7 @@ static void setP2GAttr() {
 }
 
 // Particles staged per warp pass in P2G (16, 24 or 32): the engine's setting
-// (mpm_tuning.p2g_stage, or its choice from the particle density).  Every
+// (mpm_tuning.p2g_stage, else kDefaultP2GStage).  Every
 // size gives bitwise the same sums.
 template <int S, int MODE, int STAGE>
 static void p2gLaunch(const LaunchCtx& c, const StepArgs& a, int want) {

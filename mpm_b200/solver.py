@@ -298,7 +298,7 @@ class _SolverBase:
     # ---- launch settings (no counterpart in the reference) -----------------
     def tuning(self) -> dict:
         """Launch settings of the step kernels: particles per G2P work item,
-        particles staged per P2G pass (0 = chosen from density) and the
+        particles staged per P2G pass (0 = 32) and the
         largest P2G work item taken by a single warp (0 = none, -1 = chosen
         from the item counts)."""
         t = _abi.Tuning()
