@@ -417,7 +417,7 @@ public:
     // (called before the stream is destroyed).
     void releaseScratch() {
         DevMem* all[] = {&solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
-                         &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &range_[0], &range_[1], &emig_count_[0], &emig_count_[1], &emig_, &far_, &arrivals_, &far_count_, &sort_list_, &dense_list_,
+                         &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &range_[0], &range_[1], &emig_count_[0], &emig_count_[1], &emig_, &far_, &arrivals_, &moved_, &sort_list_, &dense_list_,
                          &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_, &tile_done_,
                          &tiles_, &scenes_dev_, &err_, &tmp_, &upload_[0], &upload_[1], &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
         for (DevMem* m : all) m->release();
@@ -990,7 +990,8 @@ public:
             MPM_TRY(grow(keys_[k], sizeof(uint32_t) * nk, "keys"));
             MPM_TRY(grow(vals_[k], sizeof(uint32_t) * nk, "values"));
         }
-        MPM_TRY(grow(sort_scratch_, sizeof(uint32_t) * onesweepScratchWords(nk, key_bits_), "sort scratch"));
+        MPM_TRY(grow(sort_scratch_, sizeof(uint32_t) * std::max(onesweepScratchWords(nk, key_bits_), blockSortScratchWords(nk, key_bits_)),
+                     "sort scratch"));
         // the block sort's lists: per block ranges and emigrant counts (by
         // particle buffer: the compaction clears the next step's counts), per
         // particle emigrants, far movers and the arrivals of crowded blocks
@@ -1001,10 +1002,10 @@ public:
         MPM_TRY(grow(emig_, sizeof(uint2) * nk, "emigrants"));
         MPM_TRY(grow(far_, sizeof(uint2) * nk, "far movers"));
         MPM_TRY(grow(arrivals_, sizeof(unsigned long long) * nk, "arrivals"));
-        MPM_TRY(grow(far_count_, sizeof(uint32_t) * 2, "far mover counts"));
+        MPM_TRY(grow(moved_, sizeof(uint32_t) * 8, "mover counts"));
         for (int k = 0; k < 2; ++k)
             CUDA_TRY(cudaMemsetAsync(emig_count_[k].p, 0, sizeof(uint32_t) * tb, stream_));
-        CUDA_TRY(cudaMemsetAsync(far_count_.p, 0, sizeof(uint32_t) * 2, stream_));
+        CUDA_TRY(cudaMemsetAsync(moved_.p, 0, sizeof(uint32_t) * 8, stream_));
         sort_list_cap_ = (uint32_t)std::min<size_t>(tb, nk);
         MPM_TRY(grow(sort_list_, sizeof(BlockItem) * sort_list_cap_, "block sort list"));
         dense_cap_ = (uint32_t)(nk / kDenseBlock);
@@ -1248,7 +1249,7 @@ public:
         bb.p2g_list_cap = (uint32_t)max_active_;
         bb.block_range = range_[parity_].as<uint2>();
         bb.emig_count = emig_count_[parity_ ^ 1].as<uint32_t>();
-        bb.far_count = far_count_.as<uint32_t>() + (parity_ ^ 1);
+        bb.moved = moved_.as<uint32_t>() + 4 * (parity_ ^ 1);
         bb.sort_list = sort_list_.as<BlockItem>();
         bb.sort_list_cap = sort_list_cap_;
         bb.dense_list = dense_list_.as<BlockItem>();
@@ -1311,13 +1312,16 @@ public:
             b.scenes = scenes_dev_.as<SceneDev>();
             b.nscenes = (int)scenes_.size();
             b.scene_block_base = sbb_.as<uint32_t>();
+            b.n = (uint32_t)ntot_;
+            b.sort_grid = blockSortGrid(sort_list_cap_, num_sms_);
+            b.key_bits = key_bits_;
             b.keys = keys_[kcur_].as<uint32_t>();
             b.prev_keys = keys_[1 - kcur_].as<uint32_t>();
             b.prev_range = range_[parity_ ^ 1].as<uint2>();
             b.emig_count = emig_count_[parity_].as<uint32_t>();
             b.emig = emig_.as<uint2>();
             b.far = far_.as<uint2>();
-            b.far_count = far_count_.as<uint32_t>() + parity_;
+            b.moved = moved_.as<uint32_t>() + 4 * parity_;
             b.list = sort_list_.as<BlockItem>();
             b.list_cap = sort_list_cap_;
             b.dense = dense_list_.as<BlockItem>();
@@ -1327,6 +1331,8 @@ public:
             // emigrant kernel only, which is done by then)
             b.out_keys = keys_[1 - kcur_].as<uint32_t>();
             b.out_perm = vals_[1 - kcur_].as<uint32_t>();
+            b.spare_vals = vals_[kcur_].as<uint32_t>();
+            b.radix_scratch = sort_scratch_.as<uint32_t>();
             b.err = err_.as<uint32_t>();
             // the emigrant lists beside the compaction (in sequence under
             // profiling, so that each family is timed alone)
@@ -1336,7 +1342,7 @@ public:
                 CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
                 CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
             }
-            CUDA_TRY(launchEmigrants(b, ntot_, num_sms_, overlap ? compact_stream_ : stream_));
+            CUDA_TRY(launchEmigrants(b, num_sms_, overlap ? compact_stream_ : stream_));
             if (overlap) CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
             mark(KF_SORT, 1);
             collect(KF_SORT);
@@ -1351,10 +1357,10 @@ public:
                     CUDA_TRY(cudaEventRecord(compact_fork_, stream_));
                     CUDA_TRY(cudaStreamWaitEvent(compact_stream_, compact_fork_, 0));
                 }
-                CUDA_TRY(launchBlockSort(b, dense_cap_, true, num_sms_, overlap ? compact_stream_ : stream_));
+                CUDA_TRY(launchBlockSortDense(b, dense_cap_, num_sms_, overlap ? compact_stream_ : stream_));
                 if (overlap) CUDA_TRY(cudaEventRecord(compact_join_, compact_stream_));
             }
-            CUDA_TRY(launchBlockSort(b, sort_list_cap_, false, num_sms_, stream_));
+            CUDA_TRY(launchBlockSort(b, stream_));
             if (dense_cap_ && overlap) CUDA_TRY(cudaStreamWaitEvent(stream_, compact_join_, 0));
             sorted_ = 1 - kcur_;
         } else {
@@ -2540,7 +2546,7 @@ private:
     size_t ntot_ = 0, max_nodes_ = 0, max_n_ = 0, max_active_ = 1, tile_stride_ = 0;
     uint32_t total_blocks_ = 0;
     int key_bits_ = 1;
-    DevMem keys_[2], vals_[2], sort_scratch_, range_[2], emig_count_[2], emig_, far_, arrivals_, far_count_, sort_list_, dense_list_, compact_scratch_, block_count_, sbb_, active_,
+    DevMem keys_[2], vals_[2], sort_scratch_, range_[2], emig_count_[2], emig_, far_, arrivals_, moved_, sort_list_, dense_list_, compact_scratch_, block_count_, sbb_, active_,
         outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, tmp_, upload_[2], g2p_items_, tmaps_, spans_, p2g_lists_;
     cudaEvent_t upload_free_[2] = {};  // the scene staged in upload_[k] has been written
     int upload_next_ = 0, upload_busy_ = -1;  // the buffer of the next scene; of the scene being added, or -1

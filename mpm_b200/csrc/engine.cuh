@@ -81,11 +81,13 @@ constexpr int kP2GBackWord = kP2GSmallWord + kMaxCombos;
 // [kSortFrontWord], [kSortBackWord], [kSortDenseWord]: entries of the block
 // sort's lists (blocks of at least kBigItem particles from the front, smaller
 // ones from the back; blocks of at least kDenseBlock apart);
+// [kSortRadixWord] .. [+ 7]: tickets of its radix passes;
 // [kSortSchedWord] .. [+ 5]: its work-item schedulers (CTAs, warps, dense).
 constexpr int kSortFrontWord = kP2GBackWord + kMaxCombos;
 constexpr int kSortBackWord = kSortFrontWord + 1;
 constexpr int kSortDenseWord = kSortFrontWord + 2;
-constexpr int kSortSchedWord = kSortFrontWord + 3;
+constexpr int kSortRadixWord = kSortFrontWord + 3;
+constexpr int kSortSchedWord = kSortRadixWord + 8;
 constexpr uint32_t kDenseBlock = 4096;
 constexpr uint32_t kBigItem = 768;
 constexpr uint32_t kWarpAutoMax = 256;

@@ -36,7 +36,7 @@ struct BlockBuffers {
     uint32_t p2g_list_cap;
     uint2* block_range;               // total_blocks: (first sorted particle, count)
     uint32_t* emig_count;             // total_blocks: cleared for the next step
-    uint32_t* far_count;              // likewise
+    uint32_t* moved;                  // likewise
     BlockItem* sort_list;             // see BlockSortArgs
     uint32_t sort_list_cap;
     BlockItem* dense_list;
@@ -62,34 +62,44 @@ cudaError_t exclusiveScan(const T* in, T* out, size_t n, T* partials, T* total, 
 size_t radixTiles(size_t n);
 size_t onesweepScratchWords(size_t n, int bits);
 cudaError_t radixSortOnesweep(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, size_t n,
-                              int bits, uint32_t* scratch, uint32_t* err, bool* result_in_b, cudaStream_t st,
-                              const uint32_t* n_dev = nullptr);
+                              int bits, uint32_t* scratch, uint32_t* err, bool* result_in_b, cudaStream_t st);
 // Block sort (sort.cu): the stable sort of `keys` (live order) given that the
 // live order is the order of the previous sort: launchEmigrants lists the
 // particles that left their blocks (counts zero before), the compaction the
-// occupied blocks with their new ranges, then launchBlockSort sorts.  Output equals radixSortOnesweep's (keys, perm).
+// occupied blocks with their new ranges, then launchBlockSort sorts, block by
+// block or, where many particles left their blocks, by radix passes over all
+// keys.  Output equals radixSortOnesweep's (keys, perm).
 struct BlockSortArgs {
     const SceneDev* scenes;
     int nscenes;
     const uint32_t* scene_block_base;
-    const uint32_t* keys;        // live order
+    uint32_t n;                  // particles
+    unsigned sort_grid;          // blockSortGrid: CTAs of the block sort
+    int key_bits;
+    uint32_t* keys;              // live order (overwritten by the radix passes)
     const uint32_t* prev_keys;   // live order: the previous step's sorted keys
     const uint2* prev_range;     // per block: (first, count) in the live order
     uint32_t* emig_count;        // per block: particles that left it for a neighbouring block
     uint2* emig;                 // (live index, key) of those of block b from prev_range[b].x on
     uint2* far;                  // (live index, key) of the other particles that left their block
-    uint32_t* far_count;
+    uint32_t* moved;             // [0] entries of far, [1] all particles that left their block,
+                                 // [2] blocks that more than kEmigMax left
     const BlockItem* list;       // occupied blocks and their new ranges, full ones from the front,
     uint32_t list_cap;           // the others from the back (kSortFrontWord, kSortBackWord)
     const BlockItem* dense;      // the blocks of at least kDenseBlock particles (kSortDenseWord)
     uint32_t* counters;
     unsigned long long* aux;     // one word per particle: arrivals that exceed shared memory
     uint32_t *out_keys, *out_perm;
+    uint32_t *spare_vals, *radix_scratch;  // of the radix passes: n words, blockSortScratchWords
     uint32_t* err;
 };
-cudaError_t launchEmigrants(const BlockSortArgs& a, size_t n, int num_sms, cudaStream_t st);
-// `dense`: the dense blocks (they may run beside the others, on another stream).
-cudaError_t launchBlockSort(const BlockSortArgs& a, unsigned max_blocks, bool dense, int num_sms, cudaStream_t st);
+size_t blockSortScratchWords(size_t n, int bits);
+unsigned blockSortGrid(unsigned max_blocks, int num_sms);
+cudaError_t launchEmigrants(const BlockSortArgs& a, int num_sms, cudaStream_t st);
+cudaError_t launchBlockSort(const BlockSortArgs& a, cudaStream_t st);
+// The blocks of at least kDenseBlock particles, at most max_blocks of them, or
+// the radix passes (it may run beside launchBlockSort, on another stream).
+cudaError_t launchBlockSortDense(const BlockSortArgs& a, unsigned max_blocks, int num_sms, cudaStream_t st);
 cudaError_t radixSortPairsInto(const uint32_t* in_keys, uint32_t* out_keys, uint32_t* out_vals, uint32_t* tmp_keys,
                                uint32_t* tmp_vals, size_t n, int bits, uint32_t* hist, uint32_t* scan_partials,
                                cudaStream_t st);

@@ -222,7 +222,7 @@ struct CompactArgs {
     uint32_t* p2g_lists;
     uint32_t p2g_list_cap;
     uint2* block_range;
-    uint32_t *emig_count, *far_count;
+    uint32_t *emig_count, *moved;
     BlockItem* sort_list;
     uint32_t sort_list_cap;
     BlockItem* dense_list;
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kCompactThreads) compactOnesweepKernel(Compact
     }
     __syncthreads();
     run += excl_s;
-    if (tile == 0 && threadIdx.x == 0) *a.far_count = 0u;
+    if (tile == 0 && threadIdx.x < 4) a.moved[threadIdx.x] = 0u;
     placeBlocks<kCompactPer>(a, b0, packed, scn, run);
 }
 
@@ -486,7 +486,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
         if (t < 4) a.counters[t] = 0u;
         if (t < kMaxCombos) a.counters[kG2PCountWord + t] = 0u;
         if (t >= kP2GListWord && t < kSortSchedWord) a.counters[t] = 0u;
-        if (t == 0) *a.far_count = 0u;
+        if (t < 4) a.moved[t] = 0u;
     }
     unsigned long long packed[1];
     int scn[1];
@@ -2432,7 +2432,7 @@ void launchCompact(const LaunchCtx& c, const BlockBuffers& bb, uint32_t total_bl
     const CompactArgs a{bb.block_count, total_blocks,     bb.scene_block_base, c.nscenes,        bb.active,
                         bb.outside,     bb.counters,      bb.block_slot,       bb.g2p_items,     bb.g2p_cap,
                         split,          bb.p2g_lists,     bb.p2g_list_cap,     bb.block_range,   bb.emig_count,
-                        bb.far_count,   bb.sort_list,     bb.sort_list_cap,    bb.dense_list,    c.scenes,
+                        bb.moved,       bb.sort_list,     bb.sort_list_cap,    bb.dense_list,    c.scenes,
                         err};
     if (total_blocks <= kClusterBlocks) {
         noteLaunches(1);

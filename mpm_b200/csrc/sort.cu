@@ -205,9 +205,8 @@ constexpr int kLookbackLimit = 1 << 22;
 constexpr int kLookWidth = 8;  // predecessor words read per look-back round trip
 
 __global__ void __launch_bounds__(kThreads) onesweepHistKernel(const uint32_t* __restrict__ keys, uint32_t n,
-                                                                const uint32_t* __restrict__ n_dev, int passes,
-                                                                int bits, uint32_t* __restrict__ ghist) {
-    if (n_dev) n = *n_dev;  // the key count is only known on the device
+                                                                int passes, int bits,
+                                                                uint32_t* __restrict__ ghist) {
     __shared__ uint32_t h[4][256];
     for (int i = threadIdx.x; i < 4 * 256; i += kThreads) (&h[0][0])[i] = 0;
     __syncthreads();
@@ -231,36 +230,27 @@ __global__ void __launch_bounds__(kThreads) onesweepHistKernel(const uint32_t* _
         if ((&h[0][0])[i]) atomicAdd(&ghist[i], (&h[0][0])[i]);
 }
 
-template <bool kIdentVals>
-__global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t* __restrict__ keys_in,
-                                                                const uint32_t* __restrict__ vals_in,
-                                                                uint32_t* __restrict__ keys_out,
-                                                                uint32_t* __restrict__ vals_out, uint32_t n,
-                                                                const uint32_t* __restrict__ n_dev,
-                                                                int shift, uint32_t mask,
-                                                                const uint32_t* __restrict__ ghist,
-                                                                uint32_t* __restrict__ tile_counter,
-                                                                uint32_t* __restrict__ status,
-                                                                uint32_t* __restrict__ err) {
-    __shared__ uint32_t cnt[kWarps][256];
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t tile_s;
-    __shared__ uint32_t tot;
-    for (int i = threadIdx.x; i < kWarps * 256; i += kThreads) (&cnt[0][0])[i] = 0;
-    if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1u);
-    {   // global start of every digit: exclusive scan of this pass's digit counts
-        const uint32_t g = ghist[threadIdx.x];
-        base[threadIdx.x] = blockExclusiveScan(g, &tot);
-    }
-    __syncthreads();
-    const uint32_t tile = tile_s;
-    // With a device-side count the grid covers the largest possible count;
-    // tiles past the actual keys leave at once (later tiles never wait on them).
-    if (n_dev) n = *n_dev;
-    if ((size_t)tile * kSortTile >= n) return;
+template <int NT>
+struct OnesweepSmem {
+    uint32_t cnt[NT / 32][256];
+    uint32_t base[256];
+    uint32_t wtot[8];
+};
+
+// One tile of a pass by a CTA of NT threads: (keys, vals) of the tile to their
+// places by digit (key >> shift) & mask, in the order of the tiles and within
+// the tile.  Every buffer is read past L1: blockSortDenseKernel runs its passes
+// in one launch, where another SM may have written it.
+template <int NT, bool kIdentVals>
+__device__ __forceinline__ void onesweepTile(OnesweepSmem<NT>& m, const uint32_t* keys_in, const uint32_t* vals_in,
+                                             uint32_t* keys_out, uint32_t* vals_out, uint32_t n, uint32_t tile,
+                                             int shift, uint32_t mask, const uint32_t* ghist, uint32_t* status,
+                                             uint32_t* err) {
+    constexpr int W = NT / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const size_t tbase = (size_t)tile * kSortTile + (size_t)warp * 32 * kSortItems;
+    for (int i = threadIdx.x; i < W * 256; i += NT) (&m.cnt[0][0])[i] = 0;
+    const size_t tbase = (size_t)tile * (NT * kSortItems) + (size_t)warp * 32 * kSortItems;
     uint32_t k[kSortItems], v[kSortItems], r[kSortItems];
     // all loads first, so that they are in flight together (the ranking
     // below synchronises the warp after every item)
@@ -268,9 +258,19 @@ __global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t
     for (int j = 0; j < kSortItems; ++j) {
         const size_t i = tbase + (size_t)j * 32 + lane;
         const bool valid = i < n;
-        k[j] = valid ? keys_in[i] : 0u;
-        v[j] = valid ? (kIdentVals ? (uint32_t)i : vals_in[i]) : 0u;
+        k[j] = valid ? __ldcg(keys_in + i) : 0u;
+        v[j] = valid ? (kIdentVals ? (uint32_t)i : __ldcg(vals_in + i)) : 0u;
     }
+    // global start of every digit: exclusive scan of this pass's digit counts
+    uint32_t start = 0;
+    if (threadIdx.x < 256) {
+        const uint32_t g = __ldcg(ghist + threadIdx.x), inc = warpInclusiveScan(g);
+        if (lane == 31) m.wtot[warp] = inc;
+        start = inc - g;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256)
+        for (int w = 0; w < warp; ++w) start += m.wtot[w];
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j) {
         const size_t i = tbase + (size_t)j * 32 + lane;
@@ -278,20 +278,20 @@ __global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t
         const uint32_t d = valid ? (k[j] >> shift) & mask : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
         const int leader = __ffs(peers) - 1;
-        const uint32_t before = valid ? cnt[warp][d] : 0u;
+        const uint32_t before = valid ? m.cnt[warp][d] : 0u;
         r[j] = before + __popc(peers & lt);
         __syncwarp();
-        if (valid && lane == leader) cnt[warp][d] = before + __popc(peers);
+        if (valid && lane == leader) m.cnt[warp][d] = before + __popc(peers);
         __syncwarp();
     }
     __syncthreads();
-    {
+    if (threadIdx.x < 256) {
         const int d = threadIdx.x;
         uint32_t run = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = cnt[w][d];
-            cnt[w][d] = run;
+        for (int w = 0; w < W; ++w) {
+            const uint32_t c = m.cnt[w][d];
+            m.cnt[w][d] = run;
             run += c;
         }
         uint32_t* mine = status + (size_t)tile * 256 + d;
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t
             }
             atomicExch(mine, kFlagPrefix | (excl + run));
         }
-        base[d] += excl;
+        m.base[d] = start + excl;
     }
     __syncthreads();
 #pragma unroll
@@ -341,11 +341,31 @@ __global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t
         const size_t i = tbase + (size_t)j * 32 + lane;
         if (i < n) {
             const uint32_t d = (k[j] >> shift) & mask;
-            const uint32_t pos = base[d] + cnt[warp][d] + r[j];
-            keys_out[pos] = k[j];
-            vals_out[pos] = v[j];
+            const uint32_t pos = m.base[d] + m.cnt[warp][d] + r[j];
+            if (pos < n) {  // (past the end only after a wait that gave up)
+                keys_out[pos] = k[j];
+                vals_out[pos] = v[j];
+            }
         }
     }
+}
+
+template <bool kIdentVals>
+__global__ void __launch_bounds__(kThreads, 4) onesweepPassKernel(const uint32_t* __restrict__ keys_in,
+                                                                const uint32_t* __restrict__ vals_in,
+                                                                uint32_t* __restrict__ keys_out,
+                                                                uint32_t* __restrict__ vals_out, uint32_t n,
+                                                                int shift, uint32_t mask,
+                                                                const uint32_t* __restrict__ ghist,
+                                                                uint32_t* __restrict__ tile_counter,
+                                                                uint32_t* __restrict__ status,
+                                                                uint32_t* __restrict__ err) {
+    __shared__ OnesweepSmem<kThreads> m;
+    __shared__ uint32_t tile_s;
+    if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1u);
+    __syncthreads();
+    onesweepTile<kThreads, kIdentVals>(m, keys_in, vals_in, keys_out, vals_out, n, tile_s, shift, mask, ghist, status,
+                                       err);
 }
 
 __global__ void __launch_bounds__(kThreads) clearRangesKernel(ClearRanges r) {
@@ -384,12 +404,9 @@ size_t onesweepScratchWords(size_t n, int bits) {
 
 // Stable sort of (keys_a, identity values) by the low `bits` bits, one kernel
 // per 8-bit pass.  `scratch` holds onesweepScratchWords(n, bits) words and is
-// cleared here.  `err` receives bit 8 if a look-back wait gave up.  With
-// `n_dev` the sort covers the first *n_dev keys (known on the device only, at
-// most n) and sorts (keys_a, vals_a) pairs instead of identity values.
+// cleared here.  `err` receives bit 8 if a look-back wait gave up.
 cudaError_t radixSortOnesweep(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, size_t n,
-                              int bits, uint32_t* scratch, uint32_t* err, bool* result_in_b, cudaStream_t st,
-                              const uint32_t* n_dev) {
+                              int bits, uint32_t* scratch, uint32_t* err, bool* result_in_b, cudaStream_t st) {
     *result_in_b = false;
     if (n == 0) return cudaSuccess;
     if (n > kCountMask) return cudaErrorInvalidValue;
@@ -409,7 +426,7 @@ cudaError_t radixSortOnesweep(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys
     // 16 keys per thread 0.072 ms for the whole sort, 4 keys 0.065 ms)
     const int hblocks = (int)std::min<size_t>((n + kThreads * 4 - 1) / (kThreads * 4), 148 * 8);
     noteLaunches(1 + passes);
-    onesweepHistKernel<<<hblocks, kThreads, 0, st>>>(keys_a, (uint32_t)n, n_dev, passes, bits, ghist);
+    onesweepHistKernel<<<hblocks, kThreads, 0, st>>>(keys_a, (uint32_t)n, passes, bits, ghist);
     uint32_t *kin = keys_a, *vin = vals_a, *kout = keys_b, *vout = vals_b;
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
@@ -417,12 +434,12 @@ cudaError_t radixSortOnesweep(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys
         if (pass_bits <= 0) pass_bits = 1;
         const uint32_t mask = (1u << pass_bits) - 1u;
         uint32_t* stat = status + (size_t)p * ntiles * 256;
-        if (p == 0 && !n_dev)
-            onesweepPassKernel<true><<<ntiles, kThreads, 0, st>>>(kin, vin, kout, vout, (uint32_t)n, n_dev, shift,
-                                                                  mask, ghist + 256 * p, counters + p, stat, err);
+        if (p == 0)
+            onesweepPassKernel<true><<<ntiles, kThreads, 0, st>>>(kin, vin, kout, vout, (uint32_t)n, shift, mask,
+                                                                  ghist + 256 * p, counters + p, stat, err);
         else
-            onesweepPassKernel<false><<<ntiles, kThreads, 0, st>>>(kin, vin, kout, vout, (uint32_t)n, n_dev, shift,
-                                                                   mask, ghist + 256 * p, counters + p, stat, err);
+            onesweepPassKernel<false><<<ntiles, kThreads, 0, st>>>(kin, vin, kout, vout, (uint32_t)n, shift, mask,
+                                                                   ghist + 256 * p, counters + p, stat, err);
         std::swap(kin, kout);
         std::swap(vin, vout);
         *result_in_b = !*result_in_b;
@@ -514,8 +531,40 @@ cudaError_t radixSortPairsInto(const uint32_t* in_keys, uint32_t* out_keys, uint
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kBsThreads = 256, kBsWarps = kBsThreads / 32;
-constexpr uint32_t kBsFarScan = 4096; // far list read by every block up to this; above, the keys themselves
+// Passes of the radix sort in one launch (see radixOneLaunch).
+__host__ __device__ inline int oddPasses(int bits) { return (bits <= 8 ? 1 : (bits + 7) / 8) | 1; }
+
+constexpr int kBsThreads = 256, kBsWarps = kBsThreads / 32, kBsCtas = 5;  // CTAs per SM
+
+// Small blocks are put together by single warps where there are more of them
+// than the CTAs of blockSortKernel could take two each, else by CTAs as well.
+__device__ __forceinline__ bool smallByCtas(const BlockSortArgs& s) {
+    return s.counters[kSortBackWord] <= 2u * s.sort_grid;
+}
+
+// Whether the step's order is formed by radix passes over all keys instead of
+// block by block.  The block sort is the slower one where many particles leave
+// their blocks: every block reads the whole list of far movers, and an arrival
+// costs more than a particle that stayed (its share of a bitonic sort).  The
+// lines are where the two routes were measured to meet (ms per step, by blocks
+// and by radix):
+//   far movers: of 1M particles, 8 a cell, 2048: 0.394 and 0.421, 4000: 0.433
+//     and 0.431; of 4M, 3 a cell, 2048: 1.384 and 1.581, 4000: 1.667 and 1.669
+//     (reading the whole scene for every block instead: 3.2 and 91);
+//   arrivals a block where single warps sort them: 1M, 8 a cell, 60 of them:
+//     0.317 and 0.327, 115: 0.346 and 0.331, 210: 0.400 and 0.332; 4M, 3 a cell,
+//     45: 1.251 and 1.362, 80: 1.372 and 1.413, 140: 1.519 and 1.441;
+//   where CTAs do: 1M, 35 a cell, 250: 0.257 and 0.274, 500: 0.278 and 0.278, 920:
+//     0.304 and 0.271; 65k, 8 a cell, 210: 0.104 and 0.122, 490: 0.124 and 0.120;
+//   a block that more particles left than shared memory sorts: 250k particles in
+//     8 blocks, one in seven leaving: 0.227 and 0.161; 1M: 0.818 and 0.276.
+constexpr uint32_t kFarMax = 4096, kWarpArrivals = 112, kCtaArrivals = 512, kEmigMax = 8192;
+__device__ __forceinline__ bool sortByRadix(const BlockSortArgs& s) {
+    if (s.n < kDenseBlock) return false;  // (blockSortDenseKernel is not launched)
+    const uint32_t blocks = s.counters[kSortFrontWord] + s.counters[kSortBackWord] + s.counters[kSortDenseWord];
+    return s.moved[0] > kFarMax || s.moved[2] ||
+           s.moved[1] > (unsigned long long)blocks * (smallByCtas(s) ? kCtaArrivals : kWarpArrivals);
+}
 
 __device__ __forceinline__ int blockScene(const uint32_t* base, int nscenes, uint32_t b) {
     int lo = 0, hi = nscenes - 1;
@@ -527,9 +576,17 @@ __device__ __forceinline__ int blockScene(const uint32_t* base, int nscenes, uin
     return lo;
 }
 
-__global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s, uint32_t n) {
+__global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s) {
+    const uint32_t n = s.n;
+    __shared__ uint32_t moved_s;
+    if (threadIdx.x == 0) moved_s = 0u;
+    if (blockIdx.x == 0)  // the radix passes' digit counts
+        for (int i = threadIdx.x; i < oddPasses(s.key_bits) * 256; i += kBsThreads) s.radix_scratch[i] = 0u;
+    __syncthreads();
+    uint32_t moved = 0;
     const uint32_t stride = gridDim.x * kBsThreads * 4;
-    for (uint32_t i0 = (blockIdx.x * kBsThreads + threadIdx.x) * 4; i0 < n; i0 += stride) {
+    const uint32_t n_round = (n + 127) / 128 * 128;  // whole warps iterate together
+    for (uint32_t i0 = (blockIdx.x * kBsThreads + threadIdx.x) * 4; i0 < n_round; i0 += stride) {
         uint32_t key[4], old[4];
         if (i0 + 4 <= n) {  // (the buffers are 256-byte aligned)
             *reinterpret_cast<uint4*>(key) = *reinterpret_cast<const uint4*>(s.keys + i0);
@@ -543,6 +600,8 @@ __global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s, ui
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint32_t home = old[j] >> 6, blk = key[j] >> 6;
+            const unsigned movers = __ballot_sync(0xffffffffu, blk != home);
+            moved += (uint32_t)__popc(movers);
             if (blk == home) continue;
             const SceneDev& sc = s.scenes[blockScene(s.scene_block_base, s.nscenes, home)];
             const uint32_t out = sc.nblocks, lh = home - sc.block_base, lb = blk - sc.block_base;
@@ -554,10 +613,25 @@ __global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s, ui
                 near = abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
             }
             const uint2 e = make_uint2(i0 + j, key[j]);
-            if (near) s.emig[s.prev_range[home].x + atomicAdd(&s.emig_count[home], 1u)] = e;
-            else s.far[atomicAdd(s.far_count, 1u)] = e;
+            // (a warp's particles are neighbours in the sorted order: most of
+            // its movers leave the same block, and share one atomic)
+            const uint32_t list = near ? home : 0xffffffffu;
+            const unsigned peers = __match_any_sync(movers, list);
+            const int leader = __ffs(peers) - 1, lane = threadIdx.x & 31;
+            uint32_t at = 0;
+            if (lane == leader) {
+                const uint32_t c = (uint32_t)__popc(peers);
+                at = atomicAdd(near ? &s.emig_count[home] : &s.moved[0], c);
+                if (near && at <= kEmigMax && at + c > kEmigMax) atomicAdd(&s.moved[2], 1u);
+            }
+            at = __shfl_sync(peers, at, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+            if (near) s.emig[s.prev_range[home].x + at] = e;
+            else s.far[at] = e;
         }
     }
+    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&moved_s, moved);
+    __syncthreads();
+    if (threadIdx.x == 0 && moved_s) atomicAdd(&s.moved[1], moved_s);
 }
 
 // A group of NW warps (a whole CTA, or one warp) that puts blocks together.
@@ -706,49 +780,24 @@ struct BlockSorter {
             auto add = [&](uint32_t slot, uint2 e) {
                 if (slot < A) arr[slot] = ((unsigned long long)(e.y & 63u) << 32) | e.x;
             };
-            const bool ordered = nfar > kBsFarScan;
-            if (ordered) {
-                // many far movers: every particle of the scene, in live order
-                const uint32_t n_round = (sc.n + N - 1) / N * N;
-                uint32_t found = 0;
-                for (uint32_t i = t; i < n_round && found < A; i += N) {
-                    const uint32_t g = sc.key_offset + i;
-                    const uint32_t key = i < sc.n ? s.keys[g] : 0xffffffffu;
-                    const bool hit = i < sc.n && (key >> 6) == blk && g - prev.x >= prev.y;
-                    const unsigned b = __ballot_sync(0xffffffffu, hit);
-                    if (lane == 0) m.wsum[warp] = (uint32_t)__popc(b);
-                    sync();
-                    uint32_t before = 0, all = 0;
+            const uint32_t E = m.nbOff[27], F = E + nfar;
+            for (uint32_t e = t; e < F; e += N) {
+                uint2 v;
+                if (e < E) {
+                    int q = 0;
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        before += w < warp ? m.wsum[w] : 0u;
-                        all += m.wsum[w];
-                    }
-                    if (hit) add(found + before + __popc(b & lt), make_uint2(g, key));
-                    found += all;
-                    sync();
+                    for (int h = 16; h > 0; h >>= 1)
+                        if (q + h < 27 && m.nbOff[q + h] <= e) q += h;
+                    v = s.emig[m.nbStart[q] + (e - m.nbOff[q])];
+                } else {
+                    v = s.far[e - E];
                 }
-                if (t == 0) m.narr = found;
-            } else {
-                const uint32_t E = m.nbOff[27], F = E + nfar;
-                for (uint32_t e = t; e < F; e += N) {
-                    uint2 v;
-                    if (e < E) {
-                        int q = 0;
-#pragma unroll
-                        for (int h = 16; h > 0; h >>= 1)
-                            if (q + h < 27 && m.nbOff[q + h] <= e) q += h;
-                        v = s.emig[m.nbStart[q] + (e - m.nbOff[q])];
-                    } else {
-                        v = s.far[e - E];
-                    }
-                    if ((v.y >> 6) == blk) add(atomicAdd(&m.narr, 1u), v);
-                }
+                if ((v.y >> 6) == blk) add(atomicAdd(&m.narr, 1u), v);
             }
             sync();
             if (t == 0 && (m.narr != A || it.count < stayed)) atomicOr(s.err, ERR_INDEX);  // never expected
             na = min(m.narr, A);
-            if (!(ordered && outside)) sort(arr, na);  // (the outside block has one cell)
+            sort(arr, na);
             for (uint32_t q = t; q < na; q += N) {
                 const uint32_t c = (uint32_t)(arr[q] >> 32), g = (uint32_t)arr[q];
                 atomicAdd(g < prev.x ? &m.arrLo[c] : &m.arrHi[c], 1u);
@@ -795,16 +844,109 @@ struct BlockSorter {
     }
 };
 
-constexpr size_t kBsSmem = std::max(sizeof(BlockSorter<kBsWarps>::Smem), kBsWarps * sizeof(BlockSorter<1>::Smem));
-constexpr size_t kBsDenseSmem = sizeof(BlockSorter<32>::Smem);
+constexpr int kRadixThreads = 1024, kRadixTile = kRadixThreads * kSortItems;
+__device__ __forceinline__ uint32_t radixMask(int bits, int width, int p) {
+    return (1u << min(width, bits - p * width)) - 1u;
+}
 
-__global__ void __launch_bounds__(kBsThreads) blockSortKernel(BlockSortArgs s) {
+// The stable sort of all keys by radix passes in one launch.  Its phases -- count
+// the digits of all passes, then the passes -- are cut into ntiles tickets
+// each, handed out in order; a phase's tickets wait until those of the phase
+// before are done.  A ticket is only ever waited for by later ones, and every
+// earlier one is done or in the hands of a running CTA, so no number of CTAs
+// need be resident; every wait is bounded all the same.  The pass count is odd,
+// so that the last one writes the sorted buffers.
+struct RadixSmem {
+    OnesweepSmem<kRadixThreads> tile;
+    uint32_t ticket;
+};
+__device__ __forceinline__ void radixOneLaunch(const BlockSortArgs& s, RadixSmem& m) {
+    const int passes = oddPasses(s.key_bits), width = (s.key_bits + passes - 1) / passes;
+    const uint32_t ntiles = (s.n + kRadixTile - 1) / kRadixTile;
+    uint32_t *ghist = s.radix_scratch, *status = ghist + passes * 256;
+    uint32_t* ctr = s.counters + kSortRadixWord;  // tickets handed out, tickets done per phase
+    const uint32_t total = (1 + passes) * ntiles;
+    for (;;) {
+        __syncthreads();  // the previous ticket's shared memory is no longer read
+        if (threadIdx.x == 0) {
+            uint32_t ticket = atomicAdd(&ctr[0], 1u);
+            if (ticket >= ntiles && ticket < total) {
+                const volatile uint32_t* done = ctr + ticket / ntiles;  // of the phase before
+                int polls = 0;
+                while (*done < ntiles) {
+                    if (++polls > kLookbackLimit) {  // never expected: give up instead of hanging
+                        atomicOr(s.err, 8u);
+                        ticket = total;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+                __threadfence();
+            }
+            m.ticket = ticket;
+        }
+        __syncthreads();
+        const uint32_t ticket = m.ticket;
+        if (ticket >= total) return;
+        const int phase = (int)(ticket / ntiles);
+        const uint32_t tile = ticket % ntiles;
+        if (phase == 0) {
+            // (emigrantKernel has cleared the digit counts; a tile clears its status words)
+            for (int i = threadIdx.x; i < passes * 256; i += kRadixThreads)
+                status[((size_t)(i >> 8) * ntiles + tile) * 256 + (i & 255)] = 0u;
+            uint32_t* h = &m.tile.cnt[0][0];  // [pass][256]
+            for (int i = threadIdx.x; i < passes * 256; i += kRadixThreads) h[i] = 0u;
+            uint32_t key[kSortItems];
+#pragma unroll
+            for (int j = 0; j < kSortItems; ++j) {
+                const uint32_t i = tile * kRadixTile + j * kRadixThreads + threadIdx.x;
+                key[j] = i < s.n ? __ldcg(s.keys + i) : 0u;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kSortItems; ++j) {
+                const bool valid = tile * kRadixTile + j * kRadixThreads + threadIdx.x < s.n;
+                for (int p = 0; p < passes; ++p) {
+                    const uint32_t d = valid ? (key[j] >> (p * width)) & radixMask(s.key_bits, width, p) : 0xffffffffu;
+                    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+                    if (valid && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&h[p * 256 + d], (uint32_t)__popc(peers));
+                }
+            }
+            __syncthreads();
+            for (int i = threadIdx.x; i < passes * 256; i += kRadixThreads)
+                if (h[i]) atomicAdd(&ghist[i], h[i]);
+        } else {
+            const int p = phase - 1;
+            const uint32_t mask = radixMask(s.key_bits, width, p);
+            uint32_t* st = status + (size_t)p * ntiles * 256;
+            const uint32_t* gh = ghist + p * 256;
+            if (p == 0) {
+                onesweepTile<kRadixThreads, true>(m.tile, s.keys, nullptr, s.out_keys, s.out_perm, s.n, tile, 0, mask, gh,
+                                                  st, s.err);
+            } else {
+                const bool back = p & 1;  // from the output to the spare buffers
+                onesweepTile<kRadixThreads, false>(m.tile, back ? s.out_keys : s.keys, back ? s.out_perm : s.spare_vals,
+                                                   back ? s.keys : s.out_keys, back ? s.spare_vals : s.out_perm, s.n,
+                                                   tile, p * width, mask, gh, st, s.err);
+            }
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) atomicAdd(&ctr[1 + phase], 1u);
+    }
+}
+
+constexpr size_t kBsSmem = std::max(sizeof(BlockSorter<kBsWarps>::Smem), kBsWarps * sizeof(BlockSorter<1>::Smem));
+constexpr size_t kBsDenseSmem = std::max(sizeof(BlockSorter<32>::Smem), sizeof(RadixSmem));
+
+__global__ void __launch_bounds__(kBsThreads, kBsCtas) blockSortKernel(BlockSortArgs s) {
     extern __shared__ unsigned long long bs_smem[];
     __shared__ uint32_t item_s;
+    if (sortByRadix(s)) return;  // blockSortDenseKernel sorts
     const uint32_t nfront = s.counters[kSortFrontWord], nback = s.counters[kSortBackWord];
-    const uint32_t nfar = *s.far_count;
+    const uint32_t nfar = s.moved[0];
     // few small blocks: by CTAs as well, whose latency is a third of a warp's
-    const bool all = nback <= 2 * gridDim.x;
+    const bool all = smallByCtas(s);
     const uint32_t ncta = nfront + (all ? nback : 0u);
     {
         auto& m = *reinterpret_cast<BlockSorter<kBsWarps>::Smem*>(bs_smem);
@@ -840,13 +982,15 @@ __global__ void __launch_bounds__(kBsThreads) blockSortKernel(BlockSortArgs s) {
     }
 }
 
-// Blocks of at least kDenseBlock particles, by CTAs of 1024 threads.
+// Blocks of at least kDenseBlock particles, by CTAs of 1024 threads; or the
+// whole sort by radix passes.
 __global__ void __launch_bounds__(1024, 1) blockSortDenseKernel(BlockSortArgs s) {
     extern __shared__ unsigned long long bs_smem[];
     __shared__ uint32_t item_s;
+    if (sortByRadix(s)) return radixOneLaunch(s, *reinterpret_cast<RadixSmem*>(bs_smem));
     const uint32_t ndense = s.counters[kSortDenseWord];
     if (ndense == 0) return;
-    const uint32_t nfar = *s.far_count;
+    const uint32_t nfar = s.moved[0];
     auto& m = *reinterpret_cast<BlockSorter<32>::Smem*>(bs_smem);
     const BlockSorter<32> g(m, s, threadIdx.x);
     for (;;) {
@@ -859,24 +1003,34 @@ __global__ void __launch_bounds__(1024, 1) blockSortDenseKernel(BlockSortArgs s)
 
 }  // namespace
 
-cudaError_t launchEmigrants(const BlockSortArgs& a, size_t n, int num_sms, cudaStream_t st) {
+unsigned blockSortGrid(unsigned max_blocks, int num_sms) {
+    return std::max(1u, std::min(max_blocks, (unsigned)(num_sms * kBsCtas)));
+}
+
+size_t blockSortScratchWords(size_t n, int bits) {
+    return (size_t)oddPasses(bits) * 256 * ((n + kRadixTile - 1) / kRadixTile + 1);
+}
+
+cudaError_t launchEmigrants(const BlockSortArgs& a, int num_sms, cudaStream_t st) {
     noteLaunches(1);
-    const unsigned grid = (unsigned)std::min<size_t>((n + kBsThreads * 4 - 1) / (kBsThreads * 4), (size_t)num_sms * 8);
-    emigrantKernel<<<std::max(1u, grid), kBsThreads, 0, st>>>(a, (uint32_t)n);
+    const unsigned grid = (unsigned)std::min<size_t>(((size_t)a.n + kBsThreads * 4 - 1) / (kBsThreads * 4), (size_t)num_sms * 8);
+    emigrantKernel<<<std::max(1u, grid), kBsThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launchBlockSort(const BlockSortArgs& a, unsigned max_blocks, bool dense, int num_sms, cudaStream_t st) {
+cudaError_t launchBlockSort(const BlockSortArgs& a, cudaStream_t st) {
     static_assert(kBsSmem <= 47 * 1024, "dynamic shared memory without an attribute");
     noteLaunches(1);
-    if (dense) {
-        const cudaError_t e = cudaFuncSetAttribute(blockSortDenseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)kBsDenseSmem);
-        if (e != cudaSuccess) return e;
-        blockSortDenseKernel<<<std::max(1u, std::min(max_blocks, (unsigned)num_sms)), 1024, kBsDenseSmem, st>>>(a);
-    } else {
-        blockSortKernel<<<std::max(1u, std::min(max_blocks, (unsigned)num_sms * 5u)), kBsThreads, kBsSmem, st>>>(a);
-    }
+    blockSortKernel<<<a.sort_grid, kBsThreads, kBsSmem, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launchBlockSortDense(const BlockSortArgs& a, unsigned max_blocks, int num_sms, cudaStream_t st) {
+    noteLaunches(1);
+    const cudaError_t e =
+        cudaFuncSetAttribute(blockSortDenseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBsDenseSmem);
+    if (e != cudaSuccess) return e;
+    blockSortDenseKernel<<<std::max(1u, std::min(max_blocks, (unsigned)num_sms)), 1024, kBsDenseSmem, st>>>(a);
     return cudaGetLastError();
 }
 
