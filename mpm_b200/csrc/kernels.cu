@@ -22,6 +22,7 @@
 #include "engine_host.hpp"
 #include "mpm_math.cuh"
 #include "particle_common.cuh"
+#include "per_device.hpp"
 
 #include <atomic>
 #include <cstdlib>
@@ -2459,14 +2460,14 @@ void launchStress(const LaunchCtx& c, int parity) {
     stressKernel<<<dim3(c.particle_blocks, c.nscenes), kThreads, 0, c.stream>>>(c.scenes, parity);
 }
 
-template <int S, int MODE, int STAGE>
-static void setP2GAttr() {
-    static bool done = false;
-    if (!done) {
-        cudaFuncSetAttribute(p2gKernel<S, MODE, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)P2GLayout<S, MODE, STAGE>::smemBytes);
-        done = true;
-    }
+// Raises a kernel's limit of dynamic shared memory on the current device.  A
+// failure stays the last error, which the caller's check after the launch reports.
+template <auto Kernel>
+static void allowSharedMemory(size_t bytes) {
+    static OncePerDevice once;
+    int device = 0;
+    cudaGetDevice(&device);
+    once(device, [&] { return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 // Particles staged per warp pass in P2G (16, 24 or 32): the engine's setting
@@ -2474,7 +2475,7 @@ static void setP2GAttr() {
 // size gives bitwise the same sums.
 template <int S, int MODE, int STAGE>
 static void p2gLaunch(const LaunchCtx& c, const StepArgs& a, int want) {
-    setP2GAttr<S, MODE, STAGE>();
+    allowSharedMemory<p2gKernel<S, MODE, STAGE>>(P2GLayout<S, MODE, STAGE>::smemBytes);
     p2gKernel<S, MODE, STAGE><<<c.persistent_blocks, P2GLayout<S, MODE, STAGE>::NT, P2GLayout<S, MODE, STAGE>::smemBytes,
                                 c.stream>>>(a, want);
 }
@@ -2491,11 +2492,7 @@ static void p2gOne(const LaunchCtx& c, const StepArgs& a, int want) {
 template <int S, int MODE>
 static void p2gWarpLaunch(const LaunchCtx& c, const StepArgs& a) {
     using W = P2GWarpLayout<S, MODE>;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(p2gWarpKernel<S, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::smemBytes);
-        attr = true;
-    }
+    allowSharedMemory<p2gWarpKernel<S, MODE>>(W::smemBytes);
     const unsigned grid = std::min<unsigned>(c.persistent_blocks, (unsigned)std::max(1, c.num_sms) * W::MIN_CTAS);
     p2gWarpKernel<S, MODE><<<grid, W::NT, W::smemBytes, c.stream>>>(a);
 }
@@ -2542,11 +2539,7 @@ void launchGrid(const LaunchCtx& c, const StepArgs& a, int S, int mode, int want
 constexpr size_t kG2PDynSmem = sizeof(float) * 2 * kG2PThreads * kPreStride;
 template <int S, bool APIC>
 static void g2pLaunch(const LaunchCtx& c, const StepArgs& a, int fused) {
-    static bool attr = [] {
-        cudaFuncSetAttribute(g2pKernel<S, APIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG2PDynSmem);
-        return true;
-    }();
-    (void)attr;
+    allowSharedMemory<g2pKernel<S, APIC>>(kG2PDynSmem);
     g2pKernel<S, APIC><<<(c.persistent_blocks * 256 + kG2PThreads - 1) / kG2PThreads, kG2PThreads, kG2PDynSmem, c.stream>>>(a, fused);
 }
 
