@@ -1084,6 +1084,7 @@ public:
         warp_check_ = true;
         warp_pending_ = false;  // a read-back issued before the sync above is stale
         for (bool& f : warp_few_) f = false;  // the new set's small items: decided on the device until read back
+        crowded_ = false;
         any_implicit_ = false;
         for (auto& s : scenes_) any_implicit_ |= s->beta > 0.f;
         MPM_TRY(ensureSolveBuffers());
@@ -1292,7 +1293,7 @@ public:
         // The block sort serves when the live order is the last sorted order
         // and the keys are G2P's (the particles have moved by one step): every
         // step but the first after an upload or a split call.
-        const bool by_blocks = incremental_ok_ && keys_valid_ && !full_sort_only_;
+        const bool by_blocks = incremental_ok_ && keys_valid_ && !full_sort_only_ && !crowded_;
         if (!keys_valid_) {
             mark(KF_KEYS, 0);
             CUDA_TRY(cudaMemsetAsync(block_count_.p, 0, sizeof(uint32_t) * total_blocks_, stream_));
@@ -1942,8 +1943,9 @@ public:
     }
 
     // Whether any combination has too few small P2G items for the warp kernel,
-    // so that its launch can be skipped: decided once after the first step
-    // that follows a change of the scene set, from that step's counts.  They
+    // so that its launch can be skipped, and whether a block is too crowded for
+    // the block sort: decided once after the first step that follows a change of
+    // the scene set, from that step's counts.  They
     // are read back asynchronously (a copy into pinned host memory and an
     // event), so the host does not wait for the GPU: the steps that follow
     // run with direct launches until the event has completed, and only then
@@ -1962,9 +1964,10 @@ public:
                 if (!host_word_) return fail(MPM_ERR_OOM, "no page-locked host word for the item-count read-back");
                 CUDA_TRY(cudaEventCreateWithFlags(&warp_event_, cudaEventDisableTiming));
             }
-            static_assert(kMaxCombos <= PinnedWords::kLine, "read-back line too short");
+            static_assert(kMaxCombos + 1 <= PinnedWords::kLine && kSortMaxWord == kP2GSmallWord + kMaxCombos,
+                          "read-back line too short");
             CUDA_TRY(cudaMemcpyAsync(host_word_, counters_.as<uint32_t>() + kP2GSmallWord,
-                                     sizeof(uint32_t) * kMaxCombos, cudaMemcpyDeviceToHost, stream_));
+                                     sizeof(uint32_t) * (kMaxCombos + 1), cudaMemcpyDeviceToHost, stream_));
             CUDA_TRY(cudaEventRecord(warp_event_, stream_));
             warp_pending_ = true;
             return MPM_OK;
@@ -1982,6 +1985,9 @@ public:
             changed |= few != warp_few_[k];
             warp_few_[k] = few;
         }
+        const bool crowded = crowdedBlock(host_word_[kMaxCombos], ntot_, key_bits_);
+        changed |= crowded != crowded_;
+        crowded_ = crowded;
         if (changed) dropGraphs();
         return MPM_OK;
     }
@@ -2554,6 +2560,8 @@ private:
     // fewer than kWarpAutoMinItems small P2G items, so the step does not
     // launch the warp kernel (see checkWarpItems, warpModeOf).
     bool warp_few_[kMaxCombos] = {};
+    // The same step found a crowded block: no block sort (see crowdedBlock).
+    bool crowded_ = false;
     bool profiling_ = false;
     bool step_timing_ = false;
     std::deque<std::pair<cudaEvent_t, cudaEvent_t>> step_events_;

@@ -73,11 +73,14 @@ constexpr int kP2GListWord = 64;
 // [kP2GSmallWord + k]: P2G items of combination k of at most kWarpAutoMax
 // particles (read back to decide the warp threshold when it is not set).
 constexpr int kP2GSmallWord = kP2GListWord + 2 * kMaxCombos;
+// [kSortMaxWord]: particles of the fullest block of at least kDenseBlock (0: none;
+// read back with the small items, see crowdedBlock).
+constexpr int kSortMaxWord = kP2GSmallWord + kMaxCombos;
 // The CTA list (c = 1) of combination k holds its items of at least
 // kBigItem particles from the front (counters[kP2GListWord + 2k + 1] of
 // them) and the others from the back (counters[kP2GBackWord + k]), so that
 // the CTAs take the long items first and the short ones fill the tail.
-constexpr int kP2GBackWord = kP2GSmallWord + kMaxCombos;
+constexpr int kP2GBackWord = kSortMaxWord + 1;
 // [kSortFrontWord], [kSortBackWord], [kSortDenseWord]: entries of the block
 // sort's lists (blocks of at least kBigItem particles from the front, smaller
 // ones from the back; blocks of at least kDenseBlock apart);
@@ -89,6 +92,24 @@ constexpr int kSortDenseWord = kSortFrontWord + 2;
 constexpr int kSortRadixWord = kSortFrontWord + 3;
 constexpr int kSortSchedWord = kSortRadixWord + 8;
 constexpr uint32_t kDenseBlock = 4096;
+// Whether a block of `count` particles of `total` in the batch is crowded: one
+// CTA puts it together, in time linear in its count, while the radix sort's time
+// goes with the total and the passes, so above a line that grows with both every
+// step sorts all keys by the radix sort.  Decided from the first step's counts
+// after a change of the scene set.  ms per step, block sort and radix sort, with
+// keys of up to 16 bits (2 passes: 32^3 grid), 24 (128^3) and more (320^3):
+//   one block, 8k: 0.073 and 0.067, 0.074 and 0.074, 0.081 and 0.086; 32k: 0.094 and
+//     0.080, 0.093 and 0.082, 0.103 and 0.101; 1M: 0.748 and 0.372, 0.747 and
+//     0.378, 0.750 and 0.394;
+//   8 blocks, 16k each: 0.095 and 0.083, 0.095 and 0.090, 0.105 and 0.109; 125k each:
+//     0.279 and 0.218, 0.278 and 0.238, 0.281 and 0.260;
+//   27 blocks, 37k each: 0.222 and 0.208, 0.220 and 0.225, 0.233 and 0.250;
+//   64 blocks, 31k each: 0.345 and 0.350, 0.343 and 0.378, 0.353 and 0.411;
+//   1M particles on 128^3, 100k of them in a block and the others spread, 1.251 and
+//     1.250, 250k 1.304 and 1.244; 4M and 250k 1.647 and 1.660.
+__host__ __device__ inline bool crowdedBlock(uint32_t count, size_t total, int key_bits) {
+    return count > (key_bits > 24 ? 4 * kDenseBlock : kDenseBlock) + total / (key_bits > 16 ? 16 : 64);
+}
 constexpr uint32_t kBigItem = 768;
 constexpr uint32_t kWarpAutoMax = 256;
 constexpr uint32_t kWarpAutoMinItems = 1024;

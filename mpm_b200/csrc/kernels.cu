@@ -349,8 +349,10 @@ __device__ __forceinline__ void placeBlocks(const CompactArgs& a, uint32_t b0, c
         a.emig_count[b] = 0u;
         if (count) {
             const BlockItem e{b, start, count, (uint32_t)scene};
-            if (count >= kDenseBlock) a.dense_list[cnext[7]++] = e;
-            else if (count >= kBigItem) a.sort_list[cnext[5]++] = e;
+            if (count >= kDenseBlock) {
+                a.dense_list[cnext[7]++] = e;
+                atomicMax(&a.counters[kSortMaxWord], count);
+            } else if (count >= kBigItem) a.sort_list[cnext[5]++] = e;
             else a.sort_list[a.sort_list_cap - 1 - cnext[6]++] = e;
         }
         // a block's items have count / items particles, the first

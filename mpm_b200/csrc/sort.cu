@@ -526,8 +526,7 @@ cudaError_t radixSortPairsInto(const uint32_t* in_keys, uint32_t* out_keys, uint
 // compaction per step, against the radix sort: 65k-particle cube 0.033 -> 0.023
 // ms, two-ball scene (1M) 0.064 -> 0.040 ms, 2M particles 0.090 -> 0.054 ms, and
 // against a sort of the particles that changed cells and a merge: slab (8.4M)
-// 0.19 -> 0.11 ms.  Six scenes of up to 60k particles in a few cells each lose
-// 0.006 ms of 0.123 (their crowded blocks are put together by one CTA each).
+// 0.19 -> 0.11 ms.  Crowded blocks (crowdedBlock) are left to the radix sort.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -558,11 +557,16 @@ __device__ __forceinline__ bool smallByCtas(const BlockSortArgs& s) {
 //     0.304 and 0.271; 65k, 8 a cell, 210: 0.104 and 0.122, 490: 0.124 and 0.120;
 //   a block that more particles left than shared memory sorts: 250k particles in
 //     8 blocks, one in seven leaving: 0.227 and 0.161; 1M: 0.818 and 0.276.
-constexpr uint32_t kFarMax = 4096, kWarpArrivals = 112, kCtaArrivals = 512, kEmigMax = 8192;
+//   a block that became crowded after the route of its scene was chosen (see
+//     crowdedBlock): one block of 65k 0.119 and 0.118, 100k 0.134 and 0.122, 250k
+//     0.236 and 0.179; 8 of 62k 0.174 and 0.179, 250k 0.487 and 0.446; 1M particles,
+//     100k of them in a block, 1.251 and 1.264, 250k 1.304 and 1.263; 4M, 250k: 1.647
+//     and 1.733.
+constexpr uint32_t kFarMax = 4096, kWarpArrivals = 112, kCtaArrivals = 512, kEmigMax = 8192, kCrowdedMax = 65536;
 __device__ __forceinline__ bool sortByRadix(const BlockSortArgs& s) {
     if (s.n < kDenseBlock) return false;  // (blockSortDenseKernel is not launched)
     const uint32_t blocks = s.counters[kSortFrontWord] + s.counters[kSortBackWord] + s.counters[kSortDenseWord];
-    return s.moved[0] > kFarMax || s.moved[2] ||
+    return s.moved[0] > kFarMax || s.moved[2] || s.counters[kSortMaxWord] > kCrowdedMax + s.n / 13 ||
            s.moved[1] > (unsigned long long)blocks * (smallByCtas(s) ? kCtaArrivals : kWarpArrivals);
 }
 
