@@ -279,10 +279,15 @@ static PinnedWords g_pinned_words;
 // ---------------------------------------------------------------------------
 // Tuning cache of the autotuner: launch settings per (device, stencil size,
 // transfer, particles-per-cell bucket), kept for the process and in a text
-// file ("<device> <S> <transfer> <bucket> <g2p_chunk> <p2g_stage>" per line;
-// the last line of a key wins).
+// file ("v<version> <device> <S> <transfer> <bucket> <g2p_chunk> <p2g_stage>
+// <p2g_warp_max>" per line; the last line of a key wins).  An entry holds for
+// the kernels that it was measured on: kVersion goes up when P2G or G2P change
+// so that other settings may be the faster ones, and lines of another version
+// are skipped (p2g_stage 16, chosen for the P2G that summed single cells, cost
+// the one that sums rows 0.128 ms instead of 0.099 on two balls of 0.5M).
 // ---------------------------------------------------------------------------
 struct TuneCache {
+    static constexpr int kVersion = 2;
     std::mutex mu;
     std::map<std::string, mpm_tuning> entries;
     bool loaded = false;
@@ -305,13 +310,12 @@ struct TuneCache {
         if (p.empty()) return;
         FILE* f = fopen(p.c_str(), "r");
         if (!f) return;
-        // one entry per line; lines of an older format (fewer values) are
-        // skipped, so their keys are tuned again
+        // one entry per line; the keys of skipped lines are tuned again
         char line[512], dev[256];
-        int S, tr, bucket, chunk, stage, warp;
+        int version, S, tr, bucket, chunk, stage, warp;
         while (fgets(line, sizeof(line), f))
-            if (sscanf(line, "%255s %d %d %d %d %d %d", dev, &S, &tr, &bucket, &chunk, &stage, &warp) == 7 &&
-                chunk >= (int)kMinG2PChunk && chunk <= (int)kMaxG2PChunk && (stage == 16 || stage == 24 || stage == 32) &&
+            if (sscanf(line, "v%d %255s %d %d %d %d %d %d", &version, dev, &S, &tr, &bucket, &chunk, &stage, &warp) == 8 &&
+                version == kVersion && chunk >= (int)kMinG2PChunk && chunk <= (int)kMaxG2PChunk && (stage == 16 || stage == 24 || stage == 32) &&
                 warp >= -1 && warp <= MPM_P2G_WARP_MAX_MAX)
                 entries[key(dev, S, tr, bucket)] = mpm_tuning{chunk, stage, warp};
         fclose(f);
@@ -325,7 +329,7 @@ struct TuneCache {
         for (size_t i = 1; i < p.size(); ++i)
             if (p[i] == '/') mkdir(p.substr(0, i).c_str(), 0755);
         if (FILE* f = fopen(p.c_str(), "a")) {
-            fprintf(f, "%s %d %d %d\n", k.c_str(), t.g2p_chunk, t.p2g_stage, t.p2g_warp_max);
+            fprintf(f, "v%d %s %d %d %d\n", kVersion, k.c_str(), t.g2p_chunk, t.p2g_stage, t.p2g_warp_max);
             fclose(f);
         }
     }
