@@ -2148,11 +2148,13 @@ public:
         if (!out) return fail(MPM_ERR_INVALID_ARG, "null output");
         *out = mpm_step_stats{};
         if (dirty_ || !counters_.p) return MPM_OK;
-        uint32_t c[4] = {0, 0, 0, 0};
+        uint32_t c[kCounterWords];
         CUDA_TRY(cudaStreamSynchronize(stream_));
         CUDA_TRY(cudaMemcpy(c, counters_.p, sizeof(c), cudaMemcpyDeviceToHost));
-        out->active_blocks = c[0];
-        out->outside_blocks = c[1];
+        // every block that holds particles is in one of the block sort's lists,
+        // the block of a scene's outside particles too
+        out->active_blocks = c[kSortFrontWord] + c[kSortBackWord] + c[kSortDenseWord] - c[3];
+        out->outside_blocks = c[3];
         out->active_nodes = c[2];
         return MPM_OK;
     }

@@ -62,8 +62,9 @@ constexpr uint32_t kMinG2PChunk = 256;
 constexpr uint32_t kMaxG2PChunk = 4096;
 constexpr uint32_t kDefaultG2PChunk = 1024;
 // Counter words: [0] work items, [1] outside items, [2] nodes with mass,
-// [8 + 8k .. 13 + 8k] work-item schedulers of combination k (k < 6),
-// [kG2PCountWord + k] G2P items of combination k.
+// [3] scenes with particles outside their grid, [8 + 8k .. 13 + 8k] work-item
+// schedulers of combination k (k < 6), [kG2PCountWord + k] G2P items of
+// combination k.
 constexpr int kMaxCombos = 6;
 constexpr int kG2PCountWord = 56;
 // [kP2GListWord + 2k + c]: P2G items of combination k in its list c (0: items

@@ -397,6 +397,7 @@ __device__ __forceinline__ void placeBlocks(const CompactArgs& a, uint32_t b0, c
             if (count > 0) {
                 const uint32_t nitems = blockItems(count, a.scenes[scene].n);
                 const uint32_t o = atomicAdd(&a.counters[1], nitems);
+                atomicAdd(&a.counters[3], 1u);
                 splitItems(a.outside + o, b, start, count, nitems, (uint32_t)scene);
             }
         }
