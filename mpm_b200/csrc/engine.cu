@@ -403,7 +403,15 @@ public:
         if (m.p && m.bytes >= b) return MPM_OK;
         return alloc(m, std::max(b, m.bytes + m.bytes / 2), what);
     }
-    // The upload buffers stay with the engine between scenes: given back at
+    // Marks the end of a use of an upload buffer in the engine's stream: the next
+    // scene's copies into it, on their own stream, wait for it.
+    struct StagingUse {
+        cudaEvent_t free;
+        cudaStream_t stream;
+        ~StagingUse() { cudaEventRecord(free, stream); }
+    };
+    // The upload buffers stay with the engine between scenes (the first one
+    // stages the blocking downloads and uploads of fields as well): given back at
     // each rebuild, the step's scratch took their memory and the next
     // construction waited for the pool to map more (one of ten two-ball
     // constructions 4 to 15 ms instead of 1.0).  Where memory runs out they
@@ -423,7 +431,7 @@ public:
         DevMem* all[] = {&solve_pofs_, &solve_prep_, &solve_T_, &solve_iter_,
                          &keys_[0], &keys_[1], &vals_[0], &vals_[1], &sort_scratch_, &range_[0], &range_[1], &emig_count_[0], &emig_count_[1], &emig_, &far_, &arrivals_, &moved_, &sort_list_, &dense_list_,
                          &compact_scratch_, &block_count_, &sbb_, &active_, &outside_, &counters_, &block_slot_, &tile_done_,
-                         &tiles_, &scenes_dev_, &err_, &tmp_, &upload_[0], &upload_[1], &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
+                         &tiles_, &scenes_dev_, &err_, &upload_[0], &upload_[1], &g2p_items_, &tmaps_, &spans_, &p2g_lists_};
         for (DevMem* m : all) m->release();
     }
 
@@ -2305,11 +2313,12 @@ public:
             return fail(MPM_ERR_INVALID_ARG, "B is only defined for APIC scenes");
         if (s.n == 0) return MPM_OK;
         const size_t bytes = sizeof(float) * per * s.n;
-        MPM_TRY(alloc(tmp_, bytes, "download buffer"));
+        MPM_TRY(alloc(upload_[0], bytes, "download buffer"));
+        StagingUse use{upload_free_[0], stream_};
         LaunchCtx c = ctx();
-        launchGatherField(c, idx, parity_, base, comps, mode, tmp_.as<float>());
+        launchGatherField(c, idx, parity_, base, comps, mode, upload_[0].as<float>());
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(host, tmp_.p, bytes, cudaMemcpyDeviceToHost, stream_));
+        CUDA_TRY(cudaMemcpyAsync(host, upload_[0].p, bytes, cudaMemcpyDeviceToHost, stream_));
         if (sync) return synchronize();
         return MPM_OK;
     }
@@ -2392,10 +2401,11 @@ public:
         // cell_vol_inv as the reference forms it: 1.0 / (h*h*h) in double, stored as float
         const float h = s.desc.stride;
         const float inv = (float)(1.0 / (double)(h * h * h));
-        MPM_TRY(grow(tmp_, sizeof(float) * nodes, "density buffer"));
-        launchDensity(ctx(), s.vstar.as<float4>(), nodes, inv, tmp_.as<float>());
+        MPM_TRY(grow(upload_[0], sizeof(float) * nodes, "density buffer"));
+        StagingUse use{upload_free_[0], stream_};
+        launchDensity(ctx(), s.vstar.as<float4>(), nodes, inv, upload_[0].as<float>());
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(host, tmp_.p, sizeof(float) * nodes, cudaMemcpyDeviceToHost, stream_));
+        CUDA_TRY(cudaMemcpyAsync(host, upload_[0].p, sizeof(float) * nodes, cudaMemcpyDeviceToHost, stream_));
         return synchronize();
     }
 
@@ -2411,9 +2421,10 @@ public:
         SceneHost& s = *scenes_[idx];
         if (s.n == 0) return MPM_OK;
         const size_t bytes = sizeof(float) * per * s.n;
-        MPM_TRY(alloc(tmp_, bytes, "upload buffer"));
-        CUDA_TRY(cudaMemcpyAsync(tmp_.p, host, bytes, cudaMemcpyHostToDevice, stream_));
-        launchScatterField(ctx(), idx, parity_, base, comps, tmp_.as<float>());
+        MPM_TRY(alloc(upload_[0], bytes, "upload buffer"));
+        StagingUse use{upload_free_[0], stream_};
+        CUDA_TRY(cudaMemcpyAsync(upload_[0].p, host, bytes, cudaMemcpyHostToDevice, stream_));
+        launchScatterField(ctx(), idx, parity_, base, comps, upload_[0].as<float>());
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaStreamSynchronize(stream_));
         s.stress_stale = true;
@@ -2559,7 +2570,7 @@ private:
     uint32_t total_blocks_ = 0;
     int key_bits_ = 1;
     DevMem keys_[2], vals_[2], sort_scratch_, range_[2], emig_count_[2], emig_, far_, arrivals_, moved_, sort_list_, dense_list_, compact_scratch_, block_count_, sbb_, active_,
-        outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, tmp_, upload_[2], g2p_items_, tmaps_, spans_, p2g_lists_;
+        outside_, counters_, block_slot_, tiles_, tile_done_, scenes_dev_, err_, upload_[2], g2p_items_, tmaps_, spans_, p2g_lists_;
     cudaEvent_t upload_free_[2] = {};  // the scene staged in upload_[k] has been written
     int upload_next_ = 0, upload_busy_ = -1;  // the buffer of the next scene; of the scene being added, or -1
     // Per combination: the first step after a change of the scene set found
