@@ -31,8 +31,10 @@ FIELDS_OUT = (_abi.FIELD_POSITION, _abi.FIELD_VELOCITY, _abi.FIELD_DET_FE, _abi.
 def scene_device_bytes(scene) -> int:
     """Device memory a scene holds while admitted: two particle buffers (41
     float planes, id, material), the dense grid (v*, and v for PIC-FLIP), its
-    share of the batch's sort buffers and block tables, and P2G tiles for its
-    blocks (bounded by its particle count)."""
+    share of the batch's sort buffers, block tables and work-item lists, P2G
+    tiles for its work items (a block's, bounded by the particle count, and one
+    for every further split of its particles) and the buffer that staged its
+    upload, which stays with the engine."""
     n = scene.n
     res = scene.resolution
     nodes = int(res[0]) * int(res[1]) * int(res[2])
@@ -41,11 +43,21 @@ def scene_device_bytes(scene) -> int:
     flip = scene.transfer == _abi.TRANSFER_PIC_FLIP
     particles = 2 * n * (41 * 4 + 4 + 2)
     grid = nodes * 16 * (2 if flip else 1)
-    sort = n * (16 + 24) + (n + 2047) // 2048 * 256 * 4 * 2  # keys and permutations, the block sort's lists, radix scratch
-    tables = blocks * (4 + 8 + 8 + 4)
+    # keys and permutations (16), emigrants, far movers and arrivals (24); the
+    # digit tables of at most 5 radix passes
+    sort = n * (16 + 24) + (n + 2047) // 2048 * 256 * 4 * 5
+    # counts (4), slots (8), two ranges (16) and two emigrant counts (8)
+    tables = blocks * 36
+    occupied = min(blocks, max(n, 1))
+    items = occupied + n // (640 if n <= 65536 else 1280) + 1
+    # per P2G item: the item and the outside one (32), tile count (4) and two
+    # list entries (8) of each of 6 combinations; per G2P item 16 for each; per
+    # occupied block an entry of the sort's list
+    lists = items * (32 + 4 + 8 * 6) + (occupied + n // 256 + 1) * 16 * 6 + occupied * 16
     S = {0: 2, 1: 3, 2: 4}[scene.interpolation]
-    tiles = min(blocks, max(n, 1)) * 7 * (S + 3) ** 3 * 4
-    return particles + grid + sort + tables + tiles
+    tiles = items * 7 * (S + 3) ** 3 * 4
+    staging = n * 34  # x, v, m, V0 and a 16-bit material
+    return particles + grid + sort + tables + lists + tiles + staging
 
 
 @dataclass
