@@ -20,7 +20,7 @@ struct LaunchCtx {
     unsigned node_blocks;       // grid.x of dense per-node kernels
     unsigned persistent_blocks; // grid of the persistent block kernels
     int num_sms;
-    int p2g_stage;              // particles staged per warp pass in P2G (16, 24 or 32)
+    int p2g_stage;              // particles staged per warp pass in the fused step's P2G (16, 24 or 32)
 };
 
 struct BlockBuffers {
@@ -168,7 +168,6 @@ void launchCfl(const LaunchCtx& c, int parity, size_t max_n, uint32_t* err);
 void launchGatherField(const LaunchCtx& c, int scene, int parity, int field, int comps, int mode, float* out);
 void preloadTransferKernels();
 void launchScatterField(const LaunchCtx& c, int scene, int parity, int field, int comps, const float* in);
-size_t p2gSmemBytes(int S, int mode);
 // Writes the kTensorMapBytes TMA tensor map of a dense float4 grid (res[3]
 // nodes) with tile box T^3 to map (host memory); returns null or a message.
 const char* encodeGridTensorMap(void* map, const void* grid, const int* res, int T);

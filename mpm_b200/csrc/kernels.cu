@@ -1036,7 +1036,7 @@ __device__ __forceinline__ void findRows(const uint32_t* keys, int count, int* b
     }
 }
 
-template <int S, int MODE, int STAGE = 16>
+template <int S, int MODE, int STAGE>
 struct P2GLayout : P2GStage<S, MODE> {
     using R = P2GStage<S, MODE>;
     static constexpr int F = R::F, T = R::T;
@@ -2473,9 +2473,9 @@ static void allowSharedMemory(size_t bytes) {
     once(device, [&] { return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
-// Particles staged per warp pass in P2G (16, 24 or 32): the engine's setting
-// (mpm_tuning.p2g_stage, else kDefaultP2GStage).  Every
-// size gives bitwise the same sums.
+// Particles staged per warp pass in P2G: in the fused step the engine's setting
+// (16, 24 or 32: mpm_tuning.p2g_stage, else kDefaultP2GStage), elsewhere
+// kDefaultP2GStage.  Every size gives bitwise the same sums.
 template <int S, int MODE, int STAGE>
 static void p2gLaunch(const LaunchCtx& c, const StepArgs& a, int want) {
     allowSharedMemory<p2gKernel<S, MODE, STAGE>>(P2GLayout<S, MODE, STAGE>::smemBytes);
@@ -2515,9 +2515,9 @@ void launchP2G(const LaunchCtx& c, const StepArgs& a, int S, int mode, int want_
         switch (mode) {                                                                \
             case MODE_APIC_FUSED: p2gOne<SS, MODE_APIC_FUSED>(c, a, want_transfer); break; \
             case MODE_FLIP: p2gOne<SS, MODE_FLIP>(c, a, want_transfer); break;         \
-            case MODE_SPLIT: p2gOne<SS, MODE_SPLIT>(c, a, want_transfer); break;       \
-            case MODE_HESS: p2gLaunch<SS, MODE_HESS, 32>(c, a, want_transfer); break;  \
-            default: p2gOne<SS, MODE_MASS>(c, a, want_transfer); break;                \
+            case MODE_SPLIT: p2gLaunch<SS, MODE_SPLIT, kDefaultP2GStage>(c, a, want_transfer); break; \
+            case MODE_HESS: p2gLaunch<SS, MODE_HESS, kDefaultP2GStage>(c, a, want_transfer); break;   \
+            default: p2gLaunch<SS, MODE_MASS, kDefaultP2GStage>(c, a, want_transfer); break;          \
         }                                                                              \
     }
     P2G_CASE(2) P2G_CASE(3) P2G_CASE(4)
@@ -2724,21 +2724,6 @@ const char* encodeGridTensorMap(void* map, const void* grid, const int* res, int
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled rejected the grid tensor map";
-}
-
-size_t p2gSmemBytes(int S, int mode) {
-#define SM_CASE(SS)                                                          \
-    if (S == SS) {                                                           \
-        switch (mode) {                                                      \
-            case MODE_APIC_FUSED: return P2GLayout<SS, MODE_APIC_FUSED>::smemBytes; \
-            case MODE_FLIP: return P2GLayout<SS, MODE_FLIP>::smemBytes;       \
-            case MODE_SPLIT: return P2GLayout<SS, MODE_SPLIT>::smemBytes;     \
-            default: return P2GLayout<SS, MODE_MASS>::smemBytes;              \
-        }                                                                    \
-    }
-    SM_CASE(2) SM_CASE(3) SM_CASE(4)
-#undef SM_CASE
-    return 0;
 }
 
 }  // namespace mpm
