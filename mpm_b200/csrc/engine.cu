@@ -1038,9 +1038,7 @@ public:
         MPM_TRY(grow(g2p_items_, sizeof(BlockItem) * g2p_cap_ * (size_t)combos().size(), "G2P items"));
         // P2G's two lists of item slots per combination (warp items, CTA items)
         MPM_TRY(grow(p2g_lists_, sizeof(uint32_t) * max_active_ * 2 * combos().size(), "P2G item lists"));
-        // [0] work items, [1] outside items, [2] active nodes, [8 + 8k .. 13 + 8k] item
-        // schedulers of the k-th stencil/transfer combination, then the G2P
-        // item counts (kG2PCountWord) and the P2G list counts (kP2GListWord)
+        // counter words: see kCounterWords
         MPM_TRY(alloc(counters_, sizeof(uint32_t) * kCounterWords, "counters"));
         if (!spans_.p) {
             MPM_TRY(alloc(spans_, sizeof(unsigned long long) * kSpanWords * kMaxCombos, "kernel spans"));
@@ -1594,8 +1592,8 @@ public:
     }
 
     // One fused simulateOneStep over every scene of the batch.  In steady state
-    // (keys and stress produced by the previous G2P, no profiling, staging
-    // size decided) the step is replayed from a CUDA graph captured once per
+    // (keys and stress produced by the previous G2P, no profiling, the first
+    // step's counts read back) the step is replayed from a CUDA graph captured once per
     // (particle buffer, key buffer) state; the launch sequence and its
     // arguments only depend on it.
     mpm_status stepOnce() {

@@ -28,13 +28,17 @@ constexpr int kSortTileKeys = kThreads * 8;  // keys per radix-sort tile (8 per 
 // has its own tile; the last of a block's items to finish adds their tiles up
 // in item order, so the grid pass reads one tile per block.  The split fixes
 // the order of P2G's sums, so it depends on nothing but the block's and its
-// scene's particle counts.  Where the line lies: at 35 particles a cell (2,200
-// a full block) whole blocks are faster than items of 2048 or 1024 (P2G 0.099,
-// 0.105 and 0.121 ms), which have too few rows each;
-// a block above 40 a cell has long rows, and scenes of few such blocks need
-// the parallelism (six scenes of up to 60k particles, P2G: items of up to 4096
-// 0.146 ms, split above 4096 into 1024s 0.116, above 2560 into 1280s 0.092;
-// into 640s 0.088, but 64 scenes of up to 500k 0.88 -> 1.03 ms).
+// scene's particle counts.  Where the line lies, ms of P2G in items of up to 2560
+// (above it 1280s) and of up to 4096: below 40 particles a cell (2,560 a full
+// block) both take whole blocks, which are faster there than items of 2048 or
+// 1024 (35 a cell: 0.099, 0.105 and 0.121), which have too few rows each.  Above,
+// scenes of up to half a million particles need the parallelism (200k at 46 a
+// cell, cubic 0.066 and 0.076, quadratic PIC-FLIP 0.037 and 0.063; 500k 0.065 and
+// 0.081, 0.055 and 0.065; six scenes of up to 60k particles 0.092 and 0.146), at a
+// million the two are level (0.119 and 0.119, 0.107 and 0.105), and at two
+// million whole blocks would be the faster ones (46 a cell 0.217 and 0.204, 0.181
+// and 0.167; 58 a cell 0.225 and 0.189, 0.183 and 0.143).  Above 2560 into 640s:
+// the six scenes 0.088, but 64 scenes of up to 500k 0.88 -> 1.03.
 constexpr uint32_t kBlockChunk = 2560;
 constexpr uint32_t kSplitChunk = 1280;
 // A scene of at most kFewParticles cannot fill the chip with such items: its

@@ -1623,9 +1623,9 @@ __global__ void __launch_bounds__(kThreads, GridBounds<S, MODE>::MIN_CTAS) gridK
 }
 
 // ---------------------------------------------------------------------------
-// G2P, fused with the particle update.  One CTA per active block: the block's
-// (S+3)^3 node tile of v* (and v) is staged in shared memory, then one thread
-// per particle.  Writes the particle to its sorted slot of the other buffer.
+// G2P, fused with the particle update.  An item of a block's particles at a time:
+// the block's (S+3)^3 node tile of v* (and v) is staged in shared memory, then one
+// thread per particle.  Writes the particle to its sorted slot of the other buffer.
 // ---------------------------------------------------------------------------
 // The loads of a particle's update, issued one particle ahead into the thread's
 // shared-memory row by cp.async (one commit group per particle, possibly
@@ -1711,7 +1711,7 @@ __device__ __forceinline__ void particleUpdate(const StepArgs& args, const Scene
         // N_z and so on (those of the APIC moment K); PIC-FLIP's of v* - v.
         // Instruction issue and load latency bound the kernel: summing the rows
         // straight into the results took seven scaled additions a row (with
-        // the loads two particles ahead and the base from the cell: two-ball
+        // the loads of g2pFetch and the base from the cell: two-ball
         // G2P 0.118 -> 0.106 ms and 62M -> 56M warp instructions, slab 1.14 ->
         // 0.98 ms).
         struct V3 {
@@ -2027,8 +2027,9 @@ __device__ __forceinline__ void mbarArrive(uint64_t* bar) {
 // every item, and the particle update reads the scene and material from
 // shared memory.
 // Resident G2P CTAs per SM the register budget is fitted to: 2 gives 128
-// registers a thread and no spills (two-ball G2P 0.132 -> 0.117 ms against 3
-// CTAs at 80 registers, which spill ~150 bytes a thread).
+// registers a thread and no spills but for cubic PIC-FLIP's 16 bytes (two-ball
+// G2P 0.132 -> 0.117 ms against 3 CTAs at 80 registers, which spill ~150 bytes a
+// thread).
 #ifndef MPM_G2P_THREADS
 #define MPM_G2P_THREADS 256
 #endif

@@ -1,12 +1,18 @@
-// sort.cu -- stable LSD radix sort of particle keys and device-wide scans.
+// sort.cu -- stable sorts of the particles' cell keys, and device-wide scans.
 //
 // Replaces the reference's unordered global atomics (src/mpm_solver3d.cu:
 // 277-286): particles are ordered by (block, cell) key every step so that the
-// P2G scatter can be done per block in a fixed order.  The sort is stable
-// (ties keep their previous order), hence bit-exact and deterministic.
-//
-// Per 8-bit digit: upsweep (per-tile digit histogram), exclusive scan of the
-// digit-major histogram, downsweep (warp match_any ranking, stable scatter).
+// P2G scatter can be done per block in a fixed order.  Every sort is stable (ties
+// keep their previous order), hence bit-exact and deterministic, and all give
+// the same order:
+//   radixSortPairsInto   LSD radix sort with a histogram, a scan and a scatter
+//                        kernel per 8-bit digit (mpm_sort_keys_device_noalloc)
+//   radixSortOnesweep    one histogram kernel, then one kernel per digit whose
+//                        tiles look back over one another's counts: a scene's
+//                        first step, uploads, crowded blocks
+//   block sort           from the last step's order: blocks put together from
+//                        the particles that stayed and those that came, or by
+//                        the radix passes in one launch where many moved
 #include <cuda_runtime.h>
 #include <stdint.h>
 
