@@ -1302,9 +1302,14 @@ struct P2GWarpLayout : P2GStage<S, MODE> {
     static constexpr int kTileFloats = (R::F * R::TN + 3) / 4 * 4;
     static constexpr int kRowInts = 20;
     static constexpr int kWarpFloats = kSceneFloats + kTileFloats + kStage * R::P4 * 4 + kRowInts;
-    // two CTAs per SM of as many warps as its shared memory holds, at most 24 in all
+    // Two CTAs per SM of as many warps as its shared memory holds, at most 20 in
+    // all: 96 registers a thread.  24 leave 80, where quadratic APIC spills 148
+    // bytes a thread (24 at 96; step of 4M particles, 1 a cell: 2.452 and 2.171 ms,
+    // 4 a cell 1.117 and 1.049; linear 2.260 and 2.235; quadratic PIC-FLIP and
+    // cubic, bound by the shared memory, unchanged); 16 without spills: 2.207, 1.047
+    // and 2.315.
     static constexpr int kWarpsPerSm = (int)(226u * 1024 / (kWarpFloats * 4));
-    static constexpr int NW = (kWarpsPerSm < 24 ? kWarpsPerSm : 24) / 2, NT = 32 * NW;
+    static constexpr int NW = (kWarpsPerSm < 20 ? kWarpsPerSm : 20) / 2, NT = 32 * NW;
     static constexpr size_t smemBytes = (size_t)NW * kWarpFloats * 4;
     static constexpr int MIN_CTAS = 2;
 };
