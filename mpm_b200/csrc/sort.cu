@@ -592,7 +592,6 @@ __global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s) {
     if (threadIdx.x == 0) moved_s = 0u;
     if (blockIdx.x == 0)  // the radix passes' digit counts
         for (int i = threadIdx.x; i < oddPasses(s.key_bits) * 256; i += kBsThreads) s.radix_scratch[i] = 0u;
-    __syncthreads();
     uint32_t moved = 0;
     const uint32_t stride = gridDim.x * kBsThreads * 4;
     const uint32_t n_round = (n + 127) / 128 * 128;  // whole warps iterate together
@@ -607,6 +606,13 @@ __global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s) {
                 old[j] = i0 + j < n ? s.prev_keys[i0 + j] : 0u;
             }
         }
+        // a warp's particles are neighbours in the sorted order: most of its movers
+        // leave the same block, and share one atomic (all four are on their way
+        // before the first is waited for)
+        const int lane = threadIdx.x & 31;
+        uint32_t at[4];
+        unsigned peers[4] = {};  // of a mover: the lanes whose movers go to the same list
+        bool near[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint32_t home = old[j] >> 6, blk = key[j] >> 6;
@@ -615,33 +621,34 @@ __global__ void __launch_bounds__(kBsThreads) emigrantKernel(BlockSortArgs s) {
             if (blk == home) continue;
             const SceneDev& sc = s.scenes[blockScene(s.scene_block_base, s.nscenes, home)];
             const uint32_t out = sc.nblocks, lh = home - sc.block_base, lb = blk - sc.block_base;
-            bool near = lh < out && lb < out;
-            if (near) {
+            near[j] = lh < out && lb < out;
+            if (near[j]) {
                 const int X = sc.nb[0], Y = sc.nb[1];
                 const int dx = (int)(lh % X) - (int)(lb % X), dy = (int)(lh / X % Y) - (int)(lb / X % Y),
                           dz = (int)(lh / (X * Y)) - (int)(lb / (X * Y));
-                near = abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
+                near[j] = abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
             }
+            peers[j] = __match_any_sync(movers, near[j] ? home : 0xffffffffu);
+            if (lane == __ffs(peers[j]) - 1)
+                at[j] = atomicAdd(near[j] ? &s.emig_count[home] : &s.moved[0], (uint32_t)__popc(peers[j]));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!peers[j]) continue;
+            const uint32_t home = old[j] >> 6, c = (uint32_t)__popc(peers[j]);
+            const int leader = __ffs(peers[j]) - 1;
+            const uint32_t first = __shfl_sync(peers[j], at[j], leader);
+            if (near[j] && lane == leader && first <= kEmigMax && first + c > kEmigMax) atomicAdd(&s.moved[2], 1u);
+            const uint32_t slot = first + (uint32_t)__popc(peers[j] & ((1u << lane) - 1u));
             const uint2 e = make_uint2(i0 + j, key[j]);
-            // (a warp's particles are neighbours in the sorted order: most of
-            // its movers leave the same block, and share one atomic)
-            const uint32_t list = near ? home : 0xffffffffu;
-            const unsigned peers = __match_any_sync(movers, list);
-            const int leader = __ffs(peers) - 1, lane = threadIdx.x & 31;
-            uint32_t at = 0;
-            if (lane == leader) {
-                const uint32_t c = (uint32_t)__popc(peers);
-                at = atomicAdd(near ? &s.emig_count[home] : &s.moved[0], c);
-                if (near && at <= kEmigMax && at + c > kEmigMax) atomicAdd(&s.moved[2], 1u);
-            }
-            at = __shfl_sync(peers, at, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-            if (near) s.emig[s.prev_range[home].x + at] = e;
-            else s.far[at] = e;
+            if (near[j]) s.emig[s.prev_range[home].x + slot] = e;
+            else s.far[slot] = e;
         }
     }
+    if (!__syncthreads_or((int)moved)) return;
     if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&moved_s, moved);
     __syncthreads();
-    if (threadIdx.x == 0 && moved_s) atomicAdd(&s.moved[1], moved_s);
+    if (threadIdx.x == 0) atomicAdd(&s.moved[1], moved_s);
 }
 
 // A group of NW warps (a whole CTA, or one warp) that puts blocks together.
@@ -952,21 +959,29 @@ constexpr size_t kBsDenseSmem = std::max(sizeof(BlockSorter<32>::Smem), sizeof(R
 __global__ void __launch_bounds__(kBsThreads, kBsCtas) blockSortKernel(BlockSortArgs s) {
     extern __shared__ unsigned long long bs_smem[];
     __shared__ uint32_t item_s;
-    if (sortByRadix(s)) return;  // blockSortDenseKernel sorts
     const uint32_t nfront = s.counters[kSortFrontWord], nback = s.counters[kSortBackWord];
     const uint32_t nfar = s.moved[0];
     // few small blocks: by CTAs as well, whose latency is a third of a warp's
     const bool all = smallByCtas(s);
     const uint32_t ncta = nfront + (all ? nback : 0u);
+    const bool fixed = ncta <= gridDim.x;  // at most one each: no scheduler
+    BlockItem it{};
+    uint2 prev{};
+    auto take = [&](uint32_t wi) {
+        it = s.list[wi < nfront ? wi : s.list_cap - 1 - (wi - nfront)];
+        prev = s.prev_range[it.block];
+    };
+    // the reads of the first block are in flight while the route is decided
+    if (fixed && blockIdx.x < ncta) take(blockIdx.x);
+    if (sortByRadix(s)) return;  // blockSortDenseKernel sorts
     {
         auto& m = *reinterpret_cast<BlockSorter<kBsWarps>::Smem*>(bs_smem);
         const BlockSorter<kBsWarps> g(m, s, threadIdx.x);
-        const bool fixed = ncta <= gridDim.x;  // at most one each: no scheduler
         for (uint32_t wi = blockIdx.x;;) {
             if (!fixed) wi = nextWorkItem(s.counters + kSortSchedWord, ncta, &item_s);
             if (wi >= ncta) break;
-            const BlockItem it = s.list[wi < nfront ? wi : s.list_cap - 1 - (wi - nfront)];
-            g.run(it, s.prev_range[it.block], nfar);
+            if (!fixed) take(wi);
+            g.run(it, prev, nfar);
             if (fixed) break;
         }
     }
