@@ -394,7 +394,9 @@ MPM_API mpm_status mpm_solver_set_tuning(mpm_solver* s, const mpm_tuning* t);
  * are real steps of the simulation (they advance it; their results are those
  * of any other settings); *steps_run (may be NULL) returns how many were
  * taken.  The cache file is $MPM_TUNE_CACHE, else
- * $XDG_CACHE_HOME/mpm_b200/tuning.txt, else ~/.cache/mpm_b200/tuning.txt.
+ * $XDG_CACHE_HOME/mpm_b200/tuning.txt, else ~/.cache/mpm_b200/tuning.txt;
+ * its lines carry the version of the kernels they were measured on, and those
+ * of another version are skipped.
  * flags: MPM_TUNE_FORCE measures even cached keys; MPM_TUNE_NO_DISK neither
  * reads nor writes the file. */
 #define MPM_TUNE_FORCE 1
